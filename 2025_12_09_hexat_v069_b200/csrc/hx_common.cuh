@@ -254,6 +254,7 @@ struct ElemCoef {
   T lam[3][2];  // lambda * m_k(sigma_k) / 8, k = axis not in the coupled pair
   T mu[3][2];   // mu * m_k(sigma_k) / 8
   T kd[3];      // Ke diagonal entry per component (same at every corner)
+  double rho;   // lambda / mu
 };
 
 // Reference corner order (NAT_COORDS) -> corner bits.

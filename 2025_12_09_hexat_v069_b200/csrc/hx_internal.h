@@ -51,11 +51,9 @@ struct DevBuf {
 };
 
 // ---- operator (hx_operator.cu) ----
-// z-chunk length for `resident` CTAs per SM; CTAs of one launch; the most
-// CTAs of any precision (the reduction workspace's size)
-int mv_kchunk(const Grid& g, int resident);
-size_t mv_num_blocks(const Grid& g, int resident);
-size_t mv_max_blocks(const Grid& g);
+// CTAs of one launch (each leaves a partial sum in the reduction workspace)
+template <typename T>
+size_t mv_num_blocks(const Grid& g);
 template <typename T>
 void launch_matvec(cudaStream_t s, int mode, const T* x, T* y, const T* fac, const uint8_t* nmask,
                    const Grid& g, const ElemCoef<T>& K, T shift, CgState* st, double* partials,

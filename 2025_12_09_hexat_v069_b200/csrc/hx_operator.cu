@@ -8,27 +8,46 @@
 //
 // Kernel design (replaces the one-thread-per-element, 24-atomics kernel of
 // src/Solvers/GPUSolver.jl:37-79 and the broadcast kernels around it):
-//  * a CTA owns a 31 x (BY-1) column of output nodes and marches along z
-//    over a chunk of node planes; its 32 x BY threads each own one element
-//    column, recomputing the one-element halo in x and y (atomic-free and
-//    deterministic);
+//  * a CTA of w warps owns a 31 x (w R - 1) column of output nodes and marches
+//    along z over a chunk of node planes; each thread owns R element columns
+//    adjacent in y, the one-element halo in x and y is recomputed (atomic-free
+//    and deterministic).  FP32: R = 2, and the two elements are the two halves
+//    of packed FP32 operations; FP64: R = 1 (see Tile);
 //  * node planes (tile + one-node halo) are staged into shared memory with
-//    cp.async into a ring of PF+1 slots: planes k+3 .. k+PF are in flight
-//    while plane k+2 is transformed in place and planes k, k+1 feed the
-//    element products (PF = mv_prefetch<T>, planes requested ahead);
-//  * the element product runs in the per-axis sum/difference (Haar) basis
-//    (45 nonzeros, see hx_common.cuh), one displacement component at a
-//    time to bound register pressure; the top-face outputs are carried in
-//    the Haar domain until the layer above adds its bottom face;
-//  * the four element columns around a node are summed with one warp
-//    shuffle (x) and one shared-memory exchange (y);
-//  * FUSED (the PCG step): the staged plane holds p_old, r, M^-1 and x
-//    (the FCG step: p_old, z and x); the in-place transform forms
-//    p = M^-1 r + beta p_old (p = z + beta p_old), and for owned nodes
-//    stores p and updates x += alpha_old p_old.  p ping-pongs between two
+//    16-byte cp.async, several planes ahead (see Stage, Smem);
+//  * the element product runs in the per-axis sum/difference (Haar) basis,
+//    where Ke is eight 3 x 3 blocks (lambda_pair); a plane's face
+//    coefficients are formed once and carried to the layer above, and so are
+//    a layer's top-face outputs;
+//  * the element columns around a node are summed in the thread (the two
+//    elements of a pair), with one warp shuffle (x) and one shared-memory
+//    exchange with the next warp (y).  That exchange is read after the next
+//    plane's barrier, so a plane costs one barrier: the node plane ke is
+//    finished while element layer ke + 1 is computed;
+//  * FUSED (the PCG step): the staged planes hold p_old, r, M^-1 and x (the
+//    FCG step: p_old, z and x).  Each thread forms p = M^-1 r + beta p_old
+//    (p = z + beta p_old) on the chunks that it copied itself, stores it to
+//    a small ring that the element products read and, for owned nodes,
+//    to p, and updates x += alpha_old p_old.  p ping-pongs between two
 //    buffers so neighbouring CTAs never read a value another CTA rewrote.
-//    The epilogue applies the free-DOF mask and the shift and reduces p.q
-//    deterministically into the CG state (alpha = rz / pq).
+//    The epilogue adds the shift and reduces p.q deterministically into the
+//    CG state (alpha = rz / pq); q stays unmasked on the fixed DOFs, where p is
+//    0 and the residual update does not read it.
+// What bounds it: instruction issue and the latency between dependent
+// instructions (12 warps per SM, 50-62% of the issue slots used), not memory
+// (the FP32 flexible-CG step moves 0.64 GB at 3.8 TB/s, the FP64 PCG step 1.47
+// GB at 4.6 TB/s).  A warp issues about 520 instructions per plane and pair of
+// element rows in FP32 and 370 per row in FP64.
+// Measured at 320 x 160 x 160 (B200), before (one element column per thread in
+// both precisions, 45-term product, two barriers per plane) and now: FP64 PCG
+// step 402 -> 319 us, FP64 K x 260 -> 205 us, FP32 PCG step 220 -> 182 us, FP32
+// flexible-CG step 207 -> 170 us; FP32 Chebyshev step and residual at 192 x 96
+// x 96: 55 -> 36 and 50 -> 36 us.
+// Measured and dropped (FP32 flexible-CG step, 320 x 160 x 160): one element
+// row per thread at 24 warps per SM 188 us; 8 warps x 2 CTAs (128 registers,
+// spills) 189-204 us; 12 x 1 201 us; 6 x 2 178 us; the plane loop unrolled
+// twice 179-208 us; positions advanced per plane instead of recomputed 176-182
+// us.
 #include <type_traits>
 
 #include "hx_internal.h"
@@ -37,26 +56,7 @@ namespace hx {
 
 namespace {
 
-constexpr int MV_BX = 32;
-constexpr int MV_BY = 8;
-// CTAs per SM (the __launch_bounds__ minimum): FP32 instantiations fit 80
-// registers and three CTAs' rings in shared memory (3% faster than two at
-// C1); FP64 ones need 128 registers.
-template <typename T>
-constexpr int mv_resident() { return sizeof(T) == 4 ? 3 : 2; }
-
-// Planes requested ahead of the layer being computed (>= 3).  A deeper ring
-// keeps more bytes in flight per SM: FP32 runs 2% faster at depth 5 than 3
-// at 320x160x160; the FP64 fused ring at depth 4 (106 KB) drops to one CTA
-// per SM and runs 50% slower, so FP64 stays at 3.
-#ifndef HX_PF32
-#define HX_PF32 5
-#endif
-#ifndef HX_PF64
-#define HX_PF64 3
-#endif
-template <typename T>
-constexpr int mv_prefetch() { return sizeof(T) == 4 ? HX_PF32 : HX_PF64; }
+constexpr int MV_BX = 32;  // lanes = element columns in x
 
 __device__ __forceinline__ unsigned smem_u32(const void* p) {
   return (unsigned)__cvta_generic_to_shared(p);
@@ -68,46 +68,173 @@ __device__ __forceinline__ void cp_async16(unsigned sdst, const void* gsrc, unsi
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sdst), "l"(gsrc),
                "r"(bytes));
 }
+__device__ __forceinline__ void cp_async16(unsigned sdst, const void* gsrc) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sdst), "l"(gsrc));
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
+// Elements per thread (R), the type that holds one value of each, warps per
+// CTA and CTAs per SM.  The forms want about 160 registers a thread (the face
+// coefficients of two planes, the carried outputs and the block in work), so
+// 12 warps fit an SM; small CTAs wait less at the barrier of a plane, large
+// ones recompute less halo.  FP64 K x fits 128 registers (16 warps: 205 us at
+// 320 x 160 x 160 against 219 us in the fused form's shape; the fused form in
+// that shape spills: 406 against 319 us).
+template <typename T, bool FUSED>
+struct Tile;
+template <bool FUSED>
+struct Tile<float, FUSED> {
+  static constexpr int R = 2, WARPS = 4, RESIDENT = 3;
+  using V = float2;
+};
+template <bool FUSED>
+struct Tile<double, FUSED> {
+  static constexpr int R = 1, WARPS = FUSED ? 6 : 8, RESIDENT = 2;
+  using V = double;
+};
+template <typename T>
+using VecOf = typename Tile<T, false>::V;
+template <typename T, bool FUSED>
+constexpr int mv_by() { return Tile<T, FUSED>::WARPS * Tile<T, FUSED>::R; }  // element rows of a CTA
+constexpr bool mode_fused(int mode) { return mode == 3 || mode == 4; }
+
+__device__ __forceinline__ double vadd(double a, double b) { return a + b; }
+__device__ __forceinline__ double vmul(double a, double b) { return a * b; }
+__device__ __forceinline__ double vfma(double a, double b, double c) { return fma(a, b, c); }
+__device__ __forceinline__ float2 vadd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 vmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+__device__ __forceinline__ double vneg(double a) { return -a; }
+__device__ __forceinline__ float2 vneg(float2 a) { return make_float2(-a.x, -a.y); }
+template <typename V>
+__device__ __forceinline__ V vzero();
+template <>
+__device__ __forceinline__ double vzero<double>() { return 0.0; }
+template <>
+__device__ __forceinline__ float2 vzero<float2>() { return make_float2(0.f, 0.f); }
+template <typename V>
+__device__ __forceinline__ V vone();
+template <>
+__device__ __forceinline__ double vone<double>() { return 1.0; }
+template <>
+__device__ __forceinline__ float2 vone<float2>() { return make_float2(1.f, 1.f); }
+
+// a - b as fma(b, m, a) with m = (-1, -1) held in registers
+__device__ __forceinline__ float2 vsubm(float2 a, float2 b, float2 m) { return __ffma2_rn(b, m, a); }
+__device__ __forceinline__ double vsubm(double a, double b, double) { return a - b; }
+// Element coefficients, one per element of the thread (both halves equal):
+// the Haar-domain operator of a box element, or (CUBE) the five numbers that
+// are left of it for equal sides (see lambda_pair).
+template <typename V, bool CUBE>
+struct CoefV {
+  V dg[3][8], lam[3][2], mu[3][2];
+};
+template <typename V>
+struct CoefV<V, true> {
+  V unit, rho, rho3, rho49, third;
+};
+__host__ inline void put(double& d, double v) { d = v; }
+__host__ inline void put(float2& d, double v) { d = make_float2((float)v, (float)v); }
+template <typename T, typename V>
+void coef_v(const ElemCoef<T>& k, CoefV<V, false>& o) {
+  for (int c = 0; c < 3; ++c) {
+    for (int s = 0; s < 8; ++s) put(o.dg[c][s], (double)k.dg[c][s]);
+    for (int s = 0; s < 2; ++s) {
+      put(o.lam[c][s], (double)k.lam[c][s]);
+      put(o.mu[c][s], (double)k.mu[c][s]);
+    }
+  }
+}
+template <typename T, typename V>
+void coef_v(const ElemCoef<T>& k, CoefV<V, true>& o) {
+  put(o.unit, (double)k.mu[0][0]);
+  put(o.rho, k.rho);
+  put(o.rho3, k.rho / 3.0);
+  put(o.rho49, (k.rho + 4.0) / 9.0);
+  put(o.third, 1.0 / 3.0);
+}
+// Loop constants that stay in vector registers: read back from shared memory,
+// so that the compiler takes them for data.  Straight from the kernel's
+// arguments it keeps them in uniform registers, which packed operations cannot
+// read: every use then costs moves.  CUBE only (the general coefficients are
+// too many for registers).
+template <typename V>
+__device__ __forceinline__ V from_shared(const volatile V* p);
+template <>
+__device__ __forceinline__ double from_shared<double>(const volatile double* p) { return *p; }
+template <>
+__device__ __forceinline__ float2 from_shared<float2>(const volatile float2* p) {
+  return make_float2(p->x, p->y);
+}
+template <typename V>
+__device__ __forceinline__ void pin_coef(CoefV<V, true>& k, const volatile V* sh) {
+  k.rho = from_shared(sh);
+  k.rho3 = from_shared(sh + 1);
+  k.rho49 = from_shared(sh + 2);
+  k.third = from_shared(sh + 3);
+}
+template <typename V>
+__device__ __forceinline__ void pin_coef(CoefV<V, false>&, const volatile V*) {}
+template <typename V>
+__device__ __forceinline__ void share_coef(const CoefV<V, true>& k, V* sh) {
+  sh[0] = k.rho;
+  sh[1] = k.rho3;
+  sh[2] = k.rho49;
+  sh[3] = k.third;
+}
+template <typename V>
+__device__ __forceinline__ void share_coef(const CoefV<V, false>&, V*) {}
+template <typename V>
+__device__ __forceinline__ V unit_of(const CoefV<V, true>& k) { return k.unit; }
+template <typename V>
+__device__ __forceinline__ V unit_of(const CoefV<V, false>&) { return vzero<V>(); }
+
 // Staging geometry.  A staged row is the 33 nodes i0-1 .. i0+31 of one
 // node row, 99 contiguous values of an interleaved vector.  It is copied in
-// 16-byte chunks (V values) starting at the 16-byte boundary at or below its
+// 16-byte chunks (W values) starting at the 16-byte boundary at or below its
 // first value, so a row takes CPR chunks and sits in shared memory with a
-// lead of (first value's index) mod V values, which depends on the row and
+// lead of (first value's index) mod W values, which depends on the row and
 // the plane.  Lanes then read node a, component c of row b at
 // b*RS + lead_b + 3a + c: a stride of 3 words (FP32) or 3 doublewords
 // (FP64) across a warp, free of bank conflicts.
-template <typename T>
+template <typename T, bool FUSED>
 struct Stage {
-  static constexpr int V = 16 / (int)sizeof(T);                // values per chunk
-  static constexpr int ROWV = 3 * (MV_BX + 1);                 // 99 values per row
-  static constexpr int CPR = (ROWV + V - 1 + V - 1) / V;       // chunks per row
-  static constexpr int RS = CPR * V;                           // row stride (values)
-  static_assert(RS >= ROWV + V - 1, "a row with any lead fits its staged chunks");
-};
-
-// Shared-memory layout (dynamic): rows of interleaved values (see Stage).
-template <typename T, int BY, bool FUSED>
-struct OpSmem {
-  static constexpr int PLANE = (BY + 1) * Stage<T>::RS;
+  static constexpr int W = 16 / (int)sizeof(T);           // values per chunk
+  static constexpr int ROWV = 3 * (MV_BX + 1);            // 99 values per row
+  static constexpr int CPR = (ROWV + W - 1 + W - 1) / W;  // chunks per row
+  static constexpr int RS = CPR * W;                      // row stride (values)
+  static constexpr int ROWS = mv_by<T, FUSED>() + 1;
+  static constexpr int PLANE = ROWS * RS;                 // values
+  static_assert(RS >= ROWV + W - 1, "a row with any lead fits its staged chunks");
   static_assert((PLANE * sizeof(T)) % 16 == 0, "planes keep 16-byte chunk alignment");
-  static constexpr int PF = mv_prefetch<T>();
-  static constexpr int NP = PF + 1;             // slots: k, k+1, k+2, k+3 .. k+PF
-  static constexpr int NR = FUSED ? PF - 1 : 1;  // slots: k+2 .. k+PF
-  static_assert(PF >= 3, "the ring needs planes k .. k+3");
-  T p[NP][PLANE];   // x or p
-  T r[NR][PLANE];   // r (FUSED)
-  T m[NR][PLANE];   // M^-1, or z in MODE 4 (FUSED)
-  T x[NR][PLANE];   // x (FUSED)
-  T red[BY][3][MV_BX];  // y-direction partials
 };
 
-template <typename T>
+// Rings of staged planes, by MODE (see k_struct).  FUSED: NS planes of each
+// input in flight (a thread transforms the chunks that it copied itself, so
+// a slot is free again at once), two or three planes of the new p.  Others: NX planes
+// of x, of which NX - 2 are in flight, and NA planes of each of the AUX
+// vectors that the epilogue reads.
+template <typename T, int MODE>
+struct Smem {
+  static constexpr bool FUSED = mode_fused(MODE);
+  static constexpr int PLANE = Stage<T, FUSED>::PLANE, WARPS = Tile<T, FUSED>::WARPS;
+  static constexpr int IN = MODE == 3 ? 4 : 3;  // FUSED: staged inputs
+  static constexpr int NS = 3;
+  static constexpr int AUX = MODE == 5 ? 3 : (MODE == 6 ? 1 : 0);
+  static constexpr int NX = FUSED ? (sizeof(T) == 4 ? 3 : 2) : (AUX ? 4 : 6);
+  static constexpr bool KEEP = NX == 2;  // plane ke is gone when its sums are ready
+  static constexpr int NA = AUX ? 3 : 0;
+  T p[NX][PLANE];
+  T in[FUSED ? NS : (AUX ? NA : 1)][FUSED ? IN : (AUX ? AUX : 1)][(FUSED || AUX) ? PLANE : 16 / (int)sizeof(T)];
+  T red[2][WARPS][3][MV_BX];  // y-direction partials, of two planes
+  VecOf<T> k[6];  // loop constants (see from_shared)
+};
+
+template <typename T, bool CUBE>
 struct OpArgs {
-  const T* pin;   // vector to multiply (MODE 0-2) or p_old (FUSED)
+  const T* pin;   // vector to multiply (MODE 0, 1, 5, 6) or p_old (FUSED)
   const T* r;     // MODE 3: residual; MODE 5, 6: right-hand side b
   const T* minv;  // MODE 3, 5: Jacobi inverse diagonal; MODE 4: preconditioned z
   T* x;           // FUSED: solution (x += alpha_old p_old on owned nodes); MODE 5:
@@ -118,7 +245,7 @@ struct OpArgs {
   const uint8_t* nmask;
   Grid g;
   int kchunk;
-  ElemCoef<T> K;
+  CoefV<VecOf<T>, CUBE> K;
   T shift;
   T omega, gamma;  // MODE 5: recurrence coefficients
   int xprev_zero;  // MODE 5: x_prev = 0 (not read)
@@ -127,426 +254,619 @@ struct OpArgs {
   double* out;
 };
 
-// 2D sum/difference transform of a node-plane face: v = corners (bx + 2by)
-// -> P = coefficients (sigma_x + 2 sigma_y).
-template <typename T>
-__device__ __forceinline__ void face_fwd(const T (&v)[4], T (&P)[4]) {
-  const T e0s = v[0] + v[1], e0d = v[1] - v[0], e1s = v[2] + v[3], e1d = v[3] - v[2];
-  P[0] = e0s + e1s;
-  P[1] = e0d + e1d;
-  P[2] = e1s - e0s;
-  P[3] = e1d - e0d;
-}
-
-// Component C of f * Lambda U: the diagonal part plus the couplings with
-// the other two components (see haar_apply in hx_common.cuh).
-template <typename T, int C>
-__device__ __forceinline__ void lambda_row(const ElemCoef<T>& K, const T (&U)[3][8], T (&Y)[8]) {
-  Y[0] = T(0);
+// Lambda in the Haar domain.  Its coefficients couple only where t = sigma xor
+// e_c agrees (e_c: the bit of the component's own axis): eight blocks of one
+// coefficient per component, through lambda where neither of the two
+// components' bits is set in t, through mu where both are.  Blocks Q and Q + 4
+// together take the z-sums s and z-differences d of the face coefficients
+// (x, Q ^ 1), (y, Q ^ 2) and (z, Q), and give the outputs of the same three,
+// so a layer's product needs few values at a time.  The z-sum of coefficient
+// 0 is a rigid translation: it is not read and its output is 0.
+template <int Q, typename V>
+__device__ __forceinline__ void lambda_pair(const CoefV<V, false>& K, V (&s)[3], V (&d)[3]) {
 #pragma unroll
-  for (int s = 1; s < 8; ++s) Y[s] = K.dg[C][s] * U[C][s];
+  for (int h = 0; h < 2; ++h) {
+    const int t = Q + 4 * h;
+    // block t: x and y from s (h = 0) or d, z from d (h = 0) or s
+    V u[3] = {h ? d[0] : s[0], h ? d[1] : s[1], h ? s[2] : d[2]}, y[3];
 #pragma unroll
-  for (int t = 1; t <= 2; ++t) {
-    const int o = (C + t) % 3;
-    const int k = 3 - C - o;
+    for (int c = 0; c < 3; ++c) {
+      const int sg = t ^ (1 << c);
+      if (!sg) {
+        y[c] = vzero<V>();
+        continue;
+      }
+      y[c] = vmul(K.dg[c][sg], u[c]);
 #pragma unroll
-    for (int sk = 0; sk < 2; ++sk) {
-      const int P = (1 << o) | (sk << k);  // sigma_C = s, sigma_o = d
-      const int Q = (1 << C) | (sk << k);  // sigma_C = d, sigma_o = s
-      Y[Q] += K.lam[k][sk] * U[o][P];
-      Y[P] += K.mu[k][sk] * U[o][Q];
+      for (int e = 1; e <= 2; ++e) {
+        const int o = (c + e) % 3, k = 3 - c - o;
+        const int bc = (t >> c) & 1, bo = (t >> o) & 1, bk = (t >> k) & 1;
+        if (bc != bo || !(t ^ (1 << o))) continue;
+        y[c] = vfma(bc ? K.mu[k][bk] : K.lam[k][bk], u[o], y[c]);
+      }
     }
+    (h ? d[0] : s[0]) = y[0];
+    (h ? d[1] : s[1]) = y[1];
+    (h ? s[2] : d[2]) = y[2];
+  }
+}
+// Equal sides h, in units of mu h / 16 (folded into the element factor), with
+// rho = lambda / mu: normal strains (t = 0) 2 u_c + rho (u_x + u_y + u_z);
+// t one bit: u_i + rho/3 (u_i + u_j) for the other two components; t two bits:
+// u_i + u_j for both of them, (rho + 4)/9 u for the third; t = 7: (u_c + sum)/3.
+// 27 operations instead of 45, and no coefficient per entry to load.
+template <int Q, typename V>
+__device__ __forceinline__ void lambda_pair(const CoefV<V, true>& K, V (&s)[3], V (&d)[3]) {
+  auto bit1 = [&](V& a, V& b) {
+    const V t = vadd(a, b);
+    a = vfma(K.rho3, t, a);
+    b = vfma(K.rho3, t, b);
+  };
+  if constexpr (Q == 0) {
+    const V t = vmul(K.rho, vadd(vadd(s[0], s[1]), d[2]));
+    s[0] = vadd(vadd(s[0], s[0]), t);
+    s[1] = vadd(vadd(s[1], s[1]), t);
+    d[2] = vadd(vadd(d[2], d[2]), t);
+    bit1(d[0], d[1]);
+    s[2] = vzero<V>();
+  } else if constexpr (Q == 1) {
+    bit1(s[1], d[2]);
+    s[0] = vzero<V>();
+    d[0] = s[2] = vadd(d[0], s[2]);
+    d[1] = vmul(K.rho49, d[1]);
+  } else if constexpr (Q == 2) {
+    bit1(s[0], d[2]);
+    s[1] = vzero<V>();
+    d[1] = s[2] = vadd(d[1], s[2]);
+    d[0] = vmul(K.rho49, d[0]);
+  } else {
+    s[0] = s[1] = vadd(s[0], s[1]);
+    d[2] = vmul(K.rho49, d[2]);
+    const V t = vmul(K.third, vadd(vadd(d[0], d[1]), s[2]));
+    d[0] = vfma(K.third, d[0], t);
+    d[1] = vfma(K.third, d[1], t);
+    s[2] = vfma(K.third, s[2], t);
   }
 }
 
 // MODE 0: q = mask(K x + s x);  MODE 1: also out[0] = x.q;
-// MODE 5: Chebyshev step of the multigrid smoother as a three-term
-//         recurrence on x: x_new = x + omega (x - x_prev) + gamma M^-1 (b - A x)
-//         with A x = mask(K x + s x); x_prev (A.x) is overwritten by x_new
-//         (each node's x_prev is read and written by its owner only; the
-//         staged x, read by the neighbours, is not written).
-// MODE 6: residual r = mask(b - K x - s x) into A.q;
-// MODE 2: CG matvec, st->pq = p.q, st->alpha = rz / pq, breakdown test;
-// MODE 3: fused PCG step (see file header), then as MODE 2;
+// MODE 3: fused PCG step (see file header): st->pq = p.q, st->alpha = rz / pq,
+//         breakdown test;
 // MODE 4: flexible-CG step: p = z + beta p_old (z from a variable
 //         preconditioner), x += alpha_old p_old, q = K p; alpha = z.r / p.q
 //         with z.r from the preconditioner's output pass (st->aux[3]); p.r
 //         = z.r + beta p_old.r and the previous step length makes p_old.r
-//         vanish, so r is not staged.
-template <typename T, int BY, int MODE, int MINB>
-__global__ void __launch_bounds__(MV_BX* BY, MINB) k_struct(OpArgs<T> A) {
-  constexpr bool FUSED = MODE == 3 || MODE == 4;
-  constexpr bool DOT = MODE >= 1 && MODE <= 4;  // reduces p.q / x.q
-  constexpr int NT = MV_BX * BY;
-  constexpr int V = Stage<T>::V;
-  constexpr int CPR = Stage<T>::CPR;
-  constexpr int RS = Stage<T>::RS;
-  constexpr int NCH = (BY + 1) * CPR;          // chunks per staged plane
-  constexpr int NCT = (NCH + NT - 1) / NT;     // chunks per thread
-  constexpr int PF = OpSmem<T, BY, FUSED>::PF;
-  constexpr int NP = OpSmem<T, BY, FUSED>::NP;
-  constexpr int NR = OpSmem<T, BY, FUSED>::NR;
+//         vanish, so r is not staged;
+// MODE 5: Chebyshev step of the multigrid smoother as a three-term
+//         recurrence on x: x_new = x + omega (x - x_prev) + gamma M^-1 (b - A x)
+//         with A x = mask(K x + s x); x_prev (A.x) is overwritten by x_new
+//         (each node's x_prev is read and written by its owner only; the
+//         staged x, read by the neighbours, is not written);
+// MODE 6: residual r = mask(b - K x - s x) into A.q.
+template <typename T, int MODE, bool CUBE>
+__global__ void __launch_bounds__(MV_BX* Tile<T, mode_fused(MODE)>::WARPS,
+                                  Tile<T, mode_fused(MODE)>::RESIDENT)
+    k_struct(const __grid_constant__ OpArgs<T, CUBE> A) {
+  using S = Smem<T, MODE>;
+  using G = Stage<T, S::FUSED>;
+  using V = VecOf<T>;
+  constexpr bool FUSED = S::FUSED;
+  constexpr bool DOT = MODE == 1 || FUSED;  // reduces x.q / p.q
+  constexpr int R = Tile<T, FUSED>::R, WARPS = S::WARPS, BY = WARPS * R;
+  constexpr int NT = MV_BX * WARPS;
+  constexpr int W = G::W, CPR = G::CPR, RS = G::RS, PLANE = G::PLANE;
+  // Chunks of a staged plane by thread: FP32 in runs of 32 chunks of a row, run
+  // wy, wy + WARPS, ... by warp wy (a row is one run of 26); FP64, whose rows are
+  // 50 chunks, one after the other.
+  constexpr bool RUNS = CPR <= 32;
+  constexpr int NCT = RUNS ? (G::ROWS + WARPS - 1) / WARPS : (G::ROWS * CPR + NT - 1) / NT;
   using VecT = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-  if (MODE >= 2 && MODE <= 4 && A.st->status != HX_RUNNING) return;
+  if (FUSED && A.st->status != HX_RUNNING) return;
   extern __shared__ __align__(16) unsigned char smraw[];
-  OpSmem<T, BY, FUSED>& sm = *reinterpret_cast<OpSmem<T, BY, FUSED>*>(smraw);
-  const Grid g = A.g;
-  const int lx = threadIdx.x, ly = threadIdx.y;
-  const int tid = lx + MV_BX * ly;
+  S& sm = *reinterpret_cast<S*>(smraw);
+  const Grid& g = A.g;
+  const int lx = threadIdx.x, wy = threadIdx.y;
+  const int tid = lx + MV_BX * wy;
   const int i0 = blockIdx.x * (MV_BX - 1), j0 = blockIdx.y * (BY - 1);
   const int k0 = blockIdx.z * A.kchunk;
   const int k1 = min(k0 + A.kchunk, g.nzn);
-  const int in = i0 - 1 + lx, jn = j0 - 1 + ly;
-  const bool col_ok = in >= 0 && jn >= 0 && in < g.nxe && jn < g.nye;
-  const bool out_ok = lx >= 1 && ly >= 1 && in < g.nxn && jn < g.nyn;
-  const int64_t nplane = (int64_t)g.nxn * g.nyn;
-  const int64_t eplane = (int64_t)g.nxe * g.nye;
-  const int64_t ndof = 3 * nplane * g.nzn;
+  const int in = i0 - 1 + lx, jn = j0 - 1 + R * wy;  // first element column, first node
+  const int nplane = g.nxn * g.nyn;
+  const int P3 = 3 * nplane;  // values per node plane (32-bit: the grid extent check bounds it)
+  const int kp_last = min(k1, g.nzn - 1);  // last plane staged
   T alpha_old = T(0), beta_old = T(0);
   if (FUSED) {
     alpha_old = (T)A.st->alpha;
     beta_old = (T)A.st->beta;
   }
 
-  // Chunk assignment, the same for every plane: this thread copies (and, in
-  // the fused modes, transforms) chunks tid, tid + NT, ... of the plane.
-  // row_off = first staged value of the chunk's row, relative to the plane's
-  // first value 3 * kp * nplane (32-bit: the grid extent check bounds it);
-  // a row's owned nodes i0 .. i0+30 (inside the grid) are the own_len values
-  // from row_off + 3; halo rows own none (bit q of own_rows clear).
-  int row_off[NCT];
-  int cbase[NCT];  // shared-memory offset of the chunk: its row's start + ccv
-  int ccv[NCT];    // offset of the chunk within its row (values)
-  unsigned own_rows = 0;
+  // Rows and nodes outside the grid are never copied: they have to be finite,
+  // and are 0.  CTAs inside the grid read only what they copied.
+  if (i0 + MV_BX >= g.nxn || j0 == 0 || j0 - 1 + BY >= g.nyn)
+    for (int i = tid; i < (int)(sizeof(S) / 16); i += NT)
+      reinterpret_cast<uint4*>(smraw)[i] = make_uint4(0u, 0u, 0u, 0u);
+
+  // Chunk assignment, the same for every plane: the chunks that this thread
+  // copies (and, in the fused modes, transforms).  rof: a chunk's first value,
+  // before rounding down to W, from the plane's first value (32-bit: the grid
+  // extent check bounds it).  use / own: chunks inside the grid / in owned rows;
+  // a row's owned nodes are the own_len values from 3 past its first, dlo the
+  // chunk's offset from them for a lead of 0.
+  int rofa[NCT], sba[NCT], dla[NCT];
+  bool use[NCT], own[NCT];
   const int own_len = 3 * (min(i0 + MV_BX - 1, g.nxn) - i0);
+  const int rstep = 3 * WARPS * g.nxn;
 #pragma unroll
   for (int q = 0; q < NCT; ++q) {
-    const int ch = min(tid + q * NT, NCH - 1);
-    const int b = ch / CPR, cc = ch - b * CPR;
+    const int ch = tid + q * NT;
+    const int b = RUNS ? wy + q * WARPS : ch / CPR, cc = RUNS ? lx : ch - b * CPR;
     const int jj = j0 - 1 + b;
-    row_off[q] = 3 * (jj * g.nxn + i0 - 1);
-    if (b >= 1 && b <= BY - 1 && jj < g.nyn) own_rows |= 1u << q;
-    ccv[q] = cc * V;
-    cbase[q] = b * RS + ccv[q];
+    // a chunk past the row's last node in the grid is not needed
+    use[q] = b <= BY && cc < CPR && jj >= 0 && jj < g.nyn && cc * W < 3 * (g.nxn - i0 + 1) + W - 1;
+    own[q] = use[q] && b >= 1 && b <= BY - 1;
+    rofa[q] = 3 * (jj * g.nxn + i0 - 1) + cc * W;
+    sba[q] = b * RS + cc * W;
+    dla[q] = cc * W - 3;
   }
-  // The first staged value of a chunk's row in plane kp has global index
-  // o = 3 nplane kp + row_off; the chunk's first value is o rounded down to
-  // a multiple of V plus ccv.
-  const int64_t P3 = 3 * nplane;
+  auto rof = [&](int q) { return RUNS ? rofa[0] + q * rstep : rofa[q]; };
+  auto sbase = [&](int q) { return RUNS ? sba[0] + q * WARPS * RS : sba[q]; };
+  auto dlo = [&](int q) { return RUNS ? dla[0] : dla[q]; };
+  __syncthreads();
+  if (tid == 0) {
+    share_coef(A.K, sm.k);
+    sm.k[4] = vneg(vone<V>());
+  }
+  __syncthreads();
 
-  // One commit group per call, empty for planes past k1, so that the
-  // wait counts below hold to the end of the chunk.  Chunks outside the
-  // vectors (planes k0-1 < 0 or nzn, rows before the first value) are
-  // zero-filled; a chunk reaching past the last value copies only its part
-  // inside.  Other values outside the grid (halo nodes beyond a row's end,
-  // halo rows beyond the plane) are copied as they lie in memory: they only
-  // feed element columns with factor 0, whose products are zero.
-  auto issue = [&](int kp, int slp, int slr) {
-    if (kp > k1) {
-      cp_async_commit();
+  // Node plane kp starts at value pv = kp * P3: a chunk's 16-byte aligned
+  // address is the plane's rounded-down base plus a 32-bit offset.
+  auto chunk_off = [&](int q, int64_t pv) { return (rof(q) + (int)(pv & (W - 1))) & ~(W - 1); };
+  auto plane_ptr = [&](auto* v, int64_t pv) { return v + (pv & ~(int64_t)(W - 1)); };
+  // Copies of plane kp of the vectors that the mode stages, chunk by chunk.
+  // Only the first and last planes hold chunks that start before the vector
+  // or reach past its end: those are cut to the part inside (the rest is 0).
+  const bool use_xp = MODE == 5 && !A.xprev_zero && A.omega != T(0);
+  const int nzn = g.nzn;
+  auto cut = [&](const T* v, T* sdst, int q, int64_t pv) {
+    const int64_t at = (pv & ~(int64_t)(W - 1)) + chunk_off(q, pv), left = P3 * (int64_t)nzn - at;
+    const unsigned bytes =
+        (at >= 0 && left > 0) ? (unsigned)((left < W ? left : (int64_t)W) * sizeof(T)) : 0u;
+    cp_async16(smem_u32(sdst + sbase(q)), v + (bytes ? at : 0), bytes);
+  };
+  auto issue = [&](int kp, T* p) {
+    if ((unsigned)kp > (unsigned)kp_last) return;
+    const int64_t pv = (int64_t)kp * P3;
+    const bool kown = kp >= k0 && kp < k1;
+    if (kp == 0 || kp == nzn - 1) {
+#pragma unroll
+      for (int q = 0; q < NCT; ++q) {
+        if (!use[q]) continue;
+        cut(A.pin, p, q, pv);
+        if (FUSED) {
+          cut(A.minv, p + PLANE, q, pv);
+          if (own[q] && kown) cut(A.x, p + 2 * PLANE, q, pv);
+          if (MODE == 3) cut(A.r, p + 3 * PLANE, q, pv);
+        }
+      }
       return;
     }
-    const bool kin = kp >= 0 && kp < g.nzn;
-    const unsigned sp = smem_u32(&sm.p[slp][0]);
-    const unsigned sr = smem_u32(&sm.r[FUSED ? slr : 0][0]);
-    const unsigned smv = smem_u32(&sm.m[FUSED ? slr : 0][0]);
-    const unsigned sx = smem_u32(&sm.x[FUSED ? slr : 0][0]);
+    const T* bp = plane_ptr(A.pin, pv);
+    const T* bm = FUSED ? plane_ptr(A.minv, pv) : nullptr;
+    const T* bx = FUSED ? plane_ptr((const T*)A.x, pv) : nullptr;
+    const T* br = MODE == 3 ? plane_ptr(A.r, pv) : nullptr;
+    const unsigned d0 = smem_u32(p);
 #pragma unroll
     for (int q = 0; q < NCT; ++q) {
-      if (q == NCT - 1 && tid + q * NT >= NCH) continue;
-      const int64_t o = (int64_t)kp * P3 + row_off[q];
-      const int64_t s = o - (o & (V - 1)) + ccv[q];
-      const int64_t left = ndof - s;
-      const unsigned bytes =
-          (kin && s >= 0 && left > 0) ? (unsigned)((left < V ? left : (int64_t)V) * sizeof(T)) : 0u;
-      const int64_t gi = bytes ? s : 0;
-      const unsigned so = (unsigned)cbase[q] * (unsigned)sizeof(T);
-      cp_async16(sp + so, A.pin + gi, bytes);
-      if (FUSED) {
-        if (MODE == 3) cp_async16(sr + so, A.r + gi, bytes);
-        cp_async16(smv + so, A.minv + gi, bytes);
-        cp_async16(sx + so, A.x + gi, bytes);
+      const int off = chunk_off(q, pv);
+      const unsigned d = d0 + sbase(q) * (int)sizeof(T);
+      if (use[q]) {
+        cp_async16(d, bp + off);
+        if (FUSED) cp_async16(d + PLANE * sizeof(T), bm + off);
+        if (MODE == 3) cp_async16(d + 3 * PLANE * sizeof(T), br + off);
+      }
+      if (FUSED && own[q] && kown) cp_async16(d + 2 * PLANE * sizeof(T), bx + off);
+    }
+  };
+  auto issue_aux = [&](int kp, T* aux) {
+    if (kp < k0 || kp >= k1) return;
+    const int64_t pv = (int64_t)kp * P3;
+    if (kp == 0 || kp == nzn - 1) {
+#pragma unroll
+      for (int q = 0; q < NCT; ++q) {
+        if (!own[q]) continue;
+        cut(A.r, aux, q, pv);
+        if (MODE == 5) cut(A.minv, aux + PLANE, q, pv);
+        if (MODE == 5 && use_xp) cut(A.x, aux + 2 * PLANE, q, pv);
+      }
+      return;
+    }
+    const T* br = plane_ptr(A.r, pv);
+    const T* bm = MODE == 5 ? plane_ptr(A.minv, pv) : nullptr;
+    const T* bx = MODE == 5 ? plane_ptr((const T*)A.x, pv) : nullptr;
+    const unsigned d0 = smem_u32(aux);
+#pragma unroll
+    for (int q = 0; q < NCT; ++q) {
+      const int off = chunk_off(q, pv);
+      const unsigned d = d0 + sbase(q) * (int)sizeof(T);
+      if (own[q]) {
+        cp_async16(d, br + off);
+        if (MODE == 5) cp_async16(d + PLANE * sizeof(T), bm + off);
+        if (MODE == 5 && use_xp) cp_async16(d + 2 * PLANE * sizeof(T), bx + off);
       }
     }
-    cp_async_commit();
   };
 
-  // FUSED: p = M^-1 r + beta p_old (MODE 4: z + beta p_old) in place, chunk
-  // by chunk; the values of owned nodes of owned planes are stored to p and
-  // advance x with the old direction (16-byte stores where a whole chunk is
-  // owned).
-  auto transform = [&](int kp, int slp, int slr) {
-    if (!FUSED) return;
+  // FUSED: p = M^-1 r + beta p_old (MODE 4: z + beta p_old) of this thread's
+  // chunks of plane kp into pd; the values of owned nodes of owned planes are
+  // stored to p and advance x with the old direction (16-byte stores where a
+  // whole chunk is owned).
+  auto transform = [&](int kp, const T* src, T* pd) {
+    if ((unsigned)kp > (unsigned)kp_last) return;
     const bool kown = kp >= k0 && kp < k1;
-    T* ps = &sm.p[slp][0];
-    const T* rs = &sm.r[slr][0];
-    const T* ms = &sm.m[slr][0];
-    const T* xs = &sm.x[slr][0];
+    const int64_t pv = (int64_t)kp * P3;
 #pragma unroll
     for (int q = 0; q < NCT; ++q) {
-      if (q == NCT - 1 && tid + q * NT >= NCH) continue;
-      const int64_t ob = (int64_t)kp * P3 + row_off[q];
-      const int o = cbase[q];
-      T pnew[V], xv[V];
-      {
-        const VecT pv = *reinterpret_cast<const VecT*>(ps + o);
-        const VecT mv = *reinterpret_cast<const VecT*>(ms + o);
-        const VecT xw = *reinterpret_cast<const VecT*>(xs + o);
-        const T* pa = reinterpret_cast<const T*>(&pv);
-        const T* ma = reinterpret_cast<const T*>(&mv);
-        const T* xa = reinterpret_cast<const T*>(&xw);
-        VecT rv{};
-        if (MODE == 3) rv = *reinterpret_cast<const VecT*>(rs + o);
-        const T* ra = reinterpret_cast<const T*>(&rv);
+      if (!use[q]) continue;
+      const T* a = src + sbase(q);
+      const VecT po = *reinterpret_cast<const VecT*>(a);
+      const VecT mv = *reinterpret_cast<const VecT*>(a + PLANE);
+      const T* pa = reinterpret_cast<const T*>(&po);
+      const T* ma = reinterpret_cast<const T*>(&mv);
+      VecT rv{};
+      if (MODE == 3) rv = *reinterpret_cast<const VecT*>(a + 3 * PLANE);
+      const T* ra = reinterpret_cast<const T*>(&rv);
+      T pnew[W];
 #pragma unroll
-        for (int t = 0; t < V; ++t) {
-          pnew[t] = (MODE == 4 ? ma[t] : ma[t] * ra[t]) + beta_old * pa[t];
-          xv[t] = xa[t] + alpha_old * pa[t];
-        }
-      }
-      *reinterpret_cast<VecT*>(ps + o) = *reinterpret_cast<const VecT*>(pnew);
-      if (!kown || !((own_rows >> q) & 1u)) continue;
-      const int64_t s = ob - (ob & (V - 1)) + ccv[q];
-      const int64_t lo = ob + 3, hi = lo + own_len;
-      if (s >= lo && s + V <= hi) {
-        *reinterpret_cast<VecT*>(A.pout + s) = *reinterpret_cast<const VecT*>(pnew);
-        *reinterpret_cast<VecT*>(A.x + s) = *reinterpret_cast<const VecT*>(xv);
-      } else if (s + V > lo && s < hi) {
+      for (int t = 0; t < W; ++t) pnew[t] = (MODE == 4 ? ma[t] : ma[t] * ra[t]) + beta_old * pa[t];
+      *reinterpret_cast<VecT*>(pd + sbase(q)) = *reinterpret_cast<const VecT*>(pnew);
+      if (!kown || !own[q]) continue;
+      const VecT xw = *reinterpret_cast<const VecT*>(a + 2 * PLANE);
+      const T* xa = reinterpret_cast<const T*>(&xw);
+      T xv[W];
 #pragma unroll
-        for (int t = 0; t < V; ++t)
-          if (s + t >= lo && s + t < hi) {
-            A.pout[s + t] = pnew[t];
-            A.x[s + t] = xv[t];
+      for (int t = 0; t < W; ++t) xv[t] = xa[t] + alpha_old * pa[t];
+      const int off = chunk_off(q, pv);
+      T* pd2 = plane_ptr(A.pout, pv) + off;
+      T* xd = plane_ptr(A.x, pv) + off;
+      // the chunk's offset from the row's first owned value
+      const int d = dlo(q) - ((rof(q) + (int)(pv & (W - 1))) & (W - 1));
+      if (d >= 0 && d + W <= own_len) {
+        *reinterpret_cast<VecT*>(pd2) = *reinterpret_cast<const VecT*>(pnew);
+        *reinterpret_cast<VecT*>(xd) = *reinterpret_cast<const VecT*>(xv);
+      } else if (d + W > 0 && d < own_len) {
+#pragma unroll
+        for (int t = 0; t < W; ++t)
+          if (d + t >= 0 && d + t < own_len) {
+            pd2[t] = pnew[t];
+            xd[t] = xv[t];
           }
       }
     }
   };
 
-  // Shared-memory offsets of this thread's nodes (lx, ly) and (lx, ly + 1)
-  // in a plane: row start + the row's lead in that plane (see Stage) + 3 lx.
-  // The leads of planes ke and ke + 1 advance by 3 nplane mod V per plane.
-  const int rowA = 3 * (jn * g.nxn + i0 - 1), rowB = rowA + 3 * g.nxn;
-  const int p3m = (int)(P3 & (V - 1));
-  int lA0 = (int)(((int64_t)(k0 - 1) * P3 + rowA) & (V - 1));
-  int lB0 = (int)(((int64_t)(k0 - 1) * P3 + rowB) & (V - 1));
-  int lA1 = (lA0 + p3m) & (V - 1), lB1 = (lB0 + p3m) & (V - 1);
-  const int baseA = ly * RS + 3 * lx, baseB = (ly + 1) * RS + 3 * lx;
-  // the four corners (bx + 2 by) of component c of the element face
-  auto face = [&](const T* ps, int a, int b, int c, T (&v)[4]) {
-    v[0] = ps[a + c];
-    v[1] = ps[a + 3 + c];
-    v[2] = ps[b + c];
-    v[3] = ps[b + 3 + c];
+  // This thread's element columns join nodes lx and lx + 1 of R + 1 node
+  // rows.  Row b of a plane whose first value has index pl (mod W) starts at
+  // b * RS + lead, lead = (pl + lead0[b]) mod W.
+  const int row0 = 3 * (jn * g.nxn + i0 - 1);
+  const int p3m = P3 & (W - 1);
+  unsigned lead0[R + 1];
+#pragma unroll
+  for (int b = 0; b <= R; ++b) lead0[b] = (unsigned)(row0 + 3 * b * g.nxn) & (W - 1);
+  const int basea = R * wy * RS + 3 * lx;
+  auto row_at = [&](int b, unsigned pl) {
+    return basea + b * RS + (int)((pl + lead0[b]) & (W - 1));
   };
-
-  // Ring slots: plane kp sits in slot (kp - k0 + 1) mod NP of the p ring
-  // and mod NR of the r / M^-1 / x ring.
-  // prologue: planes k0-1 .. k0+PF-3 requested (one group each); k0-1 and
-  // k0 staged and transformed; then k0+PF-2 into the r/M^-1/x slot of k0-1
+  // face coefficients P[c][sigma_x + 2 sigma_y] of the thread's elements from
+  // a staged plane
+  T ownn[R][3];  // KEEP: node values of the plane that `face` read last
+  auto face = [&](const T* ps, unsigned pl, V (&P)[3][4]) {
+    const T* a[R + 1];
 #pragma unroll
-  for (int d = 0; d <= PF - 2; ++d) issue(k0 - 1 + d, d, d % NR);
-  cp_async_wait<PF - 3>();
-  __syncthreads();
-  transform(k0 - 1, 0, 0);
-  transform(k0, 1, 1 % NR);
-  __syncthreads();
-  issue(k0 + PF - 2, PF - 1, (PF - 1) % NR);
-  // slots of iteration it = ke - k0 + 1: planes ke (c0), ke+1 (c1), ke+2
-  // (c2, r2: transformed), ke+PF (cm = slot of ke-1, r1: issued)
-  int c0 = 0, c1 = 1, c2 = 2, cm = NP - 1, r2 = 2 % NR, r1 = 1 % NR;
-  auto step = [](int v, int n) { return v + 1 == n ? 0 : v + 1; };
-  T Ytp[3][4];
+    for (int b = 0; b <= R; ++b) a[b] = ps + row_at(b, pl);
 #pragma unroll
-  for (int c = 0; c < 3; ++c)
+    for (int c = 0; c < 3; ++c) {
+      T s[R + 1], d[R + 1];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) Ytp[c][q] = T(0);
-  double dsum = 0.0;
-
-  // The element factor and the node mask are plain loads.  In FP32 both are
-  // fetched one plane ahead so that their latency overlaps a plane of work;
-  // in FP64 the extra live registers would spill (128-register bound), so
-  // they are loaded where they are used (so is the face carry below).
-  constexpr bool PREFETCH = sizeof(T) == 4;
-  auto load_fac = [&](int ke) -> T {
-    return (col_ok && ke >= 0 && ke < g.nze) ? A.fac[(int64_t)ke * eplane + (int64_t)jn * g.nxe + in]
-                                             : T(0);
-  };
-  auto load_mask = [&](int kn) -> unsigned {
-    if (!A.nmask || !out_ok || kn < k0 || kn >= k1) return 7u;
-    return A.nmask[(int64_t)kn * nplane + (int64_t)jn * g.nxn + in];
-  };
-  T f_next = PREFETCH ? load_fac(k0 - 1) : T(0);
-  unsigned m_next = PREFETCH ? load_mask(k0) : 7u;
-  // FP32 also carries each plane's face transform from the layer it tops to
-  // the layer it bottoms (the plane is not modified in between)
-  T Pcarry[3][4];
-#pragma unroll
-  for (int c = 0; c < 3; ++c)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) Pcarry[c][q] = T(0);
-
-  for (int ke = k0 - 1; ke < k1; ++ke) {
-    T f;
-    unsigned m_pre = 7u;
-    if (PREFETCH) {
-      f = f_next;
-      f_next = load_fac(ke + 1);
-      if (ke >= k0) {
-        m_pre = m_next;
-        m_next = load_mask(ke + 1);
+      for (int b = 0; b <= R; ++b) {
+        const T u = a[b][c], v = a[b][3 + c];
+        if (S::KEEP && b < R) ownn[b][c] = u;
+        s[b] = u + v;
+        d[b] = v - u;
       }
+      if constexpr (R == 2) {
+        P[c][0] = make_float2(s[0] + s[1], s[1] + s[2]);
+        P[c][1] = make_float2(d[0] + d[1], d[1] + d[2]);
+        P[c][2] = make_float2(s[1] - s[0], s[2] - s[1]);
+        P[c][3] = make_float2(d[1] - d[0], d[2] - d[1]);
+      } else {
+        P[c][0] = s[0] + s[1];
+        P[c][1] = d[0] + d[1];
+        P[c][2] = s[1] - s[0];
+        P[c][3] = d[1] - d[0];
+      }
+    }
+  };
+
+  // Element factors: columns outside the grid read one inside it and carry a
+  // zero scale.  Fetched one layer ahead of their use (a pointer that stays on
+  // the first and last layer; layers outside are not computed).
+  const int eplane = g.nxe * g.nye;
+  const int ie = min(max(in, 0), g.nxe - 1), je = min(max(jn, 0), g.nye - 1);
+  const T* fp = A.fac + ((int64_t)max(k0 - 1, 0) * eplane + je * g.nxe + ie);
+  const int fstep = R == 2 && jn + 1 < g.nye && jn >= 0 ? g.nxe : 0;
+  V fscale;
+  {
+    const bool cx = in >= 0 && in < g.nxe, cy = jn >= 0 && jn < g.nye;
+    if constexpr (R == 2) {
+      const bool cy1 = jn + 1 < g.nye;
+      const float2 un = CUBE ? unit_of(A.K) : make_float2(1.f, 1.f);
+      fscale = make_float2(cx && cy ? un.x : 0.f, cx && cy1 ? un.y : 0.f);
     } else {
-      f = load_fac(ke);
+      fscale = cx && cy ? (CUBE ? unit_of(A.K) : 1.0) : 0.0;
     }
-    cp_async_wait<PF - 3>();  // groups up to ke+2 complete
-    __syncthreads();  // A: planes ke, ke+1 ready; ke+2 landed; ke-1 and red consumed
-    if (ke + 2 <= k1) transform(ke + 2, c2, r2);
-    issue(ke + PF, cm, r1);  // into the slot of plane ke-1
+  }
+  auto load_fac = [&]() -> V {
+    if constexpr (R == 2)
+      return make_float2(fp[0], fp[fstep]);
+    else
+      return fp[0];
+  };
+  // Outputs and node masks: pointers that advance with the plane.  The fixed
+  // DOFs of q need no mask in the fused steps and none is applied to A x in
+  // the Chebyshev step: p and x are 0 there and so is M^-1, which every use
+  // of q and A x multiplies by or tests.
+  constexpr bool MASK = MODE == 0 || MODE == 1 || MODE == 6;
+  bool out_ok[R];
+#pragma unroll
+  for (int b = 0; b < R; ++b)
+    out_ok[b] = lx >= 1 && R * wy + b >= 1 && in < g.nxn && jn + b < g.nyn;
+  const int64_t first = (int64_t)k0 * nplane + jn * g.nxn + in;  // node of plane k0
+  const bool has_mask = MASK && A.nmask != nullptr;
+  const uint8_t* mp = has_mask ? A.nmask + first : nullptr;
+  T* qp = (MODE == 5 ? A.x : A.q) + 3 * first;
 
-    const T* pl0 = &sm.p[c0][0];
-    const T* pl1 = &sm.p[c1][0];
-    const int a0 = baseA + lA0, a1 = baseA + lA1, b1 = baseB + lB1;
-    T U[3][8];
+  double dsum = 0.0;
+  T rowS[R][3], ownp[R][3];  // plane ke: sums so far, node values
+  unsigned mk[R];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      T v[4], Pb[4], Pt[4];
-      if (PREFETCH && ke > k0 - 1) {  // this plane's face transform, from the layer below
-#pragma unroll
-        for (int q = 0; q < 4; ++q) Pb[q] = Pcarry[c][q];
-      } else {
-        face(pl0, a0, baseB + lB0, c, v);
-        face_fwd(v, Pb);
-      }
-      face(pl1, a1, b1, c, v);
-      face_fwd(v, Pt);
-      if constexpr (sizeof(T) == 4) {  // packed pairs: (q, q + 1)
-#pragma unroll
-        for (int q = 0; q < 4; q += 2) {
-          if (PREFETCH) {
-            Pcarry[c][q] = Pt[q];
-            Pcarry[c][q + 1] = Pt[q + 1];
-          }
-          const float2 b = make_float2(Pb[q], Pb[q + 1]), t = make_float2(Pt[q], Pt[q + 1]);
-          const float2 su = __fadd2_rn(b, t);
-          const float2 di = __ffma2_rn(make_float2(-1.f, -1.f), b, t);
-          U[c][q] = su.x;
-          U[c][q + 1] = su.y;
-          U[c][q + 4] = di.x;
-          U[c][q + 5] = di.y;
-        }
-      } else {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          if (PREFETCH) Pcarry[c][q] = Pt[q];
-          U[c][q] = Pb[q] + Pt[q];
-          U[c][q + 4] = Pt[q] - Pb[q];
-        }
-      }
+  for (int b = 0; b < R; ++b) mk[b] = 7u;
+  unsigned plo = (unsigned)((int64_t)(k0 - 1) * p3m) & (W - 1);  // pl of plane ke (then kn)
+  // Finishes node plane ke - 1 (owned): the neighbouring warp's partial,
+  // shift, mask, output.
+  const T wx = MODE == 5 ? T(1) + (use_xp || A.xprev_zero ? A.omega : T(0)) : T(0);
+  auto finish = [&](int par, const T* aux, unsigned pl) {
+    bool masked = false;
+    if (MASK && has_mask) {
+      unsigned all = 7u;
+      for (int b = 0; b < R; ++b) all &= mk[b];
+      masked = __any_sync(0xffffffffu, all != 7u);
     }
-    T rowS[3];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      T Y[8];
-      if (c == 0) lambda_row<T, 0>(A.K, U, Y);
-      else if (c == 1) lambda_row<T, 1>(A.K, U, Y);
-      else lambda_row<T, 2>(A.K, U, Y);
-      T F[4];
-      // bottom face: f (Y_s - Y_d) plus the layer below's top face; top
-      // face: f (Y_s + Y_d), carried to the layer above.  FP32 forms the sum
-      // and difference first and works in packed pairs (q, q + 1); in FP64
-      // that order needs more live registers than the 128-register bound.
-      if constexpr (sizeof(T) == 4) {
-        const float2 f2 = make_float2(f, f);
-#pragma unroll
-        for (int q = 0; q < 4; q += 2) {
-          const float2 ys = make_float2(Y[q], Y[q + 1]), yd = make_float2(Y[q + 4], Y[q + 5]);
-          const float2 di = __ffma2_rn(make_float2(-1.f, -1.f), yd, ys);
-          const float2 Fq = __ffma2_rn(f2, di, make_float2(Ytp[c][q], Ytp[c][q + 1]));
-          const float2 nt = __fmul2_rn(f2, __fadd2_rn(ys, yd));
-          F[q] = Fq.x;
-          F[q + 1] = Fq.y;
-          Ytp[c][q] = nt.x;
-          Ytp[c][q + 1] = nt.y;
-        }
-      } else {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const T ys = Y[q] * f, yd = Y[q + 4] * f;
-          F[q] = (ys - yd) + Ytp[c][q];
-          Ytp[c][q] = ys + yd;
-        }
-      }
-      const T as = F[0] - F[2], ad = F[1] - F[3], bs = F[0] + F[2], bd = F[1] + F[3];
-      const T c0 = as - ad, c1 = as + ad, c2 = bs - bd, c3 = bs + bd;
-      // element lx-1 contributes its +x corners to this thread's nodes
-      const T l1 = __shfl_up_sync(0xffffffffu, c1, 1);
-      const T l3 = __shfl_up_sync(0xffffffffu, c3, 1);
-      rowS[c] = c0 + l1;
-      sm.red[ly][c][lx] = c2 + l3;
-    }
-    __syncthreads();  // B: red of this layer visible
-    if (ke >= k0 && out_ok) {
-      // this node's p.q in T (3 terms), accumulated in FP64 across planes
-      T pdot = T(0);
-      const int64_t node = (int64_t)ke * nplane + (int64_t)jn * g.nxn + in;
-      const unsigned m = PREFETCH ? m_pre : (A.nmask ? A.nmask[node] : 7u);
-      const T* own = pl0 + a0;
+    for (int b = 0; b < R; ++b) {
+      T pdot = T(0);  // this node's p.q in T (3 terms), accumulated in FP64
+      T o[3];
+      const T* ax = (MODE == 5 || MODE == 6) ? aux + row_at(b, pl) : nullptr;
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        T v = rowS[c] + sm.red[ly - 1][c][lx];
-        const T xv = own[c];
-        const bool fr = (m >> c) & 1u;
-        v = fr ? v + A.shift * xv : T(0);
-        const int64_t dof = 3 * node + c;
+        T v = rowS[b][c];
+        if (b == 0) v += sm.red[par][wy][c][lx];
+        const T xv = ownp[b][c];
+        v = fma(A.shift, xv, v);
         if (MODE == 5) {
           // x_prev: read, or 0 (the step after a start from x = 0), or
           // unused (the first step: omega = 0)
-          const T xp = A.xprev_zero ? T(0) : (A.omega != T(0) ? A.x[dof] : xv);
-          A.x[dof] = fr ? xv + A.omega * (xv - xp) + A.gamma * A.minv[dof] * (A.r[dof] - v)
-                        : T(0);
+          v = fma(A.gamma * ax[PLANE + c], ax[c] - v, wx * xv);
+          if (use_xp) v = fma(-A.omega, ax[2 * PLANE + c], v);
         } else if (MODE == 6) {
-          A.q[dof] = fr ? A.r[dof] - v : T(0);
-        } else {
-          A.q[dof] = v;
+          v = ax[c] - v;
         }
+        o[c] = v;
         if (DOT) pdot = fma(xv, v, pdot);
       }
-      if (DOT) dsum += (double)pdot;
+      if (MASK && masked)
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          if (!((mk[b] >> c) & 1u)) o[c] = T(0);
+      if (out_ok[b]) {
+        T* d = qp + 3 * b * g.nxn;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) d[c] = o[c];
+        if (DOT) dsum += (double)pdot;
+      }
     }
-    c0 = step(c0, NP);
-    c1 = step(c1, NP);
-    c2 = step(c2, NP);
-    cm = step(cm, NP);
-    r2 = step(r2, NR);
-    r1 = step(r1, NR);
-    lA0 = lA1;
-    lB0 = lB1;
-    lA1 = (lA1 + p3m) & (V - 1);
-    lB1 = (lB1 + p3m) & (V - 1);
-  }
+    qp += P3;
+  };
 
-  if (MODE == 4) {
-    double v[1] = {dsum};
-    if (grid_reduce<1>(v, A.partials, &A.st->ticket[TK_MATVEC]) && tid == 0) {
-      const double pq = v[0], zr = A.st->aux[3];
-      A.st->pq = pq;
-      if (!(pq > 0.0) || !isfinite(pq) || !isfinite(zr))
-        A.st->status = HX_ST_BREAKDOWN;
-      else
-        A.st->alpha = zr / pq;
+  const V m1 = from_shared<V>(&sm.k[4]);
+  CoefV<V, CUBE> K = A.K;
+  pin_coef(K, sm.k);
+  V Ytp[3][4], Pb[3][4];
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) Ytp[c][q] = Pb[c][q] = vzero<V>();
+
+  // Prologue: the first planes requested; planes k0-1 and k0 ready, the face
+  // coefficients of plane k0-1 formed.  Slots: plane kp of p in slot (kp -
+  // k0 + 1) mod NX, of the fused inputs mod NS; aux plane kp in (kp - k0) mod
+  // NA.  One commit group per call of issue, so that the wait counts hold to
+  // the end of the chunk.
+  auto step = [](int v, int n) { return v + 1 == n ? 0 : v + 1; };
+  int sp = 0, sa = 0;  // fused: slot of plane ke + 2; else of plane ke, of aux plane ke + 1
+  if constexpr (FUSED) {
+#pragma unroll 1
+    for (int d = 0; d < S::NS; ++d) {
+      issue(k0 - 1 + d, &sm.in[d][0][0]);
+      cp_async_commit();
     }
-  } else if (DOT) {
+#pragma unroll 1
+    for (int d = 0; d < 2; ++d) {
+      cp_async_wait<S::NS - 1>();
+      transform(k0 - 1 + d, &sm.in[d][0][0], sm.p[d]);
+      issue(k0 - 1 + d + S::NS, &sm.in[d][0][0]);
+      cp_async_commit();
+    }
+    sp = 2 % S::NS;
+    __syncthreads();
+  } else {
+#pragma unroll 1
+    for (int d = 0; d < S::NX - 1; ++d) {
+      issue(k0 - 1 + d, sm.p[d]);
+      cp_async_commit();
+    }
+    cp_async_wait<S::NX - 2>();
+    __syncthreads();
+  }
+#pragma unroll
+  for (int b = 0; b < R; ++b)
+#pragma unroll
+    for (int c = 0; c < 3; ++c) ownn[b][c] = T(0);
+  if (k0 > 0) face(sm.p[0], plo, Pb);
+  V f_next = load_fac();
+  int s0 = 0;  // slot of plane ke
+
+#pragma unroll 1
+  for (int ke = k0 - 1; ke < k1; ++ke) {
+    const V f = vmul(f_next, fscale);
+    fp += ke >= 0 && ke + 1 < g.nze ? eplane : 0;
+    f_next = load_fac();
+    const int s1 = step(s0, S::NX), s2 = step(s1, S::NX);
+    if constexpr (!FUSED) cp_async_wait<(S::AUX ? 1 : S::NX - 3)>();
+    __syncthreads();  // plane ke+1 ready; red of plane ke-1 visible; plane ke-1 consumed
+    if (ke - 1 >= k0)
+      finish((ke - 1) & 1, &sm.in[S::AUX ? step(sa, S::NA) : 0][0][0], plo - p3m);
+    if constexpr (!FUSED) {
+      issue(ke - 1 + S::NX, sm.p[sp == 0 ? S::NX - 1 : sp - 1]);
+      if (S::AUX) {
+        issue_aux(ke - 2 + S::NA, &sm.in[sa][0][0]);
+        sa = step(sa, S::NA);
+      }
+      cp_async_commit();
+      sp = step(sp, S::NX);
+    } else {
+      cp_async_wait<S::NS - 1>();
+      transform(ke + 2, &sm.in[sp][0][0], sm.p[s2]);
+      issue(ke + 2 + S::NS, &sm.in[sp][0][0]);
+      cp_async_commit();
+      sp = step(sp, S::NS);
+    }
+    if (has_mask && ke >= k0) {
+#pragma unroll
+      for (int b = 0; b < R; ++b)
+        if (out_ok[b]) mk[b] = mp[b * g.nxn];
+      mp += nplane;
+    }
+
+    if constexpr (S::KEEP) {
+#pragma unroll
+      for (int b = 0; b < R; ++b)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) ownp[b][c] = ownn[b][c];
+    }
+
+    // Element layer ke: bottom face f (Y_s - Y_d) plus the layer below's top
+    // face; top face f (Y_s + Y_d), carried to the layer above.
+    V F[3][4];
+    if (ke >= 0 && ke < g.nze) {
+      V Pt[3][4];
+      face(sm.p[s1], plo + p3m, Pt);
+      const V nf = vneg(f);
+      auto blocks = [&](auto qc) {
+        constexpr int Q = decltype(qc)::value;
+        constexpr int e[3] = {Q ^ 1, Q ^ 2, Q};
+        V s[3], d[3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          if (e[c] != 0) s[c] = vadd(Pb[c][e[c]], Pt[c][e[c]]);
+          else s[c] = vzero<V>();
+          d[c] = vsubm(Pt[c][e[c]], Pb[c][e[c]], m1);
+        }
+        lambda_pair<Q>(K, s, d);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          V& y = Ytp[c][e[c]];
+          if (e[c] == 0) {
+            F[c][0] = vfma(nf, d[c], y);
+            y = vmul(f, d[c]);
+          } else {
+            F[c][e[c]] = vfma(nf, d[c], vfma(f, s[c], y));
+            y = vfma(f, d[c], vmul(f, s[c]));
+          }
+        }
+      };
+      blocks(std::integral_constant<int, 0>{});
+      blocks(std::integral_constant<int, 1>{});
+      blocks(std::integral_constant<int, 2>{});
+      blocks(std::integral_constant<int, 3>{});
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) Pb[c][q] = Pt[c][q];
+    } else {
+      // no elements below the first and above the last node plane
+      if (ke < 0) face(sm.p[s1], plo + p3m, Pb);
+#pragma unroll
+      for (int c = 0; c < 3; ++c)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) F[c][q] = Ytp[c][q];
+    }
+    // y and x transforms back to the R + 1 node rows
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const V as = vsubm(F[c][0], F[c][2], m1), ad = vsubm(F[c][1], F[c][3], m1);
+      const V bs = vadd(F[c][0], F[c][2]), bd = vadd(F[c][1], F[c][3]);
+      T s[R + 1], d[R + 1];
+      if constexpr (R == 2) {
+        s[0] = as.x;
+        d[0] = ad.x;
+        s[1] = bs.x + as.y;
+        d[1] = bd.x + ad.y;
+        s[2] = bs.y;
+        d[2] = bd.y;
+      } else {
+        s[0] = as;
+        d[0] = ad;
+        s[1] = bs;
+        d[1] = bd;
+      }
+#pragma unroll
+      for (int b = 0; b <= R; ++b) {
+        const T left = s[b] - d[b], right = s[b] + d[b];
+        // element lx-1 contributes its +x corners to this thread's nodes
+        const T t = left + __shfl_up_sync(0xffffffffu, right, 1);
+        if (b < R)
+          rowS[b][c] = t;
+        else if (wy + 1 < WARPS)
+          sm.red[ke & 1][wy + 1][c][lx] = t;
+      }
+    }
+    if constexpr (!S::KEEP) {  // the node values of plane ke: its slot lives until the next barrier
+#pragma unroll
+      for (int b = 0; b < R; ++b) {
+        const T* a = sm.p[s0] + row_at(b, plo);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) ownp[b][c] = a[c];
+      }
+    }
+    s0 = s1;
+    plo += p3m;
+  }
+  cp_async_wait<0>();
+  __syncthreads();  // red of plane k1-1 visible
+  finish((k1 - 1) & 1, &sm.in[S::AUX ? step(sa, S::NA) : 0][0][0], plo - p3m);
+
+  if (DOT) {
     double v[1] = {dsum};
     if (grid_reduce<1>(v, A.partials, &A.st->ticket[TK_MATVEC]) && tid == 0) {
       if (MODE == 1) {
         A.out[0] = v[0];
       } else {
-        const double pq = v[0];
+        const double pq = v[0], num = MODE == 4 ? A.st->aux[3] : A.st->rz;
         A.st->pq = pq;
-        if (!(pq > 0.0) || !isfinite(pq))
+        if (!(pq > 0.0) || !isfinite(pq) || (MODE == 4 && !isfinite(num)))
           A.st->status = HX_ST_BREAKDOWN;
         else
-          A.st->alpha = A.st->rz / pq;
+          A.st->alpha = num / pq;
       }
     }
   }
@@ -604,36 +924,17 @@ __global__ void k_minv(const uint8_t* __restrict__ nmask, const T* __restrict__ 
   }
 }
 
-inline dim3 mv_grid(const Grid& g, int kchunk) {
-  return dim3(cdiv(g.nxn, MV_BX - 1), cdiv(g.nyn, MV_BY - 1), cdiv(g.nzn, kchunk));
-}
-
-template <typename T, int MODE>
-void launch_struct(cudaStream_t s, const OpArgs<T>& a) {
-  constexpr bool FUSED = MODE == 3 || MODE == 4;
-  constexpr int MINB = mv_resident<T>();
-  const size_t smem = sizeof(OpSmem<T, MV_BY, FUSED>);
-  static PerDeviceOnce configured;  // per instantiation and device
-  configured.run([&] {
-    HX_CUDA(cudaFuncSetAttribute(k_struct<T, MV_BY, MODE, MINB>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  });
-  k_struct<T, MV_BY, MODE, MINB><<<mv_grid(a.g, a.kchunk), dim3(MV_BX, MV_BY), smem, s>>>(a);
-  HX_CHECK_LAUNCH();
-}
-
-}  // namespace
-
-int mv_kchunk(const Grid& g, int resident) {
-  // Node planes per CTA: the chunk length kc (at least 8, so the two staged
-  // halo planes stay a small share) that minimises (waves of resident CTAs)
-  // x (planes each CTA stages, kc + 2).  A last wave that fills few SMs
-  // costs as much as a full one; ties go to the longer chunk.
-  const int64_t cols = (int64_t)cdiv(g.nxn, MV_BX - 1) * cdiv(g.nyn, MV_BY - 1);
-  const int64_t slots = (int64_t)resident * sm_count();
+// Node planes per CTA: the chunk length kc that minimises (waves of resident
+// CTAs) x (element layers each CTA works on, kc + 1, and one for its start and
+// end).  A last wave that fills few SMs costs as much as a full one; ties go
+// to the longer chunk.  Short chunks win only where the grid leaves SMs idle.
+template <typename T, bool FUSED>
+int mv_kchunk(const Grid& g) {
+  const int64_t cols = (int64_t)cdiv(g.nxn, MV_BX - 1) * cdiv(g.nyn, mv_by<T, FUSED>() - 1);
+  const int64_t slots = (int64_t)Tile<T, FUSED>::RESIDENT * sm_count();
   int best_kc = g.nzn;
   int64_t best = INT64_MAX;
-  for (int kc = std::min(8, g.nzn); kc <= g.nzn; ++kc) {
+  for (int kc = 1; kc <= g.nzn; ++kc) {
     const int64_t waves = cdiv(cols * cdiv(g.nzn, kc), slots);
     const int64_t cost = waves * (kc + 2);
     if (cost <= best) {
@@ -644,58 +945,94 @@ int mv_kchunk(const Grid& g, int resident) {
   return best_kc;
 }
 
-size_t mv_num_blocks(const Grid& g, int resident) {
-  const dim3 gr = mv_grid(g, mv_kchunk(g, resident));
-  return (size_t)gr.x * gr.y * gr.z;
+template <typename T, bool FUSED>
+dim3 mv_grid(const Grid& g, int kchunk) {
+  return dim3(cdiv(g.nxn, MV_BX - 1), cdiv(g.nyn, mv_by<T, FUSED>() - 1), cdiv(g.nzn, kchunk));
 }
 
-size_t mv_max_blocks(const Grid& g) {
-  return std::max(mv_num_blocks(g, mv_resident<float>()), mv_num_blocks(g, mv_resident<double>()));
+template <typename T, int MODE, bool CUBE>
+void launch_one(cudaStream_t s, OpArgs<T, CUBE>& a, const ElemCoef<T>& K) {
+  constexpr size_t smem = sizeof(Smem<T, MODE>);
+  static_assert(smem % 16 == 0, "zeroed in 16-byte steps");
+  constexpr bool FUSED = mode_fused(MODE);
+  using Form = Tile<T, FUSED>;
+  static_assert(Form::RESIDENT * (smem + 1024 + 512) <= 228 * 1024, "the CTAs of an SM fit");
+  static PerDeviceOnce configured;  // per instantiation and device
+  configured.run([&] {
+    HX_CUDA(cudaFuncSetAttribute(k_struct<T, MODE, CUBE>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  });
+  coef_v(K, a.K);
+  a.kchunk = mv_kchunk<T, FUSED>(a.g);
+  k_struct<T, MODE, CUBE>
+      <<<mv_grid<T, FUSED>(a.g, a.kchunk), dim3(MV_BX, Form::WARPS), smem, s>>>(a);
+  HX_CHECK_LAUNCH();
 }
+
+// `fill` sets the mode's fields of the arguments.
+template <typename T, int MODE, typename F>
+void launch_struct(cudaStream_t s, const T* fac, const uint8_t* nmask, const Grid& g,
+                   const ElemCoef<T>& K, T shift, F&& fill) {
+  auto go = [&](auto cube) {
+    OpArgs<T, decltype(cube)::value> a{};
+    a.fac = fac;
+    a.nmask = nmask;
+    a.g = g;
+    a.shift = shift;
+    fill(a);
+    launch_one<T, MODE>(s, a, K);
+  };
+  // equal sides: every axis has the same coefficients
+  if (K.mu[0][0] == K.mu[1][0] && K.mu[1][0] == K.mu[2][0])
+    go(std::true_type{});
+  else
+    go(std::false_type{});
+}
+
+}  // namespace
+
+template <typename T>
+size_t mv_num_blocks(const Grid& g) {
+  const dim3 a = mv_grid<T, true>(g, mv_kchunk<T, true>(g));
+  const dim3 b = mv_grid<T, false>(g, mv_kchunk<T, false>(g));
+  return std::max((size_t)a.x * a.y * a.z, (size_t)b.x * b.y * b.z);
+}
+template size_t mv_num_blocks<float>(const Grid&);
+template size_t mv_num_blocks<double>(const Grid&);
 
 template <typename T>
 void launch_matvec(cudaStream_t s, int mode, const T* x, T* y, const T* fac, const uint8_t* nmask,
                    const Grid& g, const ElemCoef<T>& K, T shift, CgState* st, double* partials,
                    double* out) {
-  OpArgs<T> a{};
-  a.pin = x;
-  a.q = y;
-  a.fac = fac;
-  a.nmask = nmask;
-  a.g = g;
-  a.kchunk = mv_kchunk(g, mv_resident<T>());
-  a.K = K;
-  a.shift = shift;
-  a.st = st;
-  a.partials = partials;
-  a.out = out;
+  auto fill = [&](auto& a) {
+    a.pin = x;
+    a.q = y;
+    a.st = st;
+    a.partials = partials;
+    a.out = out;
+  };
   if (mode == 0)
-    launch_struct<T, 0>(s, a);
-  else if (mode == 1)
-    launch_struct<T, 1>(s, a);
+    launch_struct<T, 0>(s, fac, nmask, g, K, shift, fill);
   else
-    launch_struct<T, 2>(s, a);
+    launch_struct<T, 1>(s, fac, nmask, g, K, shift, fill);
 }
+template void launch_matvec<double>(cudaStream_t, int, const double*, double*, const double*,
+                                    const uint8_t*, const Grid&, const ElemCoef<double>&, double,
+                                    CgState*, double*, double*);
 
 template <typename T>
 void launch_cheb_step(cudaStream_t s, const T* x, T* xprev_new, bool xprev_zero, const T* b,
                       const T* minv, T omega, T gamma, const T* fac, const uint8_t* nmask,
                       const Grid& g, const ElemCoef<T>& K, T shift) {
-  OpArgs<T> a{};
-  a.pin = x;
-  a.x = xprev_new;
-  a.xprev_zero = xprev_zero ? 1 : 0;
-  a.r = b;
-  a.minv = minv;
-  a.omega = omega;
-  a.gamma = gamma;
-  a.fac = fac;
-  a.nmask = nmask;
-  a.g = g;
-  a.kchunk = mv_kchunk(g, mv_resident<T>());
-  a.K = K;
-  a.shift = shift;
-  launch_struct<T, 5>(s, a);
+  launch_struct<T, 5>(s, fac, nmask, g, K, shift, [&](auto& a) {
+    a.pin = x;
+    a.x = xprev_new;
+    a.xprev_zero = xprev_zero ? 1 : 0;
+    a.r = b;
+    a.minv = minv;
+    a.omega = omega;
+    a.gamma = gamma;
+  });
 }
 template void launch_cheb_step<float>(cudaStream_t, const float*, float*, bool, const float*,
                                       const float*, float, float, const float*, const uint8_t*,
@@ -704,17 +1041,11 @@ template void launch_cheb_step<float>(cudaStream_t, const float*, float*, bool, 
 template <typename T>
 void launch_residual(cudaStream_t s, const T* x, const T* b, T* r, const T* fac,
                      const uint8_t* nmask, const Grid& g, const ElemCoef<T>& K, T shift) {
-  OpArgs<T> a{};
-  a.pin = x;
-  a.r = b;
-  a.q = r;
-  a.fac = fac;
-  a.nmask = nmask;
-  a.g = g;
-  a.kchunk = mv_kchunk(g, mv_resident<T>());
-  a.K = K;
-  a.shift = shift;
-  launch_struct<T, 6>(s, a);
+  launch_struct<T, 6>(s, fac, nmask, g, K, shift, [&](auto& a) {
+    a.pin = x;
+    a.r = b;
+    a.q = r;
+  });
 }
 template void launch_residual<float>(cudaStream_t, const float*, const float*, float*,
                                      const float*, const uint8_t*, const Grid&,
@@ -724,58 +1055,17 @@ template <typename T>
 void launch_pcg_step(cudaStream_t s, const T* pin, T* pout, const T* r, const T* minv, T* x, T* q,
                      const T* fac, const uint8_t* nmask, const Grid& g, const ElemCoef<T>& K,
                      T shift, CgState* st, double* partials) {
-  OpArgs<T> a{};
-  a.pin = pin;
-  a.pout = pout;
-  a.r = r;
-  a.minv = minv;
-  a.x = x;
-  a.q = q;
-  a.fac = fac;
-  a.nmask = nmask;
-  a.g = g;
-  a.kchunk = mv_kchunk(g, mv_resident<T>());
-  a.K = K;
-  a.shift = shift;
-  a.st = st;
-  a.partials = partials;
-  launch_struct<T, 3>(s, a);
+  launch_struct<T, 3>(s, fac, nmask, g, K, shift, [&](auto& a) {
+    a.pin = pin;
+    a.pout = pout;
+    a.r = r;
+    a.minv = minv;
+    a.x = x;
+    a.q = q;
+    a.st = st;
+    a.partials = partials;
+  });
 }
-
-template <typename T>
-void launch_fcg_step(cudaStream_t s, const T* pin, T* pout, const T* z, T* x, T* q, const T* fac,
-                     const uint8_t* nmask, const Grid& g, const ElemCoef<T>& K, T shift,
-                     CgState* st, double* partials) {
-  OpArgs<T> a{};
-  a.pin = pin;
-  a.pout = pout;
-  a.minv = z;
-  a.x = x;
-  a.q = q;
-  a.fac = fac;
-  a.nmask = nmask;
-  a.g = g;
-  a.kchunk = mv_kchunk(g, mv_resident<T>());
-  a.K = K;
-  a.shift = shift;
-  a.st = st;
-  a.partials = partials;
-  launch_struct<T, 4>(s, a);
-}
-template void launch_fcg_step<double>(cudaStream_t, const double*, double*, const double*,
-                                      double*, double*, const double*, const uint8_t*,
-                                      const Grid&, const ElemCoef<double>&, double, CgState*,
-                                      double*);
-template void launch_fcg_step<float>(cudaStream_t, const float*, float*, const float*, float*,
-                                     float*, const float*, const uint8_t*, const Grid&,
-                                     const ElemCoef<float>&, float, CgState*, double*);
-
-template void launch_matvec<double>(cudaStream_t, int, const double*, double*, const double*,
-                                    const uint8_t*, const Grid&, const ElemCoef<double>&, double,
-                                    CgState*, double*, double*);
-template void launch_matvec<float>(cudaStream_t, int, const float*, float*, const float*,
-                                   const uint8_t*, const Grid&, const ElemCoef<float>&, float,
-                                   CgState*, double*, double*);
 template void launch_pcg_step<double>(cudaStream_t, const double*, double*, const double*,
                                       const double*, double*, double*, const double*,
                                       const uint8_t*, const Grid&, const ElemCoef<double>&,
@@ -784,6 +1074,28 @@ template void launch_pcg_step<float>(cudaStream_t, const float*, float*, const f
                                      const float*, float*, float*, const float*, const uint8_t*,
                                      const Grid&, const ElemCoef<float>&, float, CgState*,
                                      double*);
+
+template <typename T>
+void launch_fcg_step(cudaStream_t s, const T* pin, T* pout, const T* z, T* x, T* q, const T* fac,
+                     const uint8_t* nmask, const Grid& g, const ElemCoef<T>& K, T shift,
+                     CgState* st, double* partials) {
+  launch_struct<T, 4>(s, fac, nmask, g, K, shift, [&](auto& a) {
+    a.pin = pin;
+    a.pout = pout;
+    a.minv = z;
+    a.x = x;
+    a.q = q;
+    a.st = st;
+    a.partials = partials;
+  });
+}
+template void launch_fcg_step<double>(cudaStream_t, const double*, double*, const double*,
+                                      double*, double*, const double*, const uint8_t*,
+                                      const Grid&, const ElemCoef<double>&, double, CgState*,
+                                      double*);
+template void launch_fcg_step<float>(cudaStream_t, const float*, float*, const float*, float*,
+                                     float*, const float*, const uint8_t*, const Grid&,
+                                     const ElemCoef<float>&, float, CgState*, double*);
 
 template <typename T>
 void launch_node_diag(cudaStream_t s, const T* fac, const uint8_t* bcfree, uint8_t* nmask, T* diag,

@@ -68,6 +68,7 @@ ElemCoef<double> make_elem_coef(double dx, double dy, double dz, double nu) {
       K.lam[k][sk] = lam * m(k, sk) / 8.0;
       K.mu[k][sk] = mu * m(k, sk) / 8.0;
     }
+  K.rho = lam / mu;
   return K;
 }
 
@@ -81,6 +82,7 @@ ElemCoef<float> to_float(const ElemCoef<double>& k) {
     }
     f.kd[c] = (float)k.kd[c];
   }
+  f.rho = k.rho;
   return f;
 }
 
@@ -95,7 +97,8 @@ static double now_ms() {
 void ensure_workspace(hx_ctx* c) {
   if (!c->h_state) HX_CUDA(cudaMallocHost(&c->h_state, 4 * sizeof(CgState)));
   c->d_state.ensure(4);
-  const size_t nb = std::max<size_t>(mv_max_blocks(c->g), 64ull * sm_count());
+  const size_t nb = std::max<size_t>(
+      std::max(mv_num_blocks<float>(c->g), mv_num_blocks<double>(c->g)), 64ull * sm_count());
   c->d_partials.ensure(4 * nb);
   c->d_scalars.ensure(16);
 }
@@ -264,10 +267,6 @@ template CgState pcg_fused<double>(hx_ctx*, int, const double*, const double*, d
                                    double, const ElemCoef<double>&, double*, double*, double*,
                                    double*, const double*, double*, const CgState&, int, double,
                                    double, bool*);
-template CgState pcg_fused<float>(hx_ctx*, int, const float*, const float*, float*, bool, float,
-                                  const ElemCoef<float>&, float*, float*, float*, float*,
-                                  const float*, float*, const CgState&, int, double, double,
-                                  bool*);
 
 static CgState pcg_fp64(hx_ctx* c, const double* fac, const double* b, double* x, bool warm,
                         double shift, const hx_solve_opts& o, double t0, bool* timed_out) {

@@ -52,6 +52,11 @@ struct Vec16<float> {
   __device__ static float4 make(const float (&a)[4]) { return make_float4(a[0], a[1], a[2], a[3]); }
 };
 
+// M^-1 entry of a free DOF (the fixed ones' is 0); the integer test of the
+// upper half keeps FP64 comparisons off the FP64 pipe
+__device__ __forceinline__ bool is_free(double m) { return __double2hiint(m) != 0; }
+__device__ __forceinline__ bool is_free(float m) { return m != 0.f; }
+
 __device__ __forceinline__ uint32_t bf16x2_bits(float a, float b) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&h);
@@ -174,7 +179,8 @@ __global__ void k_cg_update(T* __restrict__ x, const T* __restrict__ p, T* __res
     cg_finish_iteration(st, v[0], v[1]);
 }
 
-// Second half of a fused PCG iteration: r -= alpha q, dots, tests.  With
+// Second half of a fused PCG iteration: r -= alpha q on the free DOFs (M^-1
+// is 0 on the fixed ones, where the operator leaves q unmasked), dots, tests.  With
 // ys: also ys = BF16(D^-1/2 r) of the new residual (the learned
 // preconditioner's input, D^-1/2 = sqrt(minv)).  16-byte vector accesses
 // (4 FP32 or 2 FP64 entries per thread and step), then a scalar tail.
@@ -200,7 +206,7 @@ __global__ void k_cg_update2(T* __restrict__ r, const T* __restrict__ q,
     float ya[W];
 #pragma unroll
     for (int e = 0; e < W; ++e) {
-      ra[e] -= alpha * qa[e];
+      ra[e] = is_free(ma[e]) ? ra[e] - alpha * qa[e] : T(0);
       ya[e] = dinv_sqrt((float)ma[e]) * (float)ra[e];
       rz += (double)ra[e] * (double)(ma[e] * ra[e]);
       rr += (double)ra[e] * (double)ra[e];
@@ -215,7 +221,7 @@ __global__ void k_cg_update2(T* __restrict__ r, const T* __restrict__ q,
     }
   }
   for (int64_t i = nv * W + gtid(); i < n; i += gstride()) {
-    const T ri = r[i] - alpha * q[i];
+    const T ri = is_free(minv[i]) ? r[i] - alpha * q[i] : T(0);
     r[i] = ri;
     if (ys) ys[i] = __float2bfloat16_rn(dinv_sqrt((float)minv[i]) * (float)ri);
     rz += (double)ri * (double)(minv[i] * ri);
