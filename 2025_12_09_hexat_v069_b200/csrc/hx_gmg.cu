@@ -705,8 +705,8 @@ CgState solve_gmg(hx_ctx* c, const double* fac, const double* b, double* x, bool
   // a multigrid solve takes tens of iterations and the V-cycle's kernels run
   // whole even after the state has stopped: two iterations per graph launch
   // waste at most one cycle
-  const int reps = 1;
-  CgState sf = run_batched(c, 0, reps, body, o.wall_limit_ms, t0, timed_out, 0);
+  GraphLoop loop(c, 0, 1, body);
+  CgState sf = loop.run(false, o.wall_limit_ms, t0, timed_out);
   if (sf.status != HX_ST_BREAKDOWN && sf.iter > 0) {
     double* pk = ((sf.iter - 1) % 2 == 0) ? P0 : P1;
     launch_axpy_state<double>(c->stream, x, x, pk, n, st, 0);

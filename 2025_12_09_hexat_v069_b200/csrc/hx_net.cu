@@ -639,7 +639,6 @@ static CgState learned_fcg(hx_ctx* c, const double* fac, const double* b, double
     one(P1, P0);
     one(P0, P1);
   };
-  const int reps = std::max(1, auto_batch(g, o.check_every) / 2);
   double best = s0.rel_res;
   int best_it = 0;
   CgState sf{};
@@ -656,7 +655,8 @@ static CgState learned_fcg(hx_ctx* c, const double* fac, const double* b, double
     stalled = !o.learned_no_fallback && sv.iter - best_it > std::max(500, sv.iter / 4);
     return !stalled;
   };
-  sf = run_batched(c, 0, reps, body, o.wall_limit_ms, t0, timed_out, 0, keep_going);
+  GraphLoop loop(c, 0, 1, body);
+  sf = loop.run(true, o.wall_limit_ms, t0, timed_out, 0, keep_going);
   if (sf.status != HX_RUNNING) stalled = false;
   // pending x += alpha p of the last completed iteration
   if (sf.status != HX_ST_BREAKDOWN && sf.iter > 0) {
@@ -675,7 +675,7 @@ static CgState learned_fcg(hx_ctx* c, const double* fac, const double* b, double
   CgState sj = pcg_fused<double>(c, 0, fac, b, x, true, shift, c->K, r, P0, P1, q, minv, nullptr,
                                  fresh_state(o.tol, oj.max_iter, 1, o.divergence_checks != 0,
                                              false),
-                                 auto_batch(g, o.check_every), o.wall_limit_ms, t0, timed_out);
+                                 auto_batch(o.check_every), o.wall_limit_ms, t0, timed_out);
   *iters_out += sj.iter;
   return sj;
 }
@@ -776,36 +776,32 @@ static CgState learned_fcg_mixed(hx_ctx* c, const double* fac, const double* b, 
   st.aux[2] = st.rr;
   st.max_iter = o.max_iter;
   put_state(c, 1, st);
-  // the V-cycle's kernels run whole after the state has stopped: batches of
-  // two iterations for multigrid (tens of iterations per solve)
-  const int reps = multigrid ? 1 : std::max(1, auto_batch(g, o.check_every) / 2);
-  int parity = 0;  // which P buffer holds p_{k-1}: P1 when parity == 0
   double best = so_h.rel_res;
   int best_it = 0;
   bool stalled = false;
   CgState sf{};
   __nv_bfloat16* ys = multigrid ? nullptr : N.ys.ensure(n + 8);
+  auto one = [&](float* pi, float* po) {
+    if (multigrid) {
+      gmg_vcycle<float>(c, r32, z32);
+      launch_fcg_coeffs<float>(c->stream, z32, q32, r32, n, c->d_partials.p, si);
+    } else {
+      precond_z<float>(c, r32, minv32, si, scale_mul, z32, q32, false, ys);
+    }
+    launch_fcg_step<float>(c->stream, pi, po, z32, d32, q32, fac32, c->d_nmask.p, g, K32, sh32,
+                           si, c->d_partials.p);
+    launch_cg_update2<float>(c->stream, r32, q32, minv32, n, si, c->d_partials.p, ys);
+  };
+  // iterations alternate p from P1 to P0 and back.  Two iterations per launch:
+  // the preconditioner's kernels run whole after the state has stopped
+  GraphLoop loop(c, 1, 1, [&]() {
+    one(P1, P0);
+    one(P0, P1);
+  });
   for (;;) {
-    float* Pin = parity ? P0 : P1;
-    float* Pout = parity ? P1 : P0;
     // ys = BF16(D^-1/2 r32) of the (replaced) residual; then every residual
     // update keeps it current
     if (!multigrid) launch_dinv_bf16<float>(c->stream, r32, minv32, ys, n);
-    auto one = [&](float* pi, float* po) {
-      if (multigrid) {
-        gmg_vcycle<float>(c, r32, z32);
-        launch_fcg_coeffs<float>(c->stream, z32, q32, r32, n, c->d_partials.p, si);
-      } else {
-        precond_z<float>(c, r32, minv32, si, scale_mul, z32, q32, false, ys);
-      }
-      launch_fcg_step<float>(c->stream, pi, po, z32, d32, q32, fac32, c->d_nmask.p, g, K32,
-                             sh32, si, c->d_partials.p);
-      launch_cg_update2<float>(c->stream, r32, q32, minv32, n, si, c->d_partials.p, ys);
-    };
-    auto body = [&]() {
-      one(Pin, Pout);
-      one(Pout, Pin);
-    };
     // a batch ends on a reliable-update pause, convergence, failure, or
     // stagnation of the recursive residual (relative to ||b||, as the true
     // one) by the test of solve_learned
@@ -818,13 +814,14 @@ static CgState learned_fcg_mixed(hx_ctx* c, const double* fac, const double* b, 
       return !stalled;
     };
     const int it_before = st.iter;
-    sf = run_batched(c, 1, reps, body, o.wall_limit_ms, t0, timed_out, 0, keep_going);
+    sf = loop.run(!multigrid, o.wall_limit_ms, t0, timed_out, 0, keep_going);
     const int done = sf.iter - it_before;
     *iters_out += done;
-    float* pk = (done % 2 == 1) ? Pout : Pin;  // p of the last completed iteration
-    if (done % 2 == 1) parity ^= 1;
+    float* pk = (done % 2 == 1) ? P0 : P1;  // p of the last completed iteration
     if (sf.status != HX_ST_BREAKDOWN && done > 0)
       launch_axpy_state<float>(c->stream, d32, d32, pk, n, si, 0);  // pending step
+    if (pk == P0)  // the next iteration reads P1
+      HX_CUDA(cudaMemcpyAsync(P1, P0, n * sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
     // fold the FP32 correction into x and replace the residual in FP64
     launch_ir_correct(c->stream, x, d32, n, so);
     launch_fill_zero(c->stream, d32, n * sizeof(float));
@@ -927,8 +924,9 @@ int pcg_snapshots(hx_ctx* c, const double* f, const double* fac, int every, int 
     launch_cg_update2<double>(c->stream, r, q, c->d_minv.p, n, st, c->d_partials.p);
   };
   bool to = false;
+  GraphLoop loop(c, 0, every / 2, body);
   while (taken < count) {
-    CgState s = run_batched(c, 0, every / 2, body, 0.0, 0.0, &to, 1);
+    CgState s = loop.run(false, 0.0, 0.0, &to, 1);
     HX_CUDA(cudaMemcpyAsync(snaps + (size_t)taken * n, x, n * sizeof(double),
                             cudaMemcpyDeviceToDevice, c->stream));
     ++taken;

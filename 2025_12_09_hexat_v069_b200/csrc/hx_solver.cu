@@ -95,7 +95,7 @@ static double now_ms() {
 // Workspace
 // ---------------------------------------------------------------------------
 void ensure_workspace(hx_ctx* c) {
-  if (!c->h_state) HX_CUDA(cudaMallocHost(&c->h_state, 4 * sizeof(CgState)));
+  if (!c->h_state) HX_CUDA(cudaMallocHost(&c->h_state, 6 * sizeof(CgState)));
   c->d_state.ensure(4);
   const size_t nb = std::max<size_t>(
       std::max(mv_num_blocks<float>(c->g), mv_num_blocks<double>(c->g)), 64ull * sm_count());
@@ -138,15 +138,13 @@ CgState get_state(hx_ctx* c, int slot) {
   return c->h_state[slot];
 }
 
-// Run `body` (a sequence of launches on c->stream) `reps` times as one CUDA
-// graph launch per poll; stop when the state in `slot` leaves RUNNING, the
-// wall-clock limit is hit, or after `max_launches` graph launches (0: no
-// limit).  Returns the final state.
-CgState run_batched(hx_ctx* c, int slot, int reps, const std::function<void()>& body,
-                    double wall_limit_ms, double t0, bool* timed_out, int max_launches,
-                    const std::function<bool(const CgState&)>& keep_going) {
+// A graph of a solve is captured and instantiated once: that costs about 4 us
+// of host time per node, which a learned solve on 128 x 64 x 64 (32 iterations
+// of 45 nodes, rebuilt after each of its 8 reliable updates) used to pay for
+// with 55 of its 124 ms.
+GraphLoop::GraphLoop(hx_ctx* c, int slot, int reps, const std::function<void()>& body)
+    : c_(c), slot_(slot) {
   cudaGraph_t graph = nullptr;
-  cudaGraphExec_t exec = nullptr;
   const int64_t before = launch_counter();
   HX_CUDA(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
   try {
@@ -156,42 +154,67 @@ CgState run_batched(hx_ctx* c, int slot, int reps, const std::function<void()>& 
     if (graph) cudaGraphDestroy(graph);
     throw;
   }
-  const int64_t per_graph = launch_counter() - before;
+  per_graph_ = launch_counter() - before;
   launch_counter() = before;  // captured, not yet launched
   HX_CUDA(cudaStreamEndCapture(c->stream, &graph));
-  cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
+  cudaError_t e = cudaGraphInstantiate(&exec_, graph, 0);
   cudaGraphDestroy(graph);
-  HX_CUDA(ie);
-  CgState st{};
-  *timed_out = false;
-  try {
-    for (int nl = 1;; ++nl) {
-      HX_CUDA(cudaGraphLaunch(exec, c->stream));
-      launch_counter() += per_graph;
-      st = get_state(c, slot);
-      if (st.status != HX_RUNNING) break;
-      if (max_launches > 0 && nl >= max_launches) break;
-      if (keep_going && !keep_going(st)) break;
-      if (wall_limit_ms > 0 && now_ms() - t0 > wall_limit_ms) {
-        *timed_out = true;
-        break;
-      }
-    }
-  } catch (...) {
-    cudaGraphExecDestroy(exec);
-    throw;
+  for (int i = 0; i < 2 && e == cudaSuccess; ++i)
+    e = cudaEventCreateWithFlags(&ev_[i], cudaEventDisableTiming);
+  if (e != cudaSuccess) {
+    release();
+    HX_CUDA(e);
   }
-  HX_CUDA(cudaGraphExecDestroy(exec));
+}
+
+void GraphLoop::release() {
+  if (exec_) cudaGraphExecDestroy(exec_);
+  for (auto& ev : ev_)
+    if (ev) cudaEventDestroy(ev);
+  exec_ = nullptr;
+  ev_[0] = ev_[1] = nullptr;
+}
+
+GraphLoop::~GraphLoop() { release(); }
+
+CgState GraphLoop::run(bool ahead, double wall_limit_ms, double t0, bool* timed_out,
+                       int max_launches, const std::function<bool(const CgState&)>& keep_going) {
+  // the state after launch i goes to pinned mirror entry 4 + i % 2
+  int launched = 0;
+  auto launch = [&] {
+    const int k = launched & 1;
+    HX_CUDA(cudaGraphLaunch(exec_, c_->stream));
+    launch_counter() += per_graph_;
+    HX_CUDA(cudaMemcpyAsync(c_->h_state + 4 + k, c_->d_state.p + slot_, sizeof(CgState),
+                            cudaMemcpyDeviceToHost, c_->stream));
+    HX_CUDA(cudaEventRecord(ev_[k], c_->stream));
+    ++launched;
+  };
+  *timed_out = false;
+  ahead = ahead && max_launches == 0;
+  CgState st{};
+  for (int i = 0;; ++i) {
+    while (launched <= i + (ahead ? 1 : 0)) launch();
+    HX_CUDA(cudaEventSynchronize(ev_[i & 1]));
+    st = c_->h_state[4 + (i & 1)];
+    if (st.status != HX_RUNNING) break;
+    if (max_launches > 0 && i + 1 >= max_launches) break;
+    if (keep_going && !keep_going(st)) break;
+    if (wall_limit_ms > 0 && now_ms() - t0 > wall_limit_ms) {
+      *timed_out = true;
+      break;
+    }
+  }
+  // a launch ahead may have moved a state that was still running
+  if (ahead) st = get_state(c_, slot_);
   return st;
 }
 
-int auto_batch(const Grid& g, int check_every) {
-  if (check_every > 0) return check_every;
-  const int64_t n = g.dofs();
-  if (n > 4000000) return 16;
-  if (n > 400000) return 32;
-  return 64;
-}
+// Iterations per graph of the Jacobi loops.  The next graph is launched before
+// the last one's state is read, so a short graph leaves no gap: 16 iterations
+// are 32 nodes to instantiate and at least 150 us of GPU work, against about
+// 10 us of host work per launch.
+int auto_batch(int check_every) { return check_every > 0 ? check_every : 16; }
 
 // Jacobi set-up: node masks, diagonal, shift, M^-1 (FP64) into c->d_minv.
 // Returns max diagonal over free DOFs.
@@ -252,8 +275,8 @@ CgState pcg_fused(hx_ctx* c, int slot, const T* fac, const T* b, T* x, bool warm
     launch_cg_update2<T>(c->stream, r, q, minv, n, st, c->d_partials.p);
     if (xbest) launch_axpy_state<T>(c->stream, xbest, x, P1, n, st, 2);
   };
-  const int reps = std::max(1, check_every / 2);
-  CgState sf = run_batched(c, slot, reps, body, wall_ms, t0, timed_out, 0);
+  GraphLoop loop(c, slot, std::max(1, check_every / 2), body);
+  CgState sf = loop.run(true, wall_ms, t0, timed_out);
   // apply the pending step x_{k+1} = x_k + alpha_k p_k (not after a breakdown,
   // whose alpha is invalid); p_k sits in P[(iter-1) % 2]
   if (sf.status != HX_ST_BREAKDOWN && sf.iter > 0) {
@@ -279,7 +302,7 @@ static CgState pcg_fp64(hx_ctx* c, const double* fac, const double* b, double* x
   const CgState init =
       fresh_state(o.tol, o.max_iter, 1, o.divergence_checks != 0, o.keep_best != 0);
   return pcg_fused<double>(c, 0, fac, b, x, warm, shift, c->K, r, P0, P1, q, c->d_minv.p, xbest,
-                           init, auto_batch(c->g, o.check_every), o.wall_limit_ms, t0, timed_out);
+                           init, auto_batch(o.check_every), o.wall_limit_ms, t0, timed_out);
 }
 
 // FP64 true residual ||b - (K+sI)x|| / ||b||.
@@ -368,29 +391,26 @@ CgState solve_mixed(hx_ctx* c, const double* fac, const double* b, double* x, bo
   st.aux[2] = st.rr;
   st.max_iter = o.max_iter;
   put_state(c, 1, st);
-  const int reps = std::max(1, auto_batch(g, o.check_every) / 2);
-  int parity = 0;  // which P buffer holds p_{k-1}: P1 when parity == 0
+  // iterations alternate p from P1 to P0 and back
+  GraphLoop loop(c, 1, std::max(1, auto_batch(o.check_every) / 2), [&]() {
+    launch_pcg_step<float>(c->stream, P1, P0, r32, minv32, d32, q32, fac32, c->d_nmask.p, g, K32,
+                           sh32, si, c->d_partials.p);
+    launch_cg_update2<float>(c->stream, r32, q32, minv32, n, si, c->d_partials.p);
+    launch_pcg_step<float>(c->stream, P0, P1, r32, minv32, d32, q32, fac32, c->d_nmask.p, g, K32,
+                           sh32, si, c->d_partials.p);
+    launch_cg_update2<float>(c->stream, r32, q32, minv32, n, si, c->d_partials.p);
+  });
   for (;;) {
-    float* Pin = parity ? P0 : P1;
-    float* Pout = parity ? P1 : P0;
-    auto body = [&]() {
-      launch_pcg_step<float>(c->stream, Pin, Pout, r32, minv32, d32, q32, fac32, c->d_nmask.p, g,
-                             K32, sh32, si, c->d_partials.p);
-      launch_cg_update2<float>(c->stream, r32, q32, minv32, n, si, c->d_partials.p);
-      launch_pcg_step<float>(c->stream, Pout, Pin, r32, minv32, d32, q32, fac32, c->d_nmask.p, g,
-                             K32, sh32, si, c->d_partials.p);
-      launch_cg_update2<float>(c->stream, r32, q32, minv32, n, si, c->d_partials.p);
-    };
     const int it_before = st.iter;
-    CgState sf = run_batched(c, 1, reps, body, o.wall_limit_ms, t0, timed_out, 0);
+    CgState sf = loop.run(true, o.wall_limit_ms, t0, timed_out);
     const int done = sf.iter - it_before;
     *inner_total += done;
-    // p_k of the last completed iteration: iterations alternate Pin -> Pout
-    float* pk = (done % 2 == 1) ? Pout : Pin;
-    if (done % 2 == 1) parity ^= 1;
+    float* pk = (done % 2 == 1) ? P0 : P1;  // p of the last completed iteration
     if (sf.status != HX_ST_BREAKDOWN && done > 0) {
       launch_axpy_state<float>(c->stream, d32, d32, pk, n, si, 0);  // pending step
     }
+    if (pk == P0)  // the next iteration reads P1
+      HX_CUDA(cudaMemcpyAsync(P1, P0, n * sizeof(float), cudaMemcpyDeviceToDevice, c->stream));
     // fold the FP32 correction into x and replace the residual in FP64
     launch_ir_correct(c->stream, x, d32, n, so);
     launch_fill_zero(c->stream, d32, n * sizeof(float));
@@ -678,13 +698,17 @@ hx_status filter_grid(hx_ctx* c, const Grid& g, const double h[3], const double*
     if (rep) *rep = R;
     return HX_OK;
   }
-  auto body = [&]() {
-    launch_filter_matvec(c->stream, p, q, g, F, st, c->d_partials.p);
-    launch_cg_update<double>(c->stream, x, p, r, q, invd, nn, st, c->d_partials.p);
-    launch_cg_pupdate<double>(c->stream, p, r, invd, nn, st);
-  };
-  bool to = false;
-  CgState sf = run_batched(c, 2, 10, body, 0.0, t0, &to, 0);
+  // 10 iterations between tests of the residual, launched one by one: a filter
+  // takes 10 to 20 iterations, too few to pay for a graph
+  CgState sf = s0;
+  while (sf.status == HX_RUNNING) {
+    for (int i = 0; i < 10; ++i) {
+      launch_filter_matvec(c->stream, p, q, g, F, st, c->d_partials.p);
+      launch_cg_update<double>(c->stream, x, p, r, q, invd, nn, st, c->d_partials.p);
+      launch_cg_pupdate<double>(c->stream, p, r, invd, nn, st);
+    }
+    sf = get_state(c, 2);
+  }
   launch_filter_extract(c->stream, x, out, g);
   HX_CUDA(cudaStreamSynchronize(c->stream));
   R.iterations = sf.iter;

@@ -10,14 +10,33 @@ namespace hx {
 CgState fresh_state(double tol, int max_iter, int check_every, bool divchecks, bool keep_best);
 void put_state(hx_ctx* c, int slot, const CgState& s);
 CgState get_state(hx_ctx* c, int slot);
-int auto_batch(const Grid& g, int check_every);
-// Capture `reps` x body into one CUDA graph and launch it until the state of
-// `slot` leaves HX_RUNNING, `max_launches` (> 0) launches were made, the wall
-// limit passed, or keep_going (if given) returns false for the state read
-// after a launch.
-CgState run_batched(hx_ctx* c, int slot, int reps, const std::function<void()>& body,
-                    double wall_limit_ms, double t0, bool* timed_out, int max_launches,
-                    const std::function<bool(const CgState&)>& keep_going = {});
+int auto_batch(int check_every);
+// `reps` x body (launches on c->stream that read and advance the state of
+// `slot`) captured into one CUDA graph, once; run() launches it as often as a
+// solve needs, over all its reliable updates.
+class GraphLoop {
+ public:
+  GraphLoop(hx_ctx* c, int slot, int reps, const std::function<void()>& body);
+  ~GraphLoop();
+  GraphLoop(const GraphLoop&) = delete;
+  GraphLoop& operator=(const GraphLoop&) = delete;
+  // Launches until the state leaves HX_RUNNING, `max_launches` (> 0) launches
+  // were made, the wall limit passed, or keep_going (if given) returns false
+  // for the state read after a launch.  ahead: launch the next graph before
+  // the state of the last one is read (not with max_launches), so that the GPU
+  // does not wait for the host; once the state has stopped, one launch more
+  // runs through without effect.  Returns the state after all launches.
+  CgState run(bool ahead, double wall_limit_ms, double t0, bool* timed_out, int max_launches = 0,
+              const std::function<bool(const CgState&)>& keep_going = {});
+
+ private:
+  void release();
+  hx_ctx* c_;
+  int slot_;
+  cudaGraphExec_t exec_ = nullptr;
+  int64_t per_graph_ = 0;
+  cudaEvent_t ev_[2] = {nullptr, nullptr};
+};
 // node masks, diagonal, shift and M^-1 (FP64) for `fac`; returns max diag
 double jacobi_setup_public(hx_ctx* c, const double* fac, double shift_factor, double* shift_out);
 template <typename T>
