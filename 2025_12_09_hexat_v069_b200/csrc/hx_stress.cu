@@ -146,36 +146,101 @@ __global__ void k_energy(const double* __restrict__ u, Grid g, ElemCoef<double> 
   }
 }
 
-// One bisection step of the OC update (state aux: l1, l2, lmid).
-__global__ void k_oc_step(const double* __restrict__ x, const double* __restrict__ dc,
-                          const double* __restrict__ dv, int64_t n, double volfrac, double move,
-                          double* __restrict__ xnew, CgState* st, double* partials) {
+// The OC bisection, several steps per pass over the elements.  A step's decision
+// needs the volume at the middle of the current interval (state aux: l1, l2; the
+// last middle in aux[2]); a pass sums it at the 2^OC_LEVELS - 1 middles that the
+// next OC_LEVELS steps can reach (a binary tree, node c's halves 2c and 2c + 1,
+// the lower half where the volume is within its bound), and its last block
+// then takes the steps.  The middles are formed by the same halving as step by
+// step, so the decisions are the same unless a volume is within rounding of its
+// bound.  Each element costs one square root and division for all middles:
+//   x sqrt(d / (l dv)) = [x sqrt(d / dv)] / sqrt(l),
+// the bracket kept in xnew after the first pass (k_oc_finish overwrites it).
+// At 160 x 80 x 80 elements the 55 steps took 0.88 ms as 100 launches of one step
+// and take 0.39 ms (0.49 ms with four levels per pass: the 15-value reduction
+// costs more than the passes it saves).
+constexpr int OC_LEVELS = 3, OC_NODES = (1 << OC_LEVELS) - 1;
+
+__device__ __forceinline__ double oc_bracket(double x, double dc, const double* dv, int64_t e) {
+  return x * sqrt(fmax(-dc, 0.0) / (dv ? dv[e] : 1.0));
+}
+
+// 1 / sqrt(middle of tree node c) of the interval [lo, hi]
+__device__ __forceinline__ double oc_middle(double lo, double hi, int c) {
+  for (int bit = 31 - __clz(c) - 1; bit >= 0; --bit) {
+    const double m = 0.5 * (lo + hi);
+    if ((c >> bit) & 1) lo = m; else hi = m;
+  }
+  return 1.0 / sqrt(0.5 * (lo + hi));
+}
+
+__global__ void k_oc_table(const CgState* st, double* tab) {
+  if (threadIdx.x < OC_NODES) tab[threadIdx.x] = oc_middle(st->aux[0], st->aux[1], threadIdx.x + 1);
+}
+
+__global__ void __launch_bounds__(256, 2)
+    k_oc_pass(const double* __restrict__ x, const double* __restrict__ dc,
+              const double* __restrict__ dv, int64_t n, double volfrac, double move,
+              double* __restrict__ bracket, int first, CgState* st, double* partials, double* tab,
+              int max_steps) {
   if (st->status != HX_RUNNING) return;
-  const double l1 = st->aux[0], l2 = st->aux[1];
-  const double lmid = 0.5 * (l1 + l2);
-  double vol = 0.0;
+  double rs[OC_NODES], vol[OC_NODES];
+#pragma unroll
+  for (int c = 0; c < OC_NODES; ++c) {
+    rs[c] = tab[c];
+    vol[c] = 0.0;
+  }
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const double xe = x[e];
+    double g;
+    if (first) {
+      g = oc_bracket(xe, dc[e], dv, e);
+      bracket[e] = g;
+    } else {
+      g = bracket[e];
+    }
+    const double lo = fmax(0.0, xe - move), hi = fmin(1.0, xe + move);
+#pragma unroll
+    for (int c = 0; c < OC_NODES; ++c) vol[c] += fmin(fmax(g * rs[c], lo), hi);
+  }
+  if (!grid_reduce<OC_NODES>(vol, partials, &st->ticket[TK_AUX])) return;
+  __shared__ double ab[2];
+  if (threadIdx.x == 0) {
+    double a = st->aux[0], b = st->aux[1];
+    int c = 1, it = st->iter, status = HX_RUNNING;
+    for (int l = 0; l < OC_LEVELS && it < max_steps && status == HX_RUNNING; ++l) {
+      const double lmid = 0.5 * (a + b);
+      double v = 0.0;
+#pragma unroll
+      for (int k = 0; k < OC_NODES; ++k) v = k == c - 1 ? vol[k] : v;
+      const bool over = v > volfrac * (double)n;
+      if (over) a = lmid; else b = lmid;
+      c = 2 * c + (over ? 1 : 0);
+      ++it;
+      st->aux[2] = lmid;
+      if (!((b - a) / (a + b) > 1e-3)) status = HX_ST_CONVERGED;
+    }
+    st->aux[0] = ab[0] = a;
+    st->aux[1] = ab[1] = b;
+    st->iter = it;
+    st->status = status;
+  }
+  __syncthreads();
+  if (threadIdx.x < OC_NODES) tab[threadIdx.x] = oc_middle(ab[0], ab[1], threadIdx.x + 1);
+}
+
+// x_new at the last middle
+__global__ void k_oc_finish(const double* __restrict__ x, const double* __restrict__ dc,
+                            const double* __restrict__ dv, int64_t n, double move,
+                            const CgState* st, double* __restrict__ xnew) {
+  const double lmid = st->aux[2];
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
        e += (int64_t)gridDim.x * blockDim.x) {
     const double xe = x[e];
     const double be = sqrt(fmax(-dc[e], 0.0) / (lmid * (dv ? dv[e] : 1.0)));
-    double xn = xe * be;
     const double lo = fmax(0.0, xe - move), hi = fmin(1.0, xe + move);
-    xn = fmin(fmax(xn, lo), hi);
-    xnew[e] = xn;
-    vol += xn;
-  }
-  double v[1] = {vol};
-  if (grid_reduce<1>(v, partials, &st->ticket[TK_AUX]) && threadIdx.x == 0) {
-    double a = l1, b = l2;
-    if (v[0] > volfrac * (double)n)
-      a = lmid;
-    else
-      b = lmid;
-    st->aux[0] = a;
-    st->aux[1] = b;
-    st->aux[2] = lmid;
-    st->iter += 1;
-    if (!((b - a) / (a + b) > 1e-3)) st->status = HX_ST_CONVERGED;
+    xnew[e] = fmin(fmax(xe * be, lo), hi);
   }
 }
 
@@ -255,12 +320,20 @@ void launch_energy(cudaStream_t s, const double* u, const Grid& g, const ElemCoe
 void launch_oc(cudaStream_t s, const double* x, const double* dc, const double* dv, int64_t n,
                double volfrac, double move, double* xnew, CgState* st, double* partials,
                int max_steps) {
+  // OC_NODES partial sums per block and the table behind them: below the 256
+  // doubles per SM that every workspace holds
   const unsigned blocks =
-      (unsigned)std::max<int64_t>(1, std::min<int64_t>(cdiv(n, 256), 8LL * sm_count()));
-  for (int i = 0; i < max_steps; ++i) {
-    k_oc_step<<<blocks, 256, 0, s>>>(x, dc, dv, n, volfrac, move, xnew, st, partials);
+      (unsigned)std::max<int64_t>(1, std::min<int64_t>(cdiv(n, 256), 2LL * sm_count()));
+  double* tab = partials + (size_t)OC_NODES * blocks;
+  k_oc_table<<<1, 32, 0, s>>>(st, tab);
+  HX_CHECK_LAUNCH();
+  for (int i = 0; i < max_steps; i += OC_LEVELS) {
+    k_oc_pass<<<blocks, 256, 0, s>>>(x, dc, dv, n, volfrac, move, xnew, i == 0, st, partials, tab,
+                                     max_steps);
     HX_CHECK_LAUNCH();
   }
+  k_oc_finish<<<blocks, 256, 0, s>>>(x, dc, dv, n, move, st, xnew);
+  HX_CHECK_LAUNCH();
 }
 
 }  // namespace hx
