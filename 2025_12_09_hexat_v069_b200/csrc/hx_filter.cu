@@ -5,10 +5,20 @@
 // grid of identical box elements the assembled operator is exactly
 //   A = r^2 (Sx(x)My(x)Mz + Mx(x)Sy(x)Mz + Mx(x)My(x)Sz) + Mx(x)My(x)Mz
 // with S/M the assembled 1D stiffness/mass (tridiagonal; boundary rows carry
-// one element).  The matvec applies it separably on a 3x3x3 register window
-// that slides along z: 54 + 27 + 12 FMAs per node, no atomics, no stored
-// matrix.  ref_compat=1 reproduces the reference element whose top face is
-// at z=+dz (src/Core/Element.jl:106-107), i.e. a box 1.5*dz tall.
+// one element).
+// ref_compat=1 reproduces the reference element whose top face is at z=+dz
+// (src/Core/Element.jl:106-107), i.e. a box 1.5*dz tall.
+//
+// Jacobi-CG on it is two kernels per iteration.  The step (k_filter_step) forms
+// the new direction while it stages it, advances x with the old one, and applies
+// A plane by plane: with the z-direction split off,
+//   A = Mz (x) [r^2 (Sx My + Mx Sy) + Mx My] + Sz (x) [r^2 Mx My],
+// each plane needs two 9-point sums a, b (26 operations on a shared-memory tile)
+// and each node 6 more over three planes.  The Jacobi diagonal takes 27 values (row
+// types), so no vector holds it.  The update (k_filter_update) is the rest.  At
+// a million nodes the vectors fit the L2 and latency bounds both kernels: an
+// iteration at 161 x 81 x 81 nodes took 56 us (plain product from 27 global
+// loads per node, then two passes over five vectors) and takes 33 us.
 #include "hx_internal.h"
 
 namespace hx {
@@ -29,6 +39,14 @@ FilterCoef make_filter_coef(double dx, double dy, double dz, double radius, int 
     F.M[a][2][0] = m;  F.M[a][2][1] = 2 * m;   F.M[a][2][2] = 0;
   }
   F.r2 = radius * radius;
+  for (int x = 0; x < 3; ++x)
+    for (int y = 0; y < 3; ++y)
+      for (int z = 0; z < 3; ++z) {
+        const double sx = F.S[0][x][1], mx = F.M[0][x][1], sy = F.S[1][y][1], my = F.M[1][y][1],
+                     sz = F.S[2][z][1], mz = F.M[2][z][1];
+        F.inv[x][y][z] =
+            1.0 / (F.r2 * (sx * my * mz + mx * sy * mz + mx * my * sz) + mx * my * mz);
+      }
   F.vol8 = dx * dy * dz / 8.0;  // the RHS uses the true volume (GPUHelmholtz.jl:175-176)
   return F;
 }
@@ -36,183 +54,282 @@ FilterCoef make_filter_coef(double dx, double dy, double dz, double radius, int 
 namespace {
 
 __device__ __forceinline__ int row_type(int i, int n) {
-  return (n == 1) ? 1 : (i == 0 ? 0 : (i == n - 1 ? 2 : 1));
+  return i == 0 ? 0 : (i == n - 1 ? 2 : 1);
 }
 
-constexpr int FB_X = 32, FB_Y = 8;
+constexpr int FB_X = 32, FB_Y = 8, FB_NT = FB_X * FB_Y;
+constexpr int FS_X = FB_X + 2, FS_Y = FB_Y + 2;  // staged tile with its halo
+constexpr int FB_RESIDENT = 3;
 
-// y = A x on the node grid; MODE 2 also reduces p.q into the CG state.
-template <int MODE>
-__global__ void __launch_bounds__(FB_X* FB_Y)
-    k_filter_matvec(const double* __restrict__ x, double* __restrict__ y, Grid g, FilterCoef F,
-                    int kchunk, CgState* st, double* partials) {
-  if (MODE == 2 && st->status != HX_RUNNING) return;
-  const int i = blockIdx.x * FB_X + threadIdx.x;
-  const int j = blockIdx.y * FB_Y + threadIdx.y;
+// One CTA owns a 32 x 8 node column over planes [k0, k1) and marches along z:
+// plane kp's new direction p = D^-1 r + beta p_in goes to shared memory (tile
+// and halo; the owner also stores it and x + alpha p_in), its sums a, b to
+// registers, and q of plane kp - 1 follows from three planes' sums.  r, p_in and
+// x are loaded two planes ahead.
+__global__ void __launch_bounds__(FB_NT, FB_RESIDENT)
+    k_filter_step(const double* __restrict__ pin, double* __restrict__ pout,
+                  const double* __restrict__ r, double* __restrict__ x, double* __restrict__ q,
+                  Grid g, const __grid_constant__ FilterCoef F, int kchunk, CgState* st,
+                  double* partials) {
+  pdl_wait();
+  pdl_trigger();
+  if (st->status != HX_RUNNING) return;
+  const bool first = st->iter == 0;  // x = p_in = 0
+  const double alpha = first ? 0.0 : st->alpha, beta = first ? 0.0 : st->beta;
+  __shared__ double tile[2][FS_Y][FS_X];
+  const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + FB_X * ty;
+  const int i = blockIdx.x * FB_X + tx, j = blockIdx.y * FB_Y + ty;
   const int k0 = blockIdx.z * kchunk, k1 = min(k0 + kchunk, g.nzn);
   const bool act = i < g.nxn && j < g.nyn;
   const int64_t pl = (int64_t)g.nxn * g.nyn;
-  const int tx = row_type(i, g.nxn), ty = row_type(j, g.nyn);
-  double Sx[3], Mx[3], Sy[3], My[3];
-#pragma unroll
-  for (int t = 0; t < 3; ++t) {
-    Sx[t] = F.S[0][tx][t];
-    Mx[t] = F.M[0][tx][t];
-    Sy[t] = F.S[1][ty][t];
-    My[t] = F.M[1][ty][t];
+  const int rx = row_type(min(i, g.nxn - 1), g.nxn), ry = row_type(min(j, g.nyn - 1), g.nyn);
+  // Nodes outside the grid are staged as 0, so that only the diagonal entries
+  // depend on the row; the off-diagonal ones are m and -s everywhere.
+  const double mx1 = F.M[0][rx][1], sx1 = F.S[0][rx][1], my1 = F.M[1][ry][1], sy1 = F.S[1][ry][1];
+  // halo node of the staged tile that this thread fills besides its own: two
+  // rows of 34, then two columns of 8
+  const bool halo = tid < 2 * FS_X + 2 * FB_Y;
+  int hx, hy;
+  if (tid < 2 * FS_X) {
+    hx = tid % FS_X;
+    hy = tid < FS_X ? 0 : FS_Y - 1;
+  } else {
+    hx = ((tid - 2 * FS_X) & 1) ? FS_X - 1 : 0;
+    hy = 1 + min((tid - 2 * FS_X) >> 1, FB_Y - 1);
   }
-  auto ld = [&](int a, int b, int k) -> double {
-    const int ii = i + a, jj = j + b;
-    if (!act || k < 0 || k >= g.nzn || ii < 0 || jj < 0 || ii >= g.nxn || jj >= g.nyn) return 0.0;
-    return __ldg(&x[(int64_t)k * pl + (int64_t)jj * g.nxn + ii]);
+  const int hi = blockIdx.x * FB_X - 1 + hx, hj = blockIdx.y * FB_Y - 1 + hy;
+  const bool hact = halo && hi >= 0 && hj >= 0 && hi < g.nxn && hj < g.nyn;
+  const int hrx = row_type(min(max(hi, 0), g.nxn - 1), g.nxn),
+            hry = row_type(min(max(hj, 0), g.nyn - 1), g.nyn);
+  const int64_t own = (int64_t)j * g.nxn + i, hown = (int64_t)hj * g.nxn + hi;
+  // values of the next plane and of the one after it: one plane's work does not
+  // cover the latency of its loads
+  struct In {
+    double r, p, x, hr, hp;
   };
-  double w[3][3][3];  // [a][b][c] for offsets -1..1
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-#pragma unroll
-    for (int b = 0; b < 3; ++b) {
-      w[a][b][0] = 0.0;
-      w[a][b][1] = ld(a - 1, b - 1, k0 - 1);
-      w[a][b][2] = ld(a - 1, b - 1, k0);
-    }
-  double dsum = 0.0;
-  for (int k = k0; k < k1; ++k) {
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-      for (int b = 0; b < 3; ++b) {
-        w[a][b][0] = w[a][b][1];
-        w[a][b][1] = w[a][b][2];
-        w[a][b][2] = ld(a - 1, b - 1, k + 1);
-      }
-    const int tz = row_type(k, g.nzn);
-    const double* Sz = F.S[2][tz];
-    const double* Mz = F.M[2][tz];
-    double yMM[3], ySM[3], yMS[3];
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-      double zM[3], zS[3];
-#pragma unroll
-      for (int b = 0; b < 3; ++b) {
-        zM[b] = Mz[0] * w[a][b][0] + Mz[1] * w[a][b][1] + Mz[2] * w[a][b][2];
-        zS[b] = Sz[0] * w[a][b][0] + Sz[1] * w[a][b][1] + Sz[2] * w[a][b][2];
-      }
-      yMM[a] = My[0] * zM[0] + My[1] * zM[1] + My[2] * zM[2];
-      ySM[a] = Sy[0] * zM[0] + Sy[1] * zM[1] + Sy[2] * zM[2];
-      yMS[a] = My[0] * zS[0] + My[1] * zS[1] + My[2] * zS[2];
-    }
-    double v = 0.0;
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-      v += F.r2 * (Sx[a] * yMM[a] + Mx[a] * (ySM[a] + yMS[a])) + Mx[a] * yMM[a];
+  auto load = [&](int kp, int64_t o) {
+    double nr = 0, np = 0, nx = 0, nhr = 0, nhp = 0;
+    if (kp < 0 || kp >= g.nzn || kp > k1) return In{0, 0, 0, 0, 0};
     if (act) {
-      y[(int64_t)k * pl + (int64_t)j * g.nxn + i] = v;
-      if (MODE != 0) dsum += w[1][1][1] * v;
+      nr = r[o + own];
+      if (!first) {
+        np = pin[o + own];
+        if (kp >= k0 && kp < k1) nx = x[o + own];
+      }
     }
+    if (hact) {
+      nhr = r[o + hown];
+      if (!first) nhp = pin[o + hown];
+    }
+    return In{nr, np, nx, nhr, nhp};
+  };
+  In n0 = load(k0 - 1, (k0 - 1) * pl), n1 = load(k0, k0 * pl);
+  double a0 = 0, a1 = 0, b0 = 0, b1 = 0, p1 = 0, dsum = 0.0;  // planes kp - 2, kp - 1
+  const int rz0 = row_type(max(k0 - 1, 0), g.nzn);
+  double iv = F.inv[rx][ry][rz0], ivh = F.inv[hrx][hry][rz0];  // of plane kp
+  int64_t o = (k0 - 1) * pl;                                   // first node of plane kp
+  for (int kp = k0 - 1; kp <= k1; ++kp) {
+    double(*t)[FS_X] = tile[kp & 1];
+    if (kp == 1 || kp == g.nzn - 1) {
+      const int rz = row_type(kp, g.nzn);
+      iv = F.inv[rx][ry][rz];
+      ivh = F.inv[hrx][hry][rz];
+    }
+    const double pn = iv * n0.r + beta * n0.p;
+    const double xn = n0.x + alpha * n0.p;
+    t[ty + 1][tx + 1] = pn;
+    if (halo) t[hy][hx] = ivh * n0.hr + beta * n0.hp;
+    if (act && kp >= k0 && kp < k1) {
+      pout[o + own] = pn;
+      x[o + own] = xn;
+    }
+    n0 = n1;
+    n1 = load(kp + 2, o + 2 * pl);
+    __syncthreads();  // plane kp staged (its buffer was last read two planes ago)
+    double a2 = 0.0, b2 = 0.0;
+    if (kp >= 0 && kp < g.nzn) {
+      double xm[3], xs[3];
+#pragma unroll
+      for (int b = 0; b < 3; ++b) {
+        const double v = t[ty + b][tx + 1], w = t[ty + b][tx] + t[ty + b][tx + 2];
+        xm[b] = fma(mx1, v, F.M[0][1][0] * w);
+        xs[b] = fma(sx1, v, F.S[0][1][0] * w);
+      }
+      const double wm = xm[0] + xm[2];
+      const double mm = fma(my1, xm[1], F.M[1][1][0] * wm), ms = fma(sy1, xm[1], F.S[1][1][0] * wm);
+      const double sm = fma(my1, xs[1], F.M[1][1][0] * (xs[0] + xs[2]));
+      a2 = fma(F.r2, sm + ms, mm);
+      b2 = F.r2 * mm;
+    }
+    if (kp > k0 && act) {
+      const int zt = row_type(kp - 1, g.nzn);
+      const double v = fma(F.M[2][zt][1], a1, F.M[2][1][0] * (a0 + a2)) +
+                       fma(F.S[2][zt][1], b1, F.S[2][1][0] * (b0 + b2));
+      q[o - pl + own] = v;
+      dsum += p1 * v;
+    }
+    a0 = a1;
+    a1 = a2;
+    b0 = b1;
+    b1 = b2;
+    p1 = pn;
+    o += pl;
   }
-  if (MODE != 0) {
-    double vv[1] = {dsum};
-    if (grid_reduce<1>(vv, partials, &st->ticket[TK_MATVEC]) && threadIdx.x == 0 &&
-        threadIdx.y == 0) {
-      const double pq = vv[0];
-      st->pq = pq;
-      if (!(pq > 0.0) || !isfinite(pq))
-        st->status = HX_ST_BREAKDOWN;
-      else
-        st->alpha = st->rz / pq;
-    }
+  double vv[1] = {dsum};
+  if (grid_reduce<1>(vv, partials, &st->ticket[TK_MATVEC]) && tid == 0) {
+    const double pq = vv[0];
+    st->pq = pq;
+    if (!(pq > 0.0) || !isfinite(pq))
+      st->status = HX_ST_BREAKDOWN;
+    else
+      st->alpha = st->rz / pq;
   }
 }
 
-__global__ void k_filter_invdiag(double* __restrict__ invd, Grid g, FilterCoef F) {
-  const int64_t nn = g.nodes();
-  for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < nn;
-       n += (int64_t)gridDim.x * blockDim.x) {
-    const int i = (int)(n % g.nxn);
-    const int64_t r = n / g.nxn;
-    const int j = (int)(r % g.nyn), k = (int)(r / g.nyn);
-    const int tx = row_type(i, g.nxn), ty = row_type(j, g.nyn), tz = row_type(k, g.nzn);
-    const double sx = F.S[0][tx][1], mx = F.M[0][tx][1];
-    const double sy = F.S[1][ty][1], my = F.M[1][ty][1];
-    const double sz = F.S[2][tz][1], mz = F.M[2][tz][1];
-    const double d = F.r2 * (sx * my * mz + mx * sy * mz + mx * my * sz) + mx * my * mz;
-    invd[n] = 1.0 / d;
+// The kernels below take node (element) rows by warp: no division per entry.
+
+// r -= alpha q, r.D^-1 r and r.r, tests, beta.
+__global__ void __launch_bounds__(FB_NT)
+    k_filter_update(double* __restrict__ r, const double* __restrict__ q, Grid g,
+                    const __grid_constant__ FilterCoef F, CgState* st, double* partials) {
+  pdl_wait();
+  pdl_trigger();
+  if (st->status != HX_RUNNING) return;
+  const double alpha = st->alpha;
+  __shared__ CgState s0;  // read after grid_reduce's barriers
+  load_state(&s0, st);
+  double rz = 0, rr = 0;
+  const unsigned rows = (unsigned)g.nyn * (unsigned)g.nzn;
+  for (unsigned row = blockIdx.x * FB_Y + threadIdx.y; row < rows; row += gridDim.x * FB_Y) {
+    const int k = row / (unsigned)g.nyn, j = row - k * (unsigned)g.nyn;
+    const int ty = row_type(j, g.nyn), tz = row_type(k, g.nzn);
+    const double in = F.inv[1][ty][tz], lo = F.inv[0][ty][tz], hi = F.inv[2][ty][tz];
+    const int64_t o = (int64_t)row * g.nxn;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < g.nxn; i += FB_X) {
+      const double ri = r[o + i] - alpha * q[o + i];
+      r[o + i] = ri;
+      const double d = i == 0 ? lo : (i == g.nxn - 1 ? hi : in);
+      rz += ri * (d * ri);
+      rr += ri * ri;
+    }
   }
+  double v[2] = {rz, rr};
+  if (grid_reduce<2>(v, partials, &st->ticket[TK_UPDATE]) && threadIdx.x + threadIdx.y == 0)
+    cg_finish_iteration(st, s0, v[0], v[1]);
 }
 
-// b_n = vol/8 * sum of rho over the (up to 8) elements around node n
-// (GPUHelmholtz.jl:39-50 scatters the same sums with atomics).
-__global__ void k_filter_rhs(const double* __restrict__ rho, double* __restrict__ b, Grid g,
-                             double vol8) {
-  const int64_t nn = g.nodes();
-  for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < nn;
-       n += (int64_t)gridDim.x * blockDim.x) {
-    const int i = (int)(n % g.nxn);
-    const int64_t r = n / g.nxn;
-    const int j = (int)(r % g.nyn), k = (int)(r / g.nyn);
-    double s = 0.0;
+// r_n = vol/8 * sum of rho over the (up to 8) elements around node n
+// (GPUHelmholtz.jl:39-50 scatters the same sums with atomics), and the CG
+// state of x = 0.
+__global__ void __launch_bounds__(FB_NT)
+    k_filter_init(const double* __restrict__ rho, double* __restrict__ r, Grid g,
+                  const __grid_constant__ FilterCoef F, CgState* st, double* partials) {
+  double rz = 0, rr = 0;
+  const unsigned rows = (unsigned)g.nyn * (unsigned)g.nzn;
+  for (unsigned row = blockIdx.x * FB_Y + threadIdx.y; row < rows; row += gridDim.x * FB_Y) {
+    const int k = row / (unsigned)g.nyn, j = row - k * (unsigned)g.nyn;
+    const int ty = row_type(j, g.nyn), tz = row_type(k, g.nzn);
+    for (int i = threadIdx.x; i < g.nxn; i += FB_X) {
+      double s = 0.0;
 #pragma unroll
-    for (int dk = -1; dk <= 0; ++dk)
+      for (int dk = -1; dk <= 0; ++dk)
 #pragma unroll
-      for (int dj = -1; dj <= 0; ++dj)
+        for (int dj = -1; dj <= 0; ++dj)
 #pragma unroll
-        for (int di = -1; di <= 0; ++di) {
-          const int ei = i + di, ej = j + dj, ek = k + dk;
-          if (ei >= 0 && ej >= 0 && ek >= 0 && ei < g.nxe && ej < g.nye && ek < g.nze)
-            s += rho[((int64_t)ek * g.nye + ej) * g.nxe + ei];
-        }
-    b[n] = s * vol8;
+          for (int di = -1; di <= 0; ++di) {
+            const int ei = i + di, ej = j + dj, ek = k + dk;
+            if (ei >= 0 && ej >= 0 && ek >= 0 && ei < g.nxe && ej < g.nye && ek < g.nze)
+              s += rho[((int64_t)ek * g.nye + ej) * g.nxe + ei];
+          }
+      const double ri = s * F.vol8;
+      r[(int64_t)row * g.nxn + i] = ri;
+      rz += ri * (F.inv[row_type(i, g.nxn)][ty][tz] * ri);
+      rr += ri * ri;
+    }
+  }
+  double v[2] = {rz, rr};
+  if (grid_reduce<2>(v, partials, &st->ticket[TK_INIT]) && threadIdx.x + threadIdx.y == 0) {
+    st->rz = v[0];
+    st->rr = v[1];
+    st->bnorm = sqrt(v[1]);
+    st->iter = 0;
+    st->best_rel = INFINITY;
+    st->snap = 0;
+    st->rel_res = v[1] == 0.0 ? 0.0 : 1.0;
+    st->status = v[1] == 0.0 ? HX_ST_ZERO_RHS : (isfinite(v[1]) ? HX_RUNNING : HX_ST_NONFINITE);
   }
 }
 
 // element value = mean of its 8 nodal values (GPUHelmholtz.jl:78-89)
-__global__ void k_filter_extract(const double* __restrict__ x, double* __restrict__ out, Grid g) {
-  const int64_t ne = g.elems();
+__global__ void __launch_bounds__(FB_NT)
+    k_filter_extract(const double* __restrict__ x, const double* __restrict__ p, double alpha,
+                     double* __restrict__ out, Grid g) {
+  const unsigned rows = (unsigned)g.nye * (unsigned)g.nze;
   const int64_t pl = (int64_t)g.nxn * g.nyn;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < ne;
-       e += (int64_t)gridDim.x * blockDim.x) {
-    const int i = (int)(e % g.nxe);
-    const int64_t r = e / g.nxe;
-    const int j = (int)(r % g.nye), k = (int)(r / g.nye);
-    const int64_t n0 = (int64_t)k * pl + (int64_t)j * g.nxn + i;
-    const double s = x[n0] + x[n0 + 1] + x[n0 + g.nxn + 1] + x[n0 + g.nxn] + x[n0 + pl] +
-                     x[n0 + pl + 1] + x[n0 + pl + g.nxn + 1] + x[n0 + pl + g.nxn];
-    out[e] = s / 8.0;
+  for (unsigned row = blockIdx.x * FB_Y + threadIdx.y; row < rows; row += gridDim.x * FB_Y) {
+    const int k = row / (unsigned)g.nye, j = row - k * (unsigned)g.nye;
+    for (int i = threadIdx.x; i < g.nxe; i += FB_X) {
+      const int64_t n0 = (int64_t)k * pl + (int64_t)j * g.nxn + i;
+      auto at = [&](int64_t n) { return x[n] + alpha * p[n]; };
+      const double s = at(n0) + at(n0 + 1) + at(n0 + g.nxn + 1) + at(n0 + g.nxn) + at(n0 + pl) +
+                       at(n0 + pl + 1) + at(n0 + pl + g.nxn + 1) + at(n0 + pl + g.nxn);
+      out[(int64_t)row * g.nxe + i] = s / 8.0;
+    }
   }
 }
 
-unsigned flat_blocks(int64_t n) {
-  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(cdiv(n, 256), 16LL * sm_count()));
+unsigned row_blocks(int64_t rows) {
+  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(cdiv(rows, FB_Y), 8LL * sm_count()));
+}
+
+// Planes per CTA of the step: one wave of resident CTAs (two halo planes are
+// staged per chunk), but at least 4 planes.
+dim3 step_grid(const Grid& g, int* kchunk) {
+  const int64_t cols = (int64_t)cdiv(g.nxn, FB_X) * cdiv(g.nyn, FB_Y);
+  const int64_t nch = std::max<int64_t>(1, (int64_t)FB_RESIDENT * sm_count() / cols);
+  const int kc = std::min(g.nzn, std::max(4, (int)cdiv(g.nzn, nch)));
+  *kchunk = kc;
+  return dim3(cdiv(g.nxn, FB_X), cdiv(g.nyn, FB_Y), cdiv(g.nzn, kc));
 }
 
 }  // namespace
 
-void launch_filter_matvec(cudaStream_t s, const double* x, double* y, const Grid& g,
+size_t filter_blocks(const Grid& g) {
+  int kc;
+  const dim3 a = step_grid(g, &kc);
+  return std::max<size_t>((size_t)a.x * a.y * a.z, row_blocks((int64_t)g.nyn * g.nzn));
+}
+
+void launch_filter_init(cudaStream_t s, const double* rho, double* r, const Grid& g,
+                        const FilterCoef& F, CgState* st, double* partials) {
+  k_filter_init<<<row_blocks((int64_t)g.nyn * g.nzn), dim3(FB_X, FB_Y), 0, s>>>(rho, r, g, F, st,
+                                                                              partials);
+  HX_CHECK_LAUNCH();
+}
+
+void launch_filter_step(cudaStream_t s, const double* pin, double* pout, const double* r,
+                        double* x, double* q, const Grid& g, const FilterCoef& F, CgState* st,
+                        double* partials) {
+  int kc;
+  const dim3 grid = step_grid(g, &kc);
+  launch_dep(one_wave((int64_t)grid.x * grid.y * grid.z, FB_RESIDENT), k_filter_step, grid,
+             dim3(FB_X, FB_Y), 0, s, pin, pout, r, x, q, g, F, kc, st, partials);
+  HX_CHECK_LAUNCH();
+}
+
+void launch_filter_update(cudaStream_t s, double* r, const double* q, const Grid& g,
                           const FilterCoef& F, CgState* st, double* partials) {
-  const int64_t cols = (int64_t)cdiv(g.nxn, FB_X) * cdiv(g.nyn, FB_Y);
-  const int nch = (int)std::max<int64_t>(1, (4LL * sm_count() + cols - 1) / cols);
-  const int kc = std::max(4, (int)cdiv(g.nzn, nch));
-  const dim3 grid(cdiv(g.nxn, FB_X), cdiv(g.nyn, FB_Y), cdiv(g.nzn, kc));
-  const dim3 block(FB_X, FB_Y);
-  if (st)
-    k_filter_matvec<2><<<grid, block, 0, s>>>(x, y, g, F, kc, st, partials);
-  else
-    k_filter_matvec<0><<<grid, block, 0, s>>>(x, y, g, F, kc, st, partials);
+  const unsigned blocks = row_blocks((int64_t)g.nyn * g.nzn);
+  launch_dep(one_wave(blocks, 7), k_filter_update, blocks, dim3(FB_X, FB_Y), 0, s, r, q, g, F, st,
+             partials);
   HX_CHECK_LAUNCH();
 }
 
-void launch_filter_invdiag(cudaStream_t s, double* invd, const Grid& g, const FilterCoef& F) {
-  k_filter_invdiag<<<flat_blocks(g.nodes()), 256, 0, s>>>(invd, g, F);
-  HX_CHECK_LAUNCH();
-}
-
-void launch_filter_rhs(cudaStream_t s, const double* rho, double* b, const Grid& g, double vol8) {
-  k_filter_rhs<<<flat_blocks(g.nodes()), 256, 0, s>>>(rho, b, g, vol8);
-  HX_CHECK_LAUNCH();
-}
-
-void launch_filter_extract(cudaStream_t s, const double* x, double* out, const Grid& g) {
-  k_filter_extract<<<flat_blocks(g.elems()), 256, 0, s>>>(x, out, g);
+void launch_filter_extract(cudaStream_t s, const double* x, const double* p, double alpha,
+                           double* out, const Grid& g) {
+  k_filter_extract<<<row_blocks((int64_t)g.nye * g.nze), dim3(FB_X, FB_Y), 0, s>>>(x, p, alpha,
+                                                                                 out, g);
   HX_CHECK_LAUNCH();
 }
 

@@ -85,11 +85,15 @@ __global__ void k_coarse_bc(const uint8_t* __restrict__ bf, uint8_t* __restrict_
 // first Chebyshev step from x = 0: x = (1/theta) M^-1 b
 __global__ void k_cheb_first(const float* __restrict__ b, const float* __restrict__ minv,
                              float* __restrict__ x, float inv_theta, int64_t n) {
+  pdl_wait();
+  pdl_trigger();
   for (int64_t i = gt(); i < n; i += gs()) x[i] = inv_theta * minv[i] * b[i];
 }
 
 template <typename TD, typename TS>
 __global__ void k_copy_cvt(TD* __restrict__ d, const TS* __restrict__ s, int64_t n) {
+  pdl_wait();
+  pdl_trigger();
   for (int64_t i = gt(); i < n; i += gs()) d[i] = (TD)s[i];
 }
 
@@ -150,6 +154,8 @@ __global__ void k_coarse_finish(float* __restrict__ x, const float* __restrict__
 template <typename T>
 __global__ void k_fcg_coeffs(const T* __restrict__ z, const T* __restrict__ q_old,
                              const T* __restrict__ r, int64_t n, double* partials, CgState* st) {
+  pdl_wait();
+  pdl_trigger();
   if (st->status != HX_RUNNING) return;
   double zq = 0.0, zr = 0.0;
   for (int64_t i = gt(); i < n; i += gs()) {
@@ -294,6 +300,8 @@ __global__ void k_cvt_f64(TD* __restrict__ d, const double* __restrict__ s, int6
 // x = Ainv b (n x n, FP32): one warp per row, b read through the cache
 __global__ void k_dense_gemv(const float* __restrict__ Ainv, const float* __restrict__ b,
                              float* __restrict__ x, int64_t n) {
+  pdl_wait();
+  pdl_trigger();
   const int64_t w = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (w >= n) return;
@@ -519,7 +527,8 @@ static void cheb_smooth(hx_ctx* c, hx_ctx::GmgLevel& L, const float* b, float* x
   int k;    // steps done
   if (xzero) {
     cur = (m % 2 == 1) ? 0 : 1;  // x_1 .. x_m alternate, x_m in L.x
-    k_cheb_first<<<gblocks(n), 256, 0, s>>>(b, L.minv.p, buf[cur], 1.0f / theta, n);
+    launch_dep(small_vec(n), k_cheb_first, gblocks(n), 256, 0, s, b, L.minv.p, buf[cur], 1.0f / theta,
+               n);
     HX_CHECK_LAUNCH();
     k = 1;
   } else {
@@ -568,7 +577,7 @@ void gmg_vcycle(hx_ctx* c, const T* r, T* z) {
     b0 = r;
     x0 = z;
   } else {
-    k_copy_cvt<float, T><<<gblocks(n0), 256, 0, s>>>(L0.b.p, r, n0);
+    launch_dep(small_vec(n0), k_copy_cvt<float, T>, gblocks(n0), 256, 0, s, L0.b.p, r, n0);
     HX_CHECK_LAUNCH();
     b0 = L0.b.p;
     x0 = L0.x.p;
@@ -595,7 +604,7 @@ void gmg_vcycle(hx_ctx* c, const T* r, T* z) {
     bx(nl - 1, b, x);
     if (G.direct) {
       // coarsest level (the only one for small grids): its dense inverse
-      k_dense_gemv<<<(unsigned)cdiv(n * 32, 256), 256, 0, s>>>(G.ainv.p, b, x, n);
+      launch_dep(true, k_dense_gemv, (unsigned)cdiv(n * 32, 256), 256, 0, s, G.ainv.p, b, x, n);
       HX_CHECK_LAUNCH();
     } else {
       // a large coarsest level: fixed-count FP32 Jacobi-PCG from zero
@@ -627,7 +636,7 @@ void gmg_vcycle(hx_ctx* c, const T* r, T* z) {
     cheb_smooth(c, L, b, x, false, false);
   }
   if constexpr (!std::is_same<T, float>::value) {
-    k_copy_cvt<T, float><<<gblocks(n0), 256, 0, s>>>(z, L0.x.p, n0);
+    launch_dep(small_vec(n0), k_copy_cvt<T, float>, gblocks(n0), 256, 0, s, z, L0.x.p, n0);
     HX_CHECK_LAUNCH();
   }
 }
@@ -637,7 +646,7 @@ template void gmg_vcycle<float>(hx_ctx*, const float*, float*);
 template <typename T>
 void launch_fcg_coeffs(cudaStream_t s, const T* z, const T* q_old, const T* r, int64_t n,
                        double* partials, CgState* st) {
-  k_fcg_coeffs<T><<<gblocks(n), 256, 0, s>>>(z, q_old, r, n, partials, st);
+  launch_dep(small_vec(n), k_fcg_coeffs<T>, gblocks(n), 256, 0, s, z, q_old, r, n, partials, st);
   HX_CHECK_LAUNCH();
 }
 template void launch_fcg_coeffs<double>(cudaStream_t, const double*, const double*,

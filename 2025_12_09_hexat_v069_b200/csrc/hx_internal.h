@@ -93,15 +93,11 @@ void launch_minv(cudaStream_t s, const uint8_t* nmask, const T* diag, T* minv, i
 
 // ---- vector kernels (hx_vector.cu) ----
 unsigned vec_blocks(int64_t n);
+bool small_vec(int64_t n);
 constexpr int VEC_THREADS = 256;
 template <typename T>
 void launch_cg_init(cudaStream_t s, const T* b, const T* q, const T* minv, T* r, T* p, int64_t n,
                     CgState* st, double* partials);
-template <typename T>
-void launch_cg_update(cudaStream_t s, T* x, const T* p, T* r, const T* q, const T* minv, int64_t n,
-                      CgState* st, double* partials);
-template <typename T>
-void launch_cg_pupdate(cudaStream_t s, T* p, const T* r, const T* minv, int64_t n, CgState* st);
 // ys (optional, n + 8 entries): BF16(D^-1/2 r) of the new residual, the
 // learned preconditioner's input
 template <typename T>
@@ -140,19 +136,30 @@ void launch_axpby(cudaStream_t s, double* r, const double* a, const double* b, i
 
 // ---- filter (hx_filter.cu) ----
 struct FilterCoef {
-  // assembled 1D tridiagonal entries per axis: [axis][0=boundary-lo row,
-  // 1=interior, 2=boundary-hi row][lo, diag, hi] for S and M
+  // assembled 1D tridiagonal entries per axis: [axis][row type: first, inner,
+  // last node][lo, diag, hi] for S and M
   double S[3][3][3];
   double M[3][3][3];
+  double inv[3][3][3];  // Jacobi inverse diagonal by row type [x][y][z]
   double r2;
   double vol8;
 };
 FilterCoef make_filter_coef(double dx, double dy, double dz, double radius, int ref_compat);
-void launch_filter_rhs(cudaStream_t s, const double* rho, double* b, const Grid& g, double vol8);
-void launch_filter_invdiag(cudaStream_t s, double* invd, const Grid& g, const FilterCoef& F);
-void launch_filter_matvec(cudaStream_t s, const double* x, double* y, const Grid& g,
+// CTAs of the largest filter launch (three partial sums each)
+size_t filter_blocks(const Grid& g);
+// r = right-hand side of rho, and the CG state of x = 0 (st->iter = 0)
+void launch_filter_init(cudaStream_t s, const double* rho, double* r, const Grid& g,
+                        const FilterCoef& F, CgState* st, double* partials);
+// one CG iteration: p_out = D^-1 r + beta p_in, x += alpha p_in (x = p_in = 0
+// in iteration 0, not read), q = A p_out, alpha; then r -= alpha q, tests, beta
+void launch_filter_step(cudaStream_t s, const double* pin, double* pout, const double* r,
+                        double* x, double* q, const Grid& g, const FilterCoef& F, CgState* st,
+                        double* partials);
+void launch_filter_update(cudaStream_t s, double* r, const double* q, const Grid& g,
                           const FilterCoef& F, CgState* st, double* partials);
-void launch_filter_extract(cudaStream_t s, const double* x, double* out, const Grid& g);
+// out = element means of x + alpha p (alpha: the pending step of the state)
+void launch_filter_extract(cudaStream_t s, const double* x, const double* p, double alpha,
+                           double* out, const Grid& g);
 
 // ---- stress / OC (hx_stress.cu) ----
 void launch_stress(cudaStream_t s, const double* u, const double* dens, double E, double nu,
@@ -212,13 +219,10 @@ struct hx_ctx {
   // host<->device staging for F32 callers
   hx::DevBuf<char> d_stage;
 
-  // filter grid and cache (the counterpart of GLOBAL_HELMHOLTZ_CACHE)
+  // grid of the last filter (for timing) and its work vectors
   hx::Grid fg{};
   double fh[3] = {1, 1, 1};
-  bool filt_ready = false;
-  double filt_radius = -1;
-  int filt_compat = -1;
-  hx::DevBuf<double> f_invd, f_x, f_r, f_p, f_q, f_b, f_rho, f_out;
+  hx::DevBuf<double> f_x, f_r, f_p, f_p2, f_q, f_rho, f_out;
 
   // filter kernel coefficients of the last filter call (for timing)
   double f_radius_last = 0;

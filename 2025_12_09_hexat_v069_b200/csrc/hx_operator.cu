@@ -361,7 +361,6 @@ __global__ void __launch_bounds__(MV_BX* Tile<T, mode_fused(MODE)>::WARPS,
   constexpr bool RUNS = CPR <= 32;
   constexpr int NCT = RUNS ? (G::ROWS + WARPS - 1) / WARPS : (G::ROWS * CPR + NT - 1) / NT;
   using VecT = typename std::conditional<sizeof(T) == 4, float4, double2>::type;
-  if (FUSED && A.st->status != HX_RUNNING) return;
   extern __shared__ __align__(16) unsigned char smraw[];
   S& sm = *reinterpret_cast<S*>(smraw);
   const Grid& g = A.g;
@@ -374,12 +373,6 @@ __global__ void __launch_bounds__(MV_BX* Tile<T, mode_fused(MODE)>::WARPS,
   const int nplane = g.nxn * g.nyn;
   const int P3 = 3 * nplane;  // values per node plane (32-bit: the grid extent check bounds it)
   const int kp_last = min(k1, g.nzn - 1);  // last plane staged
-  T alpha_old = T(0), beta_old = T(0);
-  if (FUSED) {
-    alpha_old = (T)A.st->alpha;
-    beta_old = (T)A.st->beta;
-  }
-
   // Rows and nodes outside the grid are never copied: they have to be finite,
   // and are 0.  CTAs inside the grid read only what they copied.
   if (i0 + MV_BX >= g.nxn || j0 == 0 || j0 - 1 + BY >= g.nyn)
@@ -415,6 +408,15 @@ __global__ void __launch_bounds__(MV_BX* Tile<T, mode_fused(MODE)>::WARPS,
   if (tid == 0) {
     share_coef(A.K, sm.k);
     sm.k[4] = vneg(vone<V>());
+  }
+  // everything above may overlap the previous kernel (launch_dep)
+  pdl_wait();
+  pdl_trigger();
+  if (FUSED && A.st->status != HX_RUNNING) return;
+  T alpha_old = T(0), beta_old = T(0);
+  if (FUSED) {
+    alpha_old = (T)A.st->alpha;
+    beta_old = (T)A.st->beta;
   }
   __syncthreads();
 
@@ -964,8 +966,9 @@ void launch_one(cudaStream_t s, OpArgs<T, CUBE>& a, const ElemCoef<T>& K) {
   });
   coef_v(K, a.K);
   a.kchunk = mv_kchunk<T, FUSED>(a.g);
-  k_struct<T, MODE, CUBE>
-      <<<mv_grid<T, FUSED>(a.g, a.kchunk), dim3(MV_BX, Form::WARPS), smem, s>>>(a);
+  const dim3 grid = mv_grid<T, FUSED>(a.g, a.kchunk);
+  launch_dep(one_wave((int64_t)grid.x * grid.y * grid.z, Form::RESIDENT), k_struct<T, MODE, CUBE>,
+             grid, dim3(MV_BX, Form::WARPS), smem, s, a);
   HX_CHECK_LAUNCH();
 }
 

@@ -43,6 +43,8 @@ int sm_count() {
   return n;
 }
 
+bool one_wave(int64_t ctas, int per_sm) { return ctas <= (int64_t)per_sm * sm_count(); }
+
 ElemCoef<double> make_elem_coef(double dx, double dy, double dz, double nu) {
   ElemCoef<double> K{};
   const double lam = nu / ((1.0 + nu) * (1.0 - 2.0 * nu));
@@ -657,38 +659,33 @@ hx_status filter_grid(hx_ctx* c, const Grid& g, const double h[3], const double*
   HX_REQUIRE(radius >= 0, "radius must be >= 0");
   HX_REQUIRE(max_iter >= 1, "max_iter must be >= 1");
   ensure_workspace(c);
-  const size_t nbf = 4ull * cdiv(g.nxn, 32) * cdiv(g.nyn, 8) * cdiv(g.nzn, 4);
-  c->d_partials.ensure(std::max<size_t>(c->d_partials.n, nbf));
+  c->d_partials.ensure(std::max<size_t>(c->d_partials.n, 3 * filter_blocks(g)));
   const int64_t nn = g.nodes();
   const FilterCoef F = make_filter_coef(h[0], h[1], h[2], radius, ref_compat);
-  double* invd = c->f_invd.ensure(nn);
   double* x = c->f_x.ensure(nn);
   double* r = c->f_r.ensure(nn);
-  double* p = c->f_p.ensure(nn);
+  double* p[2] = {c->f_p.ensure(nn), c->f_p2.ensure(nn)};
   double* q = c->f_q.ensure(nn);
-  double* b = c->f_b.ensure(nn);
-  const bool same_grid = c->fg.nxe == g.nxe && c->fg.nye == g.nye && c->fg.nze == g.nze &&
-                         c->fh[0] == h[0] && c->fh[1] == h[1] && c->fh[2] == h[2];
-  if (!c->filt_ready || !same_grid || std::fabs(c->filt_radius - radius) > 1e-12 ||
-      c->filt_compat != ref_compat) {
-    c->fg = g;
-    for (int a = 0; a < 3; ++a) c->fh[a] = h[a];
-    launch_filter_invdiag(c->stream, invd, g, F);
-    c->filt_ready = true;
-    c->filt_radius = radius;
-    c->filt_compat = ref_compat;
-  }
+  c->fg = g;
+  for (int a = 0; a < 3; ++a) c->fh[a] = h[a];
   c->f_used = true;
   c->f_radius_last = radius;
   c->f_compat_last = ref_compat;
-  launch_filter_rhs(c->stream, rho, b, g, F.vol8);
-  launch_fill_zero(c->stream, x, nn * sizeof(double));
   CgState* st = c->d_state.p + 2;
   put_state(c, 2, fresh_state(tol, max_iter, 10, false, false));
-  launch_cg_init<double>(c->stream, b, nullptr, invd, r, p, nn, st, c->d_partials.p);
-  CgState s0 = get_state(c, 2);
+  launch_filter_init(c->stream, rho, r, g, F, st, c->d_partials.p);
+  // 10 iterations between tests of the residual, launched one by one: a filter
+  // takes 10 to 40 iterations, too few to pay for a graph
   hx_solve_report R{};
-  if (s0.status == HX_ST_ZERO_RHS) {
+  CgState sf;
+  do {
+    for (int i = 0; i < 10; ++i) {
+      launch_filter_step(c->stream, p[1 - (i & 1)], p[i & 1], r, x, q, g, F, st, c->d_partials.p);
+      launch_filter_update(c->stream, r, q, g, F, st, c->d_partials.p);
+    }
+    sf = get_state(c, 2);
+  } while (sf.status == HX_RUNNING);
+  if (sf.status == HX_ST_ZERO_RHS) {
     // zero RHS: the reference returns the input unchanged (GPUHelmholtz.jl:179-182)
     HX_CUDA(cudaMemcpyAsync(out, rho, g.elems() * sizeof(double), cudaMemcpyDeviceToDevice,
                             c->stream));
@@ -698,18 +695,14 @@ hx_status filter_grid(hx_ctx* c, const Grid& g, const double h[3], const double*
     if (rep) *rep = R;
     return HX_OK;
   }
-  // 10 iterations between tests of the residual, launched one by one: a filter
-  // takes 10 to 20 iterations, too few to pay for a graph
-  CgState sf = s0;
-  while (sf.status == HX_RUNNING) {
-    for (int i = 0; i < 10; ++i) {
-      launch_filter_matvec(c->stream, p, q, g, F, st, c->d_partials.p);
-      launch_cg_update<double>(c->stream, x, p, r, q, invd, nn, st, c->d_partials.p);
-      launch_cg_pupdate<double>(c->stream, p, r, invd, nn, st);
-    }
-    sf = get_state(c, 2);
+  if (sf.iter == 0 && sf.status != HX_ST_BREAKDOWN) {  // stopped before the first step: x = 0
+    launch_fill_zero(c->stream, out, g.elems() * sizeof(double));
+  } else {
+    // the last step x += alpha p is pending (after a breakdown alpha is invalid
+    // and no step is)
+    const bool pending = sf.status != HX_ST_BREAKDOWN;
+    launch_filter_extract(c->stream, x, p[(sf.iter + 1) & 1], pending ? sf.alpha : 0.0, out, g);
   }
-  launch_filter_extract(c->stream, x, out, g);
   HX_CUDA(cudaStreamSynchronize(c->stream));
   R.iterations = sf.iter;
   R.rel_res = sf.rel_res;
@@ -807,7 +800,13 @@ hx_status time_kernel(hx_ctx* c, int kernel, int reps, double* avg_ms) {
     const FilterCoef F = make_filter_coef(c->fh[0], c->fh[1], c->fh[2], c->f_radius_last,
                                           c->f_compat_last);
     const Grid fg = c->fg;
-    body = [&, F, fg] { launch_filter_matvec(c->stream, c->f_p.p, c->f_q.p, fg, F, st, c->d_partials.p); };
+    // in iteration 1 with alpha = beta = 0 the step reads and writes every vector
+    ts.iter = 1;
+    put_state(c, 3, ts);
+    body = [&, F, fg] {
+      launch_filter_step(c->stream, c->f_p2.p, c->f_p.p, c->f_r.p, c->f_x.p, c->f_q.p, fg, F, st,
+                         c->d_partials.p);
+    };
   } else if (kernel == HX_KERNEL_CONV3 || kernel == HX_KERNEL_NET_APPLY) {
     body = net_time_body(c, kernel == HX_KERNEL_CONV3 ? 0 : 1);
   } else {

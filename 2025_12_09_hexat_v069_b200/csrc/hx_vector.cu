@@ -9,25 +9,12 @@
 //                  rr = r.r; convergence / divergence tests; beta = rz'/rz
 // x lags one step behind (x += alpha p happens in the next PCG step); the
 // host applies the last step with k_axpy_state once the loop stops.
-// The three-kernel form (k_cg_update + k_cg_pupdate around a plain matvec)
-// is kept for the Helmholtz filter, whose operator is not fused.
 // All reductions are FP64 and deterministic (fixed-order block partials).
 #include "hx_internal.h"
 
 namespace hx {
 
 namespace {
-
-template <typename T>
-struct Vec2;
-template <>
-struct Vec2<double> {
-  using type = double2;
-};
-template <>
-struct Vec2<float> {
-  using type = float2;
-};
 
 // 16 bytes of T, loaded and stored as one vector (W entries)
 template <typename T>
@@ -101,84 +88,6 @@ __global__ void k_cg_init(const T* __restrict__ b, const T* __restrict__ q,
   }
 }
 
-// Finalisation shared by the update kernels (runs in one thread).
-__device__ __forceinline__ void cg_finish_iteration(CgState* st, double rzn, double rr) {
-  st->iter += 1;
-  const double rel = sqrt(rr) / st->bnorm;
-  st->rr = rr;
-  const bool tested = (st->iter % st->check_every) == 0;
-  if (tested) st->rel_res = rel;
-  int status = HX_RUNNING;
-  // Order of tests as src/Solvers/GPUSolver.jl:478-511.
-  if (st->div_ratio > 0.0 && st->iter > 50 && rel > st->div_ratio * st->best_rel)
-    status = HX_ST_DIVERGED;
-  else if (!isfinite(rel))
-    status = HX_ST_NONFINITE;
-  else if (st->explode > 0.0 && rel > st->explode)
-    status = HX_ST_DIVERGED;
-  if (status == HX_RUNNING) {
-    st->snap = 0;
-    if (rel < st->best_rel) {
-      st->best_rel = rel;
-      if (st->keep_best && rel < 1e-2) st->snap = 1;
-    }
-    if (tested && rel < st->tol) {
-      status = HX_ST_CONVERGED;
-      if (st->keep_best) st->snap = 1;
-    } else if (st->iter >= st->max_iter) {
-      status = HX_ST_MAXITER;
-    } else if (st->aux[1] > 0.0) {
-      // reliable updates: pause once the recursive residual has dropped by
-      // delta since the last FP64 residual replacement
-      if (rr > st->aux[2]) st->aux[2] = rr;
-      if (rr < st->aux[1] * st->aux[1] * st->aux[2]) status = HX_ST_PAUSED;
-    }
-    st->beta = rzn / st->rz;
-    st->rz = rzn;
-  }
-  if (!tested && status != HX_RUNNING) st->rel_res = rel;
-  st->status = status;
-}
-
-template <typename T>
-__global__ void k_cg_update(T* __restrict__ x, const T* __restrict__ p, T* __restrict__ r,
-                            const T* __restrict__ q, const T* __restrict__ minv, int64_t n,
-                            CgState* st, double* partials) {
-  if (st->status != HX_RUNNING) return;
-  const T alpha = (T)st->alpha;
-  double rz = 0, rr = 0;
-  using V = typename Vec2<T>::type;
-  const int64_t n2 = n >> 1;
-  V* x2 = reinterpret_cast<V*>(x);
-  V* r2 = reinterpret_cast<V*>(r);
-  const V* p2 = reinterpret_cast<const V*>(p);
-  const V* q2 = reinterpret_cast<const V*>(q);
-  const V* m2 = reinterpret_cast<const V*>(minv);
-  for (int64_t i = gtid(); i < n2; i += gstride()) {
-    V xv = x2[i], rv = r2[i];
-    const V pv = p2[i], qv = q2[i], mv = m2[i];
-    xv.x += alpha * pv.x;
-    xv.y += alpha * pv.y;
-    rv.x -= alpha * qv.x;
-    rv.y -= alpha * qv.y;
-    x2[i] = xv;
-    r2[i] = rv;
-    rz += (double)rv.x * (double)(mv.x * rv.x) + (double)rv.y * (double)(mv.y * rv.y);
-    rr += (double)rv.x * (double)rv.x + (double)rv.y * (double)rv.y;
-  }
-  if ((n & 1) && gtid() == 0) {
-    const int64_t i = n - 1;
-    x[i] += alpha * p[i];
-    const T ri = r[i] - alpha * q[i];
-    r[i] = ri;
-    rz += (double)ri * (double)(minv[i] * ri);
-    rr += (double)ri * (double)ri;
-  }
-  double v[2] = {rz, rr};
-  if (grid_reduce<2>(v, partials, &st->ticket[TK_UPDATE]) && threadIdx.x == 0)
-    cg_finish_iteration(st, v[0], v[1]);
-}
-
 // Second half of a fused PCG iteration: r -= alpha q on the free DOFs (M^-1
 // is 0 on the fixed ones, where the operator leaves q unmasked), dots, tests.  With
 // ys: also ys = BF16(D^-1/2 r) of the new residual (the learned
@@ -188,8 +97,12 @@ template <typename T>
 __global__ void k_cg_update2(T* __restrict__ r, const T* __restrict__ q,
                              const T* __restrict__ minv, int64_t n, CgState* st,
                              double* partials, __nv_bfloat16* __restrict__ ys) {
+  pdl_wait();
+  pdl_trigger();
   if (st->status != HX_RUNNING) return;
   const T alpha = (T)st->alpha;
+  __shared__ CgState s0;  // read after grid_reduce's barriers
+  load_state(&s0, st);
   double rz = 0, rr = 0;
   using VT = Vec16<T>;
   using V = typename VT::type;
@@ -229,7 +142,7 @@ __global__ void k_cg_update2(T* __restrict__ r, const T* __restrict__ q,
   }
   double v[2] = {rz, rr};
   if (grid_reduce<2>(v, partials, &st->ticket[TK_UPDATE]) && threadIdx.x == 0)
-    cg_finish_iteration(st, v[0], v[1]);
+    cg_finish_iteration(st, s0, v[0], v[1]);
 }
 
 // ys = BF16(D^-1/2 r), as k_cg_update2 writes it (for a residual that
@@ -252,29 +165,11 @@ __global__ void k_axpy_state(T* __restrict__ dst, const T* __restrict__ x,
   // after iteration k = iter - 1 even, P1 after an odd one).  Launches of a
   // batch that run after the loop stopped then rewrite the same snapshot
   // instead of combining x with an older direction.
+  pdl_wait();
+  pdl_trigger();
   if (when_snap && !(st->snap && ((st->iter - 1) & 1) == when_snap - 1)) return;
   const T a = (T)st->alpha;
   for (int64_t i = gtid(); i < n; i += gstride()) dst[i] = x[i] + a * p[i];
-}
-
-template <typename T>
-__global__ void k_cg_pupdate(T* __restrict__ p, const T* __restrict__ r,
-                             const T* __restrict__ minv, int64_t n, const CgState* st) {
-  if (st->status != HX_RUNNING) return;
-  const T beta = (T)st->beta;
-  using V = typename Vec2<T>::type;
-  const int64_t n2 = n >> 1;
-  V* p2 = reinterpret_cast<V*>(p);
-  const V* r2 = reinterpret_cast<const V*>(r);
-  const V* m2 = reinterpret_cast<const V*>(minv);
-  for (int64_t i = gtid(); i < n2; i += gstride()) {
-    V pv = p2[i];
-    const V rv = r2[i], mv = m2[i];
-    pv.x = mv.x * rv.x + beta * pv.x;
-    pv.y = mv.y * rv.y + beta * pv.y;
-    p2[i] = pv;
-  }
-  if ((n & 1) && gtid() == 0) p[n - 1] = minv[n - 1] * r[n - 1] + beta * p[n - 1];
 }
 
 __global__ void k_copy_if_snap(double* __restrict__ dst, const double* __restrict__ src,
@@ -358,6 +253,9 @@ unsigned vec_blocks(int64_t n) {
   return (unsigned)std::max<int64_t>(1, std::min<int64_t>(want, 8LL * sm_count()));
 }
 
+// vector kernels of fewer CTAs than a wave
+bool small_vec(int64_t n) { return vec_blocks(n) < 8u * sm_count(); }
+
 template <typename T>
 void launch_cg_init(cudaStream_t s, const T* b, const T* q, const T* minv, T* r, T* p, int64_t n,
                     CgState* st, double* partials) {
@@ -366,22 +264,10 @@ void launch_cg_init(cudaStream_t s, const T* b, const T* q, const T* minv, T* r,
 }
 
 template <typename T>
-void launch_cg_update(cudaStream_t s, T* x, const T* p, T* r, const T* q, const T* minv, int64_t n,
-                      CgState* st, double* partials) {
-  k_cg_update<T><<<vec_blocks(n), VEC_THREADS, 0, s>>>(x, p, r, q, minv, n, st, partials);
-  HX_CHECK_LAUNCH();
-}
-
-template <typename T>
-void launch_cg_pupdate(cudaStream_t s, T* p, const T* r, const T* minv, int64_t n, CgState* st) {
-  k_cg_pupdate<T><<<vec_blocks(n), VEC_THREADS, 0, s>>>(p, r, minv, n, st);
-  HX_CHECK_LAUNCH();
-}
-
-template <typename T>
 void launch_cg_update2(cudaStream_t s, T* r, const T* q, const T* minv, int64_t n, CgState* st,
                        double* partials, __nv_bfloat16* ys) {
-  k_cg_update2<T><<<vec_blocks(n), VEC_THREADS, 0, s>>>(r, q, minv, n, st, partials, ys);
+  launch_dep(small_vec(n), k_cg_update2<T>, vec_blocks(n), VEC_THREADS, 0, s, r, q, minv, n, st,
+             partials, ys);
   HX_CHECK_LAUNCH();
 }
 
@@ -394,16 +280,14 @@ void launch_dinv_bf16(cudaStream_t s, const T* r, const T* minv, __nv_bfloat16* 
 template <typename T>
 void launch_axpy_state(cudaStream_t s, T* dst, const T* x, const T* p, int64_t n,
                        const CgState* st, int when_snap) {
-  k_axpy_state<T><<<vec_blocks(n), VEC_THREADS, 0, s>>>(dst, x, p, n, st, when_snap);
+  launch_dep(small_vec(n), k_axpy_state<T>, vec_blocks(n), VEC_THREADS, 0, s, dst, x, p, n, st,
+             when_snap);
   HX_CHECK_LAUNCH();
 }
 
 #define HX_INST_CG(T)                                                                         \
   template void launch_cg_init<T>(cudaStream_t, const T*, const T*, const T*, T*, T*, int64_t, \
                                   CgState*, double*);                                         \
-  template void launch_cg_update<T>(cudaStream_t, T*, const T*, T*, const T*, const T*,       \
-                                    int64_t, CgState*, double*);                              \
-  template void launch_cg_pupdate<T>(cudaStream_t, T*, const T*, const T*, int64_t, CgState*); \
   template void launch_cg_update2<T>(cudaStream_t, T*, const T*, const T*, int64_t, CgState*,  \
                                      double*, __nv_bfloat16*);                                 \
   template void launch_dinv_bf16<T>(cudaStream_t, const T*, const T*, __nv_bfloat16*,         \
