@@ -357,6 +357,10 @@ HX_API void hx_destroy(hx_ctx* c) {
     if (c->net.ev_x[i]) cudaEventDestroy(c->net.ev_x[i]);
   }
   if (c->net.ev_fork) cudaEventDestroy(c->net.ev_fork);
+  for (auto& st : c->gmg.side)
+    if (st) cudaStreamDestroy(st);
+  for (auto& e : {c->gmg.ev_fork, c->gmg.ev_join[0], c->gmg.ev_join[1]})
+    if (e) cudaEventDestroy(e);
   if (c->ev_in) cudaEventDestroy(c->ev_in);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;

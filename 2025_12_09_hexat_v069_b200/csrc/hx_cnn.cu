@@ -214,9 +214,11 @@ __device__ __forceinline__ void prolong_axis(int f, int nc, int (&i)[2], float (
 // sum of the weights inside the grid (a weighted average; for features).
 template <int CH>
 __global__ void k_restrict(const float* __restrict__ in, float* __restrict__ out, GridN gf,
-                           GridN gc, int normalise, const uint8_t* __restrict__ cmask) {
+                           GridN gc, int normalise, const uint8_t* __restrict__ cmask,
+                           const CgState* st) {
   pdl_wait();
   pdl_trigger();
+  if (st && st->status != HX_RUNNING) return;
   const int64_t nc = (int64_t)gc.nx * gc.ny * gc.nz;
   for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < nc;
        n += (int64_t)gridDim.x * blockDim.x) {
@@ -544,9 +546,11 @@ static size_t restrict_ys_smem(int cxw) {
 // Prolongation, the exact transpose of k_restrict (without normalisation):
 // fine[j][c] = (accumulate ? fine[j][c] : 0) + sum_{i: |j - 2i| <= 1} w(j - 2i) coarse[i][c].
 __global__ void k_prolong(const float* __restrict__ coarse, float* __restrict__ fine, GridN gf,
-                          GridN gc, int accumulate, const uint8_t* __restrict__ fmask) {
+                          GridN gc, int accumulate, const uint8_t* __restrict__ fmask,
+                          const CgState* st) {
   pdl_wait();
   pdl_trigger();
+  if (st && st->status != HX_RUNNING) return;
   const int64_t nf = (int64_t)gf.nx * gf.ny * gf.nz;
   for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < nf;
        n += (int64_t)gridDim.x * blockDim.x) {
@@ -834,23 +838,25 @@ void launch_restrict_ys(cudaStream_t s, const __nv_bfloat16* ys, const CgState* 
 }
 
 void launch_restrict(cudaStream_t s, int ch, const float* in, float* out, const GridN& gf,
-                     const GridN& gc, bool normalise, const uint8_t* cmask) {
+                     const GridN& gc, bool normalise, const uint8_t* cmask, const CgState* st) {
   const int64_t nc = (int64_t)gc.nx * gc.ny * gc.nz;
   HX_REQUIRE(ch == 3 || !cmask, "a DOF mask needs 3 channels");
   if (ch == 3)
-    launch_pdl(k_restrict<3>, vec_blocks(nc), 256, 0, s, in, out, gf, gc, normalise ? 1 : 0, cmask);
+    launch_pdl(k_restrict<3>, vec_blocks(nc), 256, 0, s, in, out, gf, gc, normalise ? 1 : 0, cmask,
+               st);
   else if (ch == 1)
     launch_pdl(k_restrict<1>, vec_blocks(nc), 256, 0, s, in, out, gf, gc, normalise ? 1 : 0,
-               (const uint8_t*)nullptr);
+               (const uint8_t*)nullptr, st);
   else
     throw Error{HX_BAD_ARG, "unsupported channel count"};
   HX_CHECK_LAUNCH();
 }
 
 void launch_prolong(cudaStream_t s, const float* coarse, float* fine, const GridN& gf,
-                    const GridN& gc, bool accumulate, const uint8_t* fmask) {
+                    const GridN& gc, bool accumulate, const uint8_t* fmask, const CgState* st) {
   const int64_t nf = (int64_t)gf.nx * gf.ny * gf.nz;
-  launch_pdl(k_prolong, vec_blocks(nf), 256, 0, s, coarse, fine, gf, gc, accumulate ? 1 : 0, fmask);
+  launch_pdl(k_prolong, vec_blocks(nf), 256, 0, s, coarse, fine, gf, gc, accumulate ? 1 : 0, fmask,
+             st);
   HX_CHECK_LAUNCH();
 }
 

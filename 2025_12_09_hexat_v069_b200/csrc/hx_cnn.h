@@ -54,11 +54,13 @@ void launch_restrict_ys(cudaStream_t s, const __nv_bfloat16* ys, const CgState* 
                         double scale_mul, float* out, const GridN& gf, const GridN& gc);
 // full-weighting restriction fine -> coarse node grid (ch 3 or 1), and its
 // transpose; an optional node mask (3 channels: free-DOF bits) zeroes the
-// fixed components of the output
+// fixed components of the output; with st, nothing once that state has stopped
 void launch_restrict(cudaStream_t s, int ch, const float* in, float* out, const GridN& gf,
-                     const GridN& gc, bool normalise, const uint8_t* cmask = nullptr);
+                     const GridN& gc, bool normalise, const uint8_t* cmask = nullptr,
+                     const CgState* st = nullptr);
 void launch_prolong(cudaStream_t s, const float* coarse, float* fine, const GridN& gf,
-                    const GridN& gc, bool accumulate, const uint8_t* fmask = nullptr);
+                    const GridN& gc, bool accumulate, const uint8_t* fmask = nullptr,
+                    const CgState* st = nullptr);
 // lifting E: [node][3] FP32 -> 16-channel BF16 activation (x, feat * x), and its transpose
 void launch_lift(cudaStream_t s, const float* x, const float* feat, __nv_bfloat16* X,
                  const GridN& g);

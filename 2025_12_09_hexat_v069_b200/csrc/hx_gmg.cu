@@ -84,16 +84,20 @@ __global__ void k_coarse_bc(const uint8_t* __restrict__ bf, uint8_t* __restrict_
 
 // first Chebyshev step from x = 0: x = (1/theta) M^-1 b
 __global__ void k_cheb_first(const float* __restrict__ b, const float* __restrict__ minv,
-                             float* __restrict__ x, float inv_theta, int64_t n) {
+                             float* __restrict__ x, float inv_theta, int64_t n,
+                             const CgState* st) {
   pdl_wait();
   pdl_trigger();
+  if (st && st->status != HX_RUNNING) return;
   for (int64_t i = gt(); i < n; i += gs()) x[i] = inv_theta * minv[i] * b[i];
 }
 
 template <typename TD, typename TS>
-__global__ void k_copy_cvt(TD* __restrict__ d, const TS* __restrict__ s, int64_t n) {
+__global__ void k_copy_cvt(TD* __restrict__ d, const TS* __restrict__ s, int64_t n,
+                           const CgState* st) {
   pdl_wait();
   pdl_trigger();
+  if (st && st->status != HX_RUNNING) return;
   for (int64_t i = gt(); i < n; i += gs()) d[i] = (TD)s[i];
 }
 
@@ -218,83 +222,152 @@ __global__ void k_dense_mask(double* __restrict__ A, const uint8_t* __restrict__
   }
 }
 
-// Blocked in-place Gauss-Jordan inversion (no pivoting: the matrix is
-// symmetric positive definite), GJB pivots per step.  With K the step's
-// block of rows and columns, P = inv(A_KK):
-//   A_KJ <- P A_KJ,  A_IJ <- A_IJ - A_IK P A_KJ,  A_IK <- -A_IK P,  A_KK <- P
-// (I, J outside K), in three launches: the pivot block's inverse, the row
-// panel P A_KJ and a copy of the column panel A_IK into buffers, and the
-// update of every other entry from the buffers (so no entry is read after
-// another thread rewrote it).
-constexpr int GJB = 32;
+// Blocked Gauss-Jordan inversion (no pivoting: the matrix is symmetric positive
+// definite), GJB pivots per step, one launch per step.  With K the step's block
+// of rows and columns and P = inv(A_KK):
+//   B_KJ = P A_KJ,  B_IJ = A_IJ - A_IK P A_KJ,  B_IK = -A_IK P,  B_KK = P
+// (I, J outside K).  A step reads A and writes another matrix B, so that no
+// entry is read after another CTA rewrote it; each CTA forms its part of P A_KJ
+// again (32 x 64 of it for a 64 x 64 tile).  The CTA whose tile holds the next
+// pivot block inverts that block before it ends (it is the first to start).
+// Bound by the chain from one pivot block to the next (launch, L2 reads, the
+// block's own 32 dependent pivots): 46 steps for 1275 DOFs took 2.5 ms as three
+// launches per step (a one-CTA pivot kernel, panels, update) and take about 1 ms.
+constexpr int GJB = 32, GJT = 64, GJ_NT = 256;
 
-// A_KK <- inv(A_KK) in shared memory: unblocked Gauss-Jordan, one thread
-// per entry (GJB x GJB threads), b <= GJB rows.
-__global__ void k_gj_pivot_block(double* __restrict__ A, int64_t n, int64_t k0, int b) {
-  __shared__ double P[GJB][GJB + 1];
-  const int i = threadIdx.y, j = threadIdx.x;
-  const bool in = i < b && j < b;
-  P[i][j] = in ? A[(k0 + i) * n + k0 + j] : 0.0;
-  __syncthreads();
-  for (int k = 0; k < b; ++k) {
-    const double inv = 1.0 / P[k][k];
-    const double aik = P[i][k], akj = P[k][j], aij = P[i][j];
-    double v;
-    if (i == k && j == k)
-      v = inv;
-    else if (i == k)
-      v = akj * inv;
-    else if (j == k)
-      v = -aik * inv;
-    else
-      v = aij - aik * akj * inv;
-    __syncthreads();
-    P[i][j] = v;
-    __syncthreads();
-  }
-  if (in) A[(k0 + i) * n + k0 + j] = P[i][j];
-}
-
-// rowbuf[m][j] = (P A_KJ)[m][j] for every column j (used for j outside K);
-// colbuf[i][m] = A[i][k0 + m] for every row i (used for i outside K).
-__global__ void k_gj_panels(const double* __restrict__ A, int64_t n, int64_t k0, int b,
-                            double* __restrict__ rowbuf, double* __restrict__ colbuf) {
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < b * n;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t m = t / n, j = t - m * n;
-    double s = 0.0;
-    for (int q = 0; q < b; ++q) s += A[(k0 + m) * n + k0 + q] * A[(k0 + q) * n + j];
-    rowbuf[m * n + j] = s;
-    const int64_t i = t / b, m2 = t - i * b;
-    colbuf[i * GJB + m2] = A[i * n + k0 + m2];
-  }
-}
-
-__global__ void k_gj_update(double* __restrict__ A, int64_t n, int64_t k0, int b,
-                            const double* __restrict__ rowbuf, const double* __restrict__ colbuf) {
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n * n;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = t / n, j = t - i * n;
-    const bool iK = i >= k0 && i < k0 + b, jK = j >= k0 && j < k0 + b;
-    if (iK) {
-      if (!jK) A[t] = rowbuf[(i - k0) * n + j];
-    } else if (jK) {
-      double s = 0.0;
-      for (int m = 0; m < b; ++m) s += colbuf[i * GJB + m] * A[(k0 + m) * n + j];
-      A[t] = -s;
-    } else {
-      double s = A[t];
-      for (int m = 0; m < b; ++m) s -= colbuf[i * GJB + m] * rowbuf[m * n + j];
-      A[t] = s;
+// M <- inv(M) in shared memory by unblocked Gauss-Jordan (GJ_NT threads),
+// b <= GJB rows; rows past b hold the identity.
+__device__ __forceinline__ void gj_invert(double (*M)[GJB + 1]) {
+  const int j = threadIdx.x % GJB, i0 = threadIdx.x / GJB;  // rows i0, i0 + 8, ...
+  constexpr int PER = GJB * GJB / GJ_NT, ST = GJ_NT / GJB;
+  for (int k = 0; k < GJB; ++k) {
+    const double inv = 1.0 / M[k][k], akj = M[k][j];
+    double v[PER];
+#pragma unroll
+    for (int q = 0; q < PER; ++q) {
+      const int i = i0 + q * ST;
+      const double aik = M[i][k], aij = M[i][j];
+      if (i == k)
+        v[q] = j == k ? inv : akj * inv;
+      else
+        v[q] = j == k ? -aik * inv : aij - aik * akj * inv;
     }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < PER; ++q) M[i0 + q * ST][j] = v[q];
+    __syncthreads();
   }
 }
 
-template <typename TD>
-__global__ void k_cvt_f64(TD* __restrict__ d, const double* __restrict__ s, int64_t n) {
-  for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < n;
-       t += (int64_t)gridDim.x * blockDim.x)
-    d[t] = (TD)s[t];
+// P <- inv of the first pivot block of A
+__global__ void __launch_bounds__(GJ_NT)
+    k_gj_first(const double* __restrict__ A, int n, double* __restrict__ P) {
+  __shared__ double M[GJB][GJB + 1];
+  for (int t = threadIdx.x; t < GJB * GJB; t += GJ_NT) {
+    const int i = t / GJB, j = t % GJB;
+    M[i][j] = i < n && j < n ? A[(int64_t)i * n + j] : (i == j ? 1.0 : 0.0);
+  }
+  __syncthreads();
+  gj_invert(M);
+  for (int t = threadIdx.x; t < GJB * GJB; t += GJ_NT) P[t] = M[t / GJB][t % GJB];
+}
+
+struct GjSmem {
+  double col[GJT][GJB + 1];  // A_IK of the tile's rows
+  double row[GJB][GJT];      // A_KJ of the tile's columns
+  double pr[GJB][GJT];       // P A_KJ (P itself in the columns of K)
+  double p[GJB][GJB + 1];    // P, then the next pivot block
+};
+
+// Step on pivots k0 .. k0 + GJB - 1 with their block's inverse in P; Pn receives
+// the next block's.  The last step also writes the FP32 inverse.
+__global__ void __launch_bounds__(GJ_NT)
+    k_gj_step(const double* __restrict__ A, double* __restrict__ B, int n, int k0,
+              const double* __restrict__ P, double* __restrict__ Pn, float* __restrict__ out32) {
+  pdl_wait();
+  pdl_trigger();
+  extern __shared__ __align__(16) unsigned char gsm[];
+  GjSmem& sm = *reinterpret_cast<GjSmem*>(gsm);
+  const int tiles = (n + GJT - 1) / GJT, k1 = k0 + GJB;
+  // block 0 takes the diagonal tile of the next pivot block
+  const int diag = min(k1 / GJT, tiles - 1) * (tiles + 1);
+  const int id = ((int)blockIdx.x + diag) % (tiles * tiles);
+  const int i0 = id / tiles * GJT, j0 = id % tiles * GJT;
+  const int tid = threadIdx.x;
+  for (int t = tid; t < GJT * GJB; t += GJ_NT) {
+    const int i = t / GJB, m = t % GJB;
+    sm.col[i][m] = i0 + i < n && k0 + m < n ? A[(int64_t)(i0 + i) * n + k0 + m] : 0.0;
+    const int q = t / GJT, j = t % GJT;
+    sm.row[q][j] = k0 + q < n && j0 + j < n ? A[(int64_t)(k0 + q) * n + j0 + j] : 0.0;
+  }
+  for (int t = tid; t < GJB * GJB; t += GJ_NT) sm.p[t / GJB][t % GJB] = P[t];
+  __syncthreads();
+  {
+    const int j = tid % GJT, m0 = tid / GJT * 8;  // 8 rows of one column
+    const int jk = j0 + j - k0;
+    double acc[8];
+#pragma unroll
+    for (int m = 0; m < 8; ++m) acc[m] = 0.0;
+    if (jk >= 0 && jk < GJB) {
+#pragma unroll
+      for (int m = 0; m < 8; ++m) acc[m] = sm.p[m0 + m][jk];
+    } else {
+#pragma unroll 4
+      for (int q = 0; q < GJB; ++q) {
+        const double v = sm.row[q][j];
+#pragma unroll
+        for (int m = 0; m < 8; ++m) acc[m] = fma(sm.p[m0 + m][q], v, acc[m]);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < 8; ++m) sm.pr[m0 + m][j] = acc[m];
+  }
+  __syncthreads();
+  // rows ti, ti + 16, ..., columns tj, tj + 16, ...
+  const int ti = tid / 16, tj = tid % 16;
+  double s[4][4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int i = i0 + ti + 16 * a, j = j0 + tj + 16 * c;
+      const bool jk = j >= k0 && j < k1;
+      s[a][c] = i < n && j < n && !jk ? A[(int64_t)i * n + j] : 0.0;
+    }
+#pragma unroll 4
+  for (int m = 0; m < GJB; ++m) {
+    double u[4], v[4];
+#pragma unroll
+    for (int a = 0; a < 4; ++a) u[a] = sm.col[ti + 16 * a][m];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) v[c] = sm.pr[m][tj + 16 * c];
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) s[a][c] = fma(-u[a], v[c], s[a][c]);
+  }
+  const bool next = blockIdx.x == 0 && k1 < n;
+  if (next) {  // identity past the matrix's end; P has been used
+    __syncthreads();
+    for (int t = tid; t < GJB * GJB; t += GJ_NT)
+      sm.p[t / GJB][t % GJB] = t / GJB == t % GJB ? 1.0 : 0.0;
+    __syncthreads();
+  }
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int i = i0 + ti + 16 * a, j = j0 + tj + 16 * c;
+      if (i >= n || j >= n) continue;
+      if (i >= k0 && i < k1) s[a][c] = sm.pr[i - k0][j - j0];
+      B[(int64_t)i * n + j] = s[a][c];
+      if (out32) out32[(int64_t)i * n + j] = (float)s[a][c];
+      if (next && i >= k1 && i < k1 + GJB && j >= k1 && j < k1 + GJB) sm.p[i - k1][j - k1] = s[a][c];
+    }
+  if (!next) return;
+  __syncthreads();
+  gj_invert(sm.p);
+  for (int t = tid; t < GJB * GJB; t += GJ_NT) Pn[t] = sm.p[t / GJB][t % GJB];
 }
 
 // x = Ainv b (n x n, FP32): one warp per row, b read through the cache
@@ -381,11 +454,11 @@ void gmg_setup(hx_ctx* c, const double* fac, double shift) {
     L.d.ensure(n);
     L.q.ensure(n);
     if (l == 0) {
-      k_copy_cvt<float, double><<<gblocks(ne), 256, 0, s>>>(fl, fac, ne);
+      k_copy_cvt<float, double><<<gblocks(ne), 256, 0, s>>>(fl, fac, ne, nullptr);
       HX_CHECK_LAUNCH();
       HX_CUDA(cudaMemcpyAsync(bc, c->d_bcfree.p, nn, cudaMemcpyDeviceToDevice, s));
       HX_CUDA(cudaMemcpyAsync(nm, c->d_nmask.p, nn, cudaMemcpyDeviceToDevice, s));
-      k_copy_cvt<float, double><<<gblocks(n), 256, 0, s>>>(minv, c->d_minv.p, n);
+      k_copy_cvt<float, double><<<gblocks(n), 256, 0, s>>>(minv, c->d_minv.p, n, nullptr);
       HX_CHECK_LAUNCH();
       L.shift = (float)shift;
     } else {
@@ -400,11 +473,10 @@ void gmg_setup(hx_ctx* c, const double* fac, double shift) {
       // free rigid mode on the mesh then keeps the coarse operators (and
       // the dense coarsest inverse) nonsingular too.
       L.shift = 8.f * F.shift;
-      put_state(c, 3, CgState{});
+      HX_CUDA(cudaMemsetAsync(c->d_state.p + 3, 0, sizeof(CgState), s));
       launch_node_diag<float>(s, fl, bc, nm, minv, g, make_elem_coef(h[0], h[1], h[2], c->nu),
                               c->d_partials.p, c->d_state.p + 3, c->d_scalars.p);
       launch_minv<float>(s, nm, minv, minv, nn, (double)L.shift);
-      HX_CUDA(cudaStreamSynchronize(s));  // the pinned state mirror is reused below
     }
     G.nl = l + 1;
     const bool even = g.nxe % 2 == 0 && g.nye % 2 == 0 && g.nze % 2 == 0;
@@ -419,37 +491,105 @@ void gmg_setup(hx_ctx* c, const double* fac, double shift) {
     g = gc;
     for (int a = 0; a < 3; ++a) h[a] *= 2.0;
   }
+  if (!G.ev_fork) {
+    for (auto& e : {&G.ev_fork, &G.ev_join[0], &G.ev_join[1]})
+      HX_CUDA(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
+    for (auto& st : G.side) HX_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+  }
+  // Three parts that need only the levels built above, side by side: lambda_max
+  // of level 0 on the solve's stream, lambda_max of the other levels (whose
+  // kernels leave most SMs idle) on one side stream, the coarsest level's dense
+  // inverse on the other (set-up at 320 x 160 x 160 8.0 -> 4.7 ms, with the
+  // one-launch Gauss-Jordan steps).
+  HX_CUDA(cudaEventRecord(G.ev_fork, s));
+  for (auto& st : G.side) HX_CUDA(cudaStreamWaitEvent(st, G.ev_fork, 0));
   // lambda_max(D^-1 A) of every smoothed level (all but the coarsest), from
   // the Lanczos tridiagonal of GMG_LANCZOS Jacobi-PCG steps on a random
   // right-hand side.  The largest Ritz value converges to lambda_max from
   // below much faster than power iteration; an estimate below lambda_max
   // leaves the top of the spectrum outside the Chebyshev interval, where
   // the smoother is not positive definite.
-  G.p0.ensure(G.lv[0].g.dofs());
-  G.p1.ensure(G.lv[0].g.dofs());
+  int64_t pdofs = 0;
+  for (int l = 0; l < G.nl; ++l) pdofs += (G.lv[l].g.dofs() + 3) / 4 * 4;  // 16-byte offsets
+  G.p0.ensure(pdofs);
+  G.p1.ensure(pdofs);
+  double* rec = G.lanczos.ensure(3 * GMG_LANCZOS * HX_GMG_MAX_LEVELS);
+  CgState* lst = G.lan_st.ensure(HX_GMG_MAX_LEVELS);
+  HX_CUDA(cudaMemsetAsync(lst, 0, HX_GMG_MAX_LEVELS * sizeof(CgState), s));
+  HX_CUDA(cudaEventRecord(G.ev_join[0], s));
+  HX_CUDA(cudaStreamWaitEvent(G.side[0], G.ev_join[0], 0));
+  // the second half of the partial sums serves the side stream: a launch leaves
+  // at most two per CTA, and the workspace holds four for the largest grid
+  double* part[2] = {c->d_partials.p, c->d_partials.p + c->d_partials.n / 2};
+  int64_t off = 0;
   for (int l = 0; l + 1 < G.nl; ++l) {
     auto& L = G.lv[l];
     const int64_t nn = L.g.nodes(), n = L.g.dofs();
-    CgState* st = c->d_state.p + 3;
-    k_rand_vec<<<gblocks(n), 256, 0, s>>>(L.b.p, L.nmask.p, nn);
+    cudaStream_t ls = l == 0 ? s : G.side[0];
+    double* lp = part[l == 0 ? 0 : 1];
+    float *p0 = G.p0.p + off, *p1 = G.p1.p + off;
+    off += (n + 3) / 4 * 4;
+    CgState* st = lst + l;
+    k_rand_vec<<<gblocks(n), 256, 0, ls>>>(L.b.p, L.nmask.p, nn);
     HX_CHECK_LAUNCH();
-    launch_fill_zero(s, L.x.p, n * sizeof(float));
-    put_state(c, 3, fresh_state(0.0, 1 << 30, 1, false, false));
-    launch_cg_init<float>(s, L.b.p, nullptr, L.minv.p, L.r.p, G.p1.p, n, st, c->d_partials.p);
+    launch_fill_zero(ls, L.x.p, n * sizeof(float));
+    k_coarse_reset<<<1, 32, 0, ls>>>(st, 1 << 30, 0.0);
+    HX_CHECK_LAUNCH();
+    launch_cg_init<float>(ls, L.b.p, nullptr, L.minv.p, L.r.p, p1, n, st, lp);
     // all steps queued at once; each leaves (alpha, beta, status) in rec
-    double* rec = G.lanczos.ensure(3 * GMG_LANCZOS);
     for (int it = 0; it < GMG_LANCZOS; ++it) {
-      float* pin = (it % 2 == 0) ? G.p1.p : G.p0.p;
-      float* pout = (it % 2 == 0) ? G.p0.p : G.p1.p;
-      launch_pcg_step<float>(s, pin, pout, L.r.p, L.minv.p, L.x.p, L.q.p, L.fac.p, L.nmask.p, L.g,
-                             L.K, L.shift, st, c->d_partials.p);
-      launch_cg_update2<float>(s, L.r.p, L.q.p, L.minv.p, n, st, c->d_partials.p);
-      k_record_step<<<1, 32, 0, s>>>(st, rec + 3 * it);
+      launch_pcg_step<float>(ls, it % 2 == 0 ? p1 : p0, it % 2 == 0 ? p0 : p1, L.r.p, L.minv.p,
+                             L.x.p, L.q.p, L.fac.p, L.nmask.p, L.g, L.K, L.shift, st, lp);
+      launch_cg_update2<float>(ls, L.r.p, L.q.p, L.minv.p, n, st, lp);
+      k_record_step<<<1, 32, 0, ls>>>(st, rec + 3 * (l * GMG_LANCZOS + it));
       HX_CHECK_LAUNCH();
     }
-    double h[3 * GMG_LANCZOS];
-    HX_CUDA(cudaMemcpyAsync(h, rec, sizeof(h), cudaMemcpyDeviceToHost, s));
-    HX_CUDA(cudaStreamSynchronize(s));
+  }
+  // Coarsest level: its dense inverse when small enough (blocked
+  // Gauss-Jordan in FP64), else a fixed-count FP32 PCG at every cycle.
+  {
+    auto& L = G.lv[G.nl - 1];
+    const int64_t n = L.g.dofs();
+    G.direct = n <= GMG_DIRECT_DOFS;
+    if (G.direct) {
+      cudaStream_t ds = G.side[1];
+      const int64_t nn2 = n * n;
+      double* A = G.dense.ensure(2 * nn2);  // the matrix before and after a step
+      double* B = A + nn2;
+      double* P = G.gj.ensure(2 * GJB * GJB);  // inverse pivot blocks
+      float* ainv = G.ainv.ensure(nn2);
+      HX_CUDA(cudaMemsetAsync(A, 0, nn2 * sizeof(double), ds));
+      const ElemCoef<double> K = make_elem_coef(L.h[0], L.h[1], L.h[2], c->nu);
+      k_dense_assemble<<<gblocks(L.g.elems() * 24), 256, 0, ds>>>(L.fac.p, L.g, K, A, n);
+      HX_CHECK_LAUNCH();
+      k_dense_mask<<<gblocks(nn2), 256, 0, ds>>>(A, L.nmask.p, (double)L.shift, n);
+      HX_CHECK_LAUNCH();
+      k_gj_first<<<1, GJ_NT, 0, ds>>>(A, (int)n, P);
+      HX_CHECK_LAUNCH();
+      static PerDeviceOnce configured;
+      configured.run([&] {
+        HX_CUDA(cudaFuncSetAttribute(k_gj_step, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(GjSmem)));
+      });
+      const unsigned tiles = cdiv(n, GJT);
+      for (int64_t k0 = 0, i = 0; k0 < n; k0 += GJB, ++i) {
+        launch_dep(true, k_gj_step, tiles * tiles, GJ_NT, sizeof(GjSmem), ds, A, B, (int)n,
+                   (int)k0, P + (i & 1) * GJB * GJB, P + ((i + 1) & 1) * GJB * GJB,
+                   k0 + GJB < n ? (float*)nullptr : ainv);
+        HX_CHECK_LAUNCH();
+        std::swap(A, B);
+      }
+    }
+  }
+  for (int i = 0; i < 2; ++i) {
+    HX_CUDA(cudaEventRecord(G.ev_join[i], G.side[i]));
+    HX_CUDA(cudaStreamWaitEvent(s, G.ev_join[i], 0));
+  }
+  double hrec[3 * GMG_LANCZOS * HX_GMG_MAX_LEVELS];
+  HX_CUDA(cudaMemcpyAsync(hrec, rec, sizeof(hrec), cudaMemcpyDeviceToHost, s));
+  HX_CUDA(cudaStreamSynchronize(s));
+  for (int l = 0; l + 1 < G.nl; ++l) {
+    const double* h = hrec + 3 * l * GMG_LANCZOS;
     std::vector<double> al, be;
     for (int it = 0; it < GMG_LANCZOS; ++it) {
       const double a = h[3 * it], bt = h[3 * it + 1];
@@ -459,36 +599,7 @@ void gmg_setup(hx_ctx* c, const double* fac, double shift) {
       be.push_back(bt);
       if (stt != HX_RUNNING) break;
     }
-    L.lmax = al.empty() ? 2.0f : (float)lanczos_max(al, be);
-  }
-  // Coarsest level: its dense inverse when small enough (blocked
-  // Gauss-Jordan in FP64), else a fixed-count FP32 PCG at every cycle.
-  {
-    auto& L = G.lv[G.nl - 1];
-    const int64_t n = L.g.dofs();
-    G.direct = n <= GMG_DIRECT_DOFS;
-    if (G.direct) {
-      const int64_t nn2 = n * n;
-      double* A = G.dense.ensure(nn2);
-      double* gj = G.gj.ensure(2 * GJB * n);  // row panel [GJB][n], column panel [n][GJB]
-      HX_CUDA(cudaMemsetAsync(A, 0, nn2 * sizeof(double), s));
-      const ElemCoef<double> K = make_elem_coef(L.h[0], L.h[1], L.h[2], c->nu);
-      k_dense_assemble<<<gblocks(L.g.elems() * 24), 256, 0, s>>>(L.fac.p, L.g, K, A, n);
-      HX_CHECK_LAUNCH();
-      k_dense_mask<<<gblocks(nn2), 256, 0, s>>>(A, L.nmask.p, (double)L.shift, n);
-      HX_CHECK_LAUNCH();
-      for (int64_t k0 = 0; k0 < n; k0 += GJB) {
-        const int b = (int)std::min<int64_t>(GJB, n - k0);
-        k_gj_pivot_block<<<1, dim3(GJB, GJB), 0, s>>>(A, n, k0, b);
-        HX_CHECK_LAUNCH();
-        k_gj_panels<<<gblocks(b * n), 256, 0, s>>>(A, n, k0, b, gj, gj + GJB * n);
-        HX_CHECK_LAUNCH();
-        k_gj_update<<<gblocks(nn2), 256, 0, s>>>(A, n, k0, b, gj, gj + GJB * n);
-        HX_CHECK_LAUNCH();
-      }
-      k_cvt_f64<float><<<gblocks(nn2), 256, 0, s>>>(G.ainv.ensure(nn2), A, nn2);
-      HX_CHECK_LAUNCH();
-    }
+    G.lv[l].lmax = al.empty() ? 2.0f : (float)lanczos_max(al, be);
   }
   // the coarse solve's state: zeroed once, so that its reduction tickets
   // start at 0 (k_coarse_reset renews the other fields every cycle)
@@ -496,8 +607,6 @@ void gmg_setup(hx_ctx* c, const double* fac, double shift) {
     G.coarse_st.ensure(1);
     HX_CUDA(cudaMemsetAsync(G.coarse_st.p, 0, sizeof(CgState), s));
   }
-  G.p0.ensure(G.lv[G.nl - 1].g.dofs());
-  G.p1.ensure(G.lv[G.nl - 1].g.dofs());
   G.ready = true;
   HX_CUDA(cudaStreamSynchronize(s));
   G.setup_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() -
@@ -514,7 +623,7 @@ void gmg_setup(hx_ctx* c, const double* fac, double shift) {
 // x_k and x_{k-1} alternate between x and L.d; the start is chosen so
 // that the result lands in x.
 static void cheb_smooth(hx_ctx* c, hx_ctx::GmgLevel& L, const float* b, float* x, bool xzero,
-                        bool want_residual) {
+                        bool want_residual, const CgState* st) {
   cudaStream_t s = c->stream;
   const int64_t n = L.g.dofs();
   const int m = c->gmg.degree;
@@ -528,7 +637,7 @@ static void cheb_smooth(hx_ctx* c, hx_ctx::GmgLevel& L, const float* b, float* x
   if (xzero) {
     cur = (m % 2 == 1) ? 0 : 1;  // x_1 .. x_m alternate, x_m in L.x
     launch_dep(small_vec(n), k_cheb_first, gblocks(n), 256, 0, s, b, L.minv.p, buf[cur], 1.0f / theta,
-               n);
+               n, st);
     HX_CHECK_LAUNCH();
     k = 1;
   } else {
@@ -550,18 +659,18 @@ static void cheb_smooth(hx_ctx* c, hx_ctx::GmgLevel& L, const float* b, float* x
     }
     // after a start from x = 0, x_prev = x_0 = 0
     launch_cheb_step<float>(s, buf[cur], buf[cur ^ 1], xzero && k == 1, b, L.minv.p, omega,
-                            gamma, L.fac.p, L.nmask.p, L.g, L.K, L.shift);
+                            gamma, L.fac.p, L.nmask.p, L.g, L.K, L.shift, st);
     cur ^= 1;
   }
   if (want_residual)
-    launch_residual<float>(s, x, b, L.r.p, L.fac.p, L.nmask.p, L.g, L.K, L.shift);
+    launch_residual<float>(s, x, b, L.r.p, L.fac.p, L.nmask.p, L.g, L.K, L.shift, st);
 }
 
 // z = V(r): one V-cycle on r (FP64 or FP32 DOF vector of level 0).
 // Every launch is on c->stream and needs no host round trip, so the cycle
 // can be captured in a CUDA graph.
 template <typename T>
-void gmg_vcycle(hx_ctx* c, const T* r, T* z) {
+void gmg_vcycle(hx_ctx* c, const T* r, T* z, const CgState* st) {
   auto& G = c->gmg;
   HX_REQUIRE(G.ready, "multigrid hierarchy not set up");
   cudaStream_t s = c->stream;
@@ -577,7 +686,7 @@ void gmg_vcycle(hx_ctx* c, const T* r, T* z) {
     b0 = r;
     x0 = z;
   } else {
-    launch_dep(small_vec(n0), k_copy_cvt<float, T>, gblocks(n0), 256, 0, s, L0.b.p, r, n0);
+    launch_dep(small_vec(n0), k_copy_cvt<float, T>, gblocks(n0), 256, 0, s, L0.b.p, r, n0, st);
     HX_CHECK_LAUNCH();
     b0 = L0.b.p;
     x0 = L0.x.p;
@@ -586,15 +695,18 @@ void gmg_vcycle(hx_ctx* c, const T* r, T* z) {
     b = l == 0 ? b0 : G.lv[l].b.p;
     x = l == 0 ? x0 : G.lv[l].x.p;
   };
+  // the test of the state costs a small kernel more than it can save
+  auto level_st = [&](int l) { return G.lv[l].g.dofs() > 500000 ? st : nullptr; };
   for (int l = 0; l + 1 < nl; ++l) {
     auto& L = G.lv[l];
     auto& C = G.lv[l + 1];
     const float* b;
     float* x;
     bx(l, b, x);
-    cheb_smooth(c, L, b, x, true, true);
+    cheb_smooth(c, L, b, x, true, true, level_st(l));
     // coarse right-hand side R r, zero on the coarse fixed DOFs
-    launch_restrict(s, 3, L.r.p, C.b.p, node_grid(L.g), node_grid(C.g), false, C.nmask.p);
+    launch_restrict(s, 3, L.r.p, C.b.p, node_grid(L.g), node_grid(C.g), false, C.nmask.p,
+                    level_st(l));
   }
   {
     auto& L = G.lv[nl - 1];
@@ -632,16 +744,16 @@ void gmg_vcycle(hx_ctx* c, const T* r, T* z) {
     float* x;
     bx(l, b, x);
     // x_l += P x_{l+1}, zero on the fixed DOFs; then post-smoothing from it
-    launch_prolong(s, C.x.p, x, node_grid(L.g), node_grid(C.g), true, L.nmask.p);
-    cheb_smooth(c, L, b, x, false, false);
+    launch_prolong(s, C.x.p, x, node_grid(L.g), node_grid(C.g), true, L.nmask.p, level_st(l));
+    cheb_smooth(c, L, b, x, false, false, level_st(l));
   }
   if constexpr (!std::is_same<T, float>::value) {
-    launch_dep(small_vec(n0), k_copy_cvt<T, float>, gblocks(n0), 256, 0, s, z, L0.x.p, n0);
+    launch_dep(small_vec(n0), k_copy_cvt<T, float>, gblocks(n0), 256, 0, s, z, L0.x.p, n0, st);
     HX_CHECK_LAUNCH();
   }
 }
-template void gmg_vcycle<double>(hx_ctx*, const double*, double*);
-template void gmg_vcycle<float>(hx_ctx*, const float*, float*);
+template void gmg_vcycle<double>(hx_ctx*, const double*, double*, const CgState*);
+template void gmg_vcycle<float>(hx_ctx*, const float*, float*, const CgState*);
 
 template <typename T>
 void launch_fcg_coeffs(cudaStream_t s, const T* z, const T* q_old, const T* r, int64_t n,
@@ -699,7 +811,7 @@ CgState solve_gmg(hx_ctx* c, const double* fac, const double* b, double* x, bool
   s0.beta = 0.0;
   put_state(c, 0, s0);
   auto one = [&](double* pin, double* pout) {
-    gmg_vcycle<double>(c, r, z);
+    gmg_vcycle<double>(c, r, z, st);
     launch_fcg_coeffs<double>(c->stream, z, q, r, n, c->d_partials.p, st);
     launch_fcg_step<double>(c->stream, pin, pout, z, x, q, fac, c->d_nmask.p, g, c->K, shift, st,
                             c->d_partials.p);

@@ -75,14 +75,15 @@ void launch_fcg_step(cudaStream_t s, const T* pin, T* pout, const T* z, T* x, T*
 // Multigrid smoothing (FP32): one Chebyshev step as a three-term recurrence,
 // xprev_new <- x + omega (x - xprev_new) + gamma M^-1 (b - (K + sI) x) on the
 // free DOFs (0 on the fixed ones; xprev_zero: x_prev = 0, not read); and the
-// residual r = mask(b - (K + sI) x).
+// residual r = mask(b - (K + sI) x).  With st: nothing once it has stopped.
 template <typename T>
 void launch_cheb_step(cudaStream_t s, const T* x, T* xprev_new, bool xprev_zero, const T* b,
                       const T* minv, T omega, T gamma, const T* fac, const uint8_t* nmask,
-                      const Grid& g, const ElemCoef<T>& K, T shift);
+                      const Grid& g, const ElemCoef<T>& K, T shift, const CgState* st = nullptr);
 template <typename T>
 void launch_residual(cudaStream_t s, const T* x, const T* b, T* r, const T* fac,
-                     const uint8_t* nmask, const Grid& g, const ElemCoef<T>& K, T shift);
+                     const uint8_t* nmask, const Grid& g, const ElemCoef<T>& K, T shift,
+                     const CgState* st = nullptr);
 template <typename T>
 void launch_node_diag(cudaStream_t s, const T* fac, const uint8_t* bcfree, uint8_t* nmask, T* diag,
                       const Grid& g, const ElemCoef<double>& K, double* partials, CgState* st,
@@ -250,9 +251,14 @@ struct hx_ctx {
     // direct coarsest-level solve: dense inverse (FP32, n x n) of the masked
     // coarsest operator, formed in FP64 at set-up
     bool direct = false;
-    hx::DevBuf<double> dense, gj;  // FP64 matrix being inverted; pivot row/column buffers
+    hx::DevBuf<double> dense, gj;  // FP64 matrix being inverted (two copies); pivot blocks
     hx::DevBuf<float> ainv;
-    hx::DevBuf<double> lanczos;  // (alpha, beta, status) per step of the lambda_max estimate
+    // lambda_max estimate: (alpha, beta, status) per level and step; CG states
+    hx::DevBuf<double> lanczos;
+    hx::DevBuf<hx::CgState> lan_st;
+    // set-up beside the solve's stream
+    cudaStream_t side[2] = {nullptr, nullptr};
+    cudaEvent_t ev_fork = nullptr, ev_join[2] = {nullptr, nullptr};
     double setup_ms = 0;         // set-up time accumulated over the current solve
     int degree = 2;              // Chebyshev degree per smoothing
   } gmg;

@@ -783,7 +783,7 @@ static CgState learned_fcg_mixed(hx_ctx* c, const double* fac, const double* b, 
   __nv_bfloat16* ys = multigrid ? nullptr : N.ys.ensure(n + 8);
   auto one = [&](float* pi, float* po) {
     if (multigrid) {
-      gmg_vcycle<float>(c, r32, z32);
+      gmg_vcycle<float>(c, r32, z32, si);
       launch_fcg_coeffs<float>(c->stream, z32, q32, r32, n, c->d_partials.p, si);
     } else {
       precond_z<float>(c, r32, minv32, si, scale_mul, z32, q32, false, ys);

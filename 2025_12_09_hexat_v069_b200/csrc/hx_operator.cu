@@ -412,7 +412,8 @@ __global__ void __launch_bounds__(MV_BX* Tile<T, mode_fused(MODE)>::WARPS,
   // everything above may overlap the previous kernel (launch_dep)
   pdl_wait();
   pdl_trigger();
-  if (FUSED && A.st->status != HX_RUNNING) return;
+  // MODE 5, 6 inside a solve stop with its state too
+  if ((FUSED || (MODE >= 5 && A.st)) && A.st->status != HX_RUNNING) return;
   T alpha_old = T(0), beta_old = T(0);
   if (FUSED) {
     alpha_old = (T)A.st->alpha;
@@ -1026,8 +1027,9 @@ template void launch_matvec<double>(cudaStream_t, int, const double*, double*, c
 template <typename T>
 void launch_cheb_step(cudaStream_t s, const T* x, T* xprev_new, bool xprev_zero, const T* b,
                       const T* minv, T omega, T gamma, const T* fac, const uint8_t* nmask,
-                      const Grid& g, const ElemCoef<T>& K, T shift) {
+                      const Grid& g, const ElemCoef<T>& K, T shift, const CgState* st) {
   launch_struct<T, 5>(s, fac, nmask, g, K, shift, [&](auto& a) {
+    a.st = const_cast<CgState*>(st);
     a.pin = x;
     a.x = xprev_new;
     a.xprev_zero = xprev_zero ? 1 : 0;
@@ -1039,12 +1041,14 @@ void launch_cheb_step(cudaStream_t s, const T* x, T* xprev_new, bool xprev_zero,
 }
 template void launch_cheb_step<float>(cudaStream_t, const float*, float*, bool, const float*,
                                       const float*, float, float, const float*, const uint8_t*,
-                                      const Grid&, const ElemCoef<float>&, float);
+                                      const Grid&, const ElemCoef<float>&, float, const CgState*);
 
 template <typename T>
 void launch_residual(cudaStream_t s, const T* x, const T* b, T* r, const T* fac,
-                     const uint8_t* nmask, const Grid& g, const ElemCoef<T>& K, T shift) {
+                     const uint8_t* nmask, const Grid& g, const ElemCoef<T>& K, T shift,
+                     const CgState* st) {
   launch_struct<T, 6>(s, fac, nmask, g, K, shift, [&](auto& a) {
+    a.st = const_cast<CgState*>(st);
     a.pin = x;
     a.r = b;
     a.q = r;
@@ -1052,7 +1056,7 @@ void launch_residual(cudaStream_t s, const T* x, const T* b, T* r, const T* fac,
 }
 template void launch_residual<float>(cudaStream_t, const float*, const float*, float*,
                                      const float*, const uint8_t*, const Grid&,
-                                     const ElemCoef<float>&, float);
+                                     const ElemCoef<float>&, float, const CgState*);
 
 template <typename T>
 void launch_pcg_step(cudaStream_t s, const T* pin, T* pout, const T* r, const T* minv, T* x, T* q,

@@ -102,8 +102,10 @@ hx_status export_webdata(hx_ctx* c, const char* path, const T* dens, const T* l1
 // default Chebyshev degree of the multigrid smoothing
 constexpr int GMG_DEFAULT_DEGREE = 2;
 void gmg_setup(hx_ctx* c, const double* fac, double shift);
+// st: the flexible-CG state that the cycle belongs to (its kernels on large
+// levels do nothing once that has stopped), or null
 template <typename T>
-void gmg_vcycle(hx_ctx* c, const T* r, T* z);
+void gmg_vcycle(hx_ctx* c, const T* r, T* z, const CgState* st = nullptr);
 template <typename T>
 void launch_fcg_coeffs(cudaStream_t s, const T* z, const T* q_old, const T* r, int64_t n,
                        double* partials, CgState* st);
