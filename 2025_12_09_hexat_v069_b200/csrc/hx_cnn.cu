@@ -65,13 +65,18 @@ __device__ __forceinline__ unsigned swz(int row, int h) {
 // w+24 over all 512 nodes of the tile; the result goes to part[cta][27*256]
 // (FP32), summed later in fixed order.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(NTHREADS) k_conv3_wgrad(const __nv_bfloat16* __restrict__ X,
-                                                          const __nv_bfloat16* __restrict__ D,
-                                                          float* __restrict__ part, GridN g) {
+// One launch takes all 8 uses of a network's 4 layers (job = blockIdx.z mod 8:
+// layer job & 3, transposed use below 4, forward use from there on): a layer's
+// tiles alone leave most SMs idle on the coarse levels.
+__global__ void __launch_bounds__(NTHREADS)
+    k_conv3_wgrad(const __grid_constant__ WgradJobs jobs, float* __restrict__ part, GridN g) {
+  const int job = blockIdx.z & 7;
+  const __nv_bfloat16* __restrict__ X = jobs.X[job];
+  const __nv_bfloat16* __restrict__ D = jobs.D[job];
   extern __shared__ __align__(128) unsigned char smraw[];
   __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(smraw);
   __nv_bfloat16* ds = xs + HNODES * C;  // [512 nodes][16], swizzled rows
-  const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = blockIdx.z * TZ;
+  const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = (blockIdx.z >> 3) * TZ;
   const unsigned xb = su32(xs), db = su32(ds);
   for (int ch = threadIdx.x; ch < HNODES * 2; ch += NTHREADS) {
     const int node = ch >> 1, h = ch & 1;
@@ -94,8 +99,9 @@ __global__ void __launch_bounds__(NTHREADS) k_conv3_wgrad(const __nv_bfloat16* _
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gq = lane >> 2, tq = lane & 3;
-  float* out = part + (size_t)(blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)) *
-                          (27 * 256);
+  const size_t tile = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * (size_t)(blockIdx.z >> 3));
+  const size_t tiles = (size_t)gridDim.x * gridDim.y * (gridDim.z >> 3);
+  float* out = part + (job * tiles + tile) * (27 * 256);
   // ldmatrix.trans row addresses: matrix mi = lane/8, row r = lane%8
   const int mi = lane >> 3, rr = lane & 7;
   for (int tap = warp; tap < 27; tap += 8) {
@@ -133,14 +139,23 @@ __global__ void __launch_bounds__(NTHREADS) k_conv3_wgrad(const __nv_bfloat16* _
   }
 }
 
-// Sum the per-CTA partials in a fixed order: grad[k] (+)= sum_c part[c][k].
+// Sum the per-CTA partials in a fixed order, layer blockIdx.y: grad[k] (+)= the
+// sum over the tiles of its transposed use, then += that of its forward use.
 __global__ void k_reduce_parts(const float* __restrict__ part, int nparts, int len,
                                float* __restrict__ grad, int accumulate) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= len) return;
-  double s = 0.0;
-  for (int c = 0; c < nparts; ++c) s += (double)part[(size_t)c * len + k];
-  grad[k] = accumulate ? grad[k] + (float)s : (float)s;
+  const size_t job = (size_t)nparts * len;
+  const float* pt = part + blockIdx.y * job + k;
+  const float* pf = pt + 4 * job;
+  double t = 0.0, f = 0.0;
+#pragma unroll 4
+  for (int c = 0; c < nparts; ++c) {
+    t += (double)pt[(size_t)c * len];
+    f += (double)pf[(size_t)c * len];
+  }
+  float* gr = grad + (size_t)blockIdx.y * len + k;
+  *gr = (accumulate ? *gr + (float)t : (float)t) + (float)f;
 }
 
 // Adam step on the FP32 master parameters (weights [27][16][16] per layer,
@@ -170,6 +185,10 @@ __global__ void k_pack_weights(const float* __restrict__ w, __nv_bfloat16* __res
                                __nv_bfloat16* __restrict__ wb) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= 27 * 256) return;
+  const size_t layer = (size_t)blockIdx.y * 27 * 256;
+  w += layer;
+  wf += layer;
+  wb += layer;
   const int tap = k / 256, co = (k / 16) % 16, ci = k % 16;
   const int dz = tap / 9 - 1, s = tap % 9;
   const __nv_bfloat16 v = __float2bfloat16_rn(w[k]);
@@ -767,19 +786,21 @@ size_t conv_num_tiles(const GridN& g) {
   return (size_t)d.x * d.y * d.z;
 }
 
-void launch_conv3_wgrad(cudaStream_t s, const __nv_bfloat16* X, const __nv_bfloat16* D,
-                        float* part, float* grad, bool accumulate, const GridN& g) {
+void launch_conv3_wgrad(cudaStream_t s, const WgradJobs& jobs, float* part, float* grad,
+                        bool accumulate, const GridN& g) {
   const size_t smem = (HNODES + TX * TY * TZ) * C * sizeof(__nv_bfloat16);
   static PerDeviceOnce cfg;
   cfg.run([&] {
     HX_CUDA(cudaFuncSetAttribute(k_conv3_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)smem));
   });
-  k_conv3_wgrad<<<conv_grid(g), NTHREADS, smem, s>>>(X, D, part, g);
+  dim3 grid = conv_grid(g);
+  grid.z *= 8;
+  k_conv3_wgrad<<<grid, NTHREADS, smem, s>>>(jobs, part, g);
   HX_CHECK_LAUNCH();
   const int len = 27 * 256;
-  k_reduce_parts<<<cdiv(len, 256), 256, 0, s>>>(part, (int)conv_num_tiles(g), len, grad,
-                                                accumulate ? 1 : 0);
+  k_reduce_parts<<<dim3(cdiv(len, 256), NET_LAYERS), 256, 0, s>>>(part, (int)conv_num_tiles(g), len,
+                                                                  grad, accumulate ? 1 : 0);
   HX_CHECK_LAUNCH();
 }
 
@@ -791,8 +812,9 @@ void launch_adam(cudaStream_t s, float* w, float* m, float* v, const float* grad
   HX_CHECK_LAUNCH();
 }
 
-void launch_pack_weights(cudaStream_t s, const float* w, __nv_bfloat16* wf, __nv_bfloat16* wb) {
-  k_pack_weights<<<cdiv(27 * 256, 256), 256, 0, s>>>(w, wf, wb);
+void launch_pack_weights(cudaStream_t s, const float* w, __nv_bfloat16* wf, __nv_bfloat16* wb,
+                         int layers) {
+  k_pack_weights<<<dim3(cdiv(27 * 256, 256), layers), 256, 0, s>>>(w, wf, wb);
   HX_CHECK_LAUNCH();
 }
 

@@ -37,12 +37,20 @@ void launch_conv3(cudaStream_t s, int cout, const __nv_bfloat16* X, __nv_bfloat1
 // failure-detection self test: one CTA whose wait must run out (8 x 16 x 4 nodes)
 void launch_conv3_selftest(cudaStream_t s, const __nv_bfloat16* X, __nv_bfloat16* Y,
                            const __nv_bfloat16* W, int* err);
-// grad (+)= dW of one layer from the per-CTA partials
-void launch_conv3_wgrad(cudaStream_t s, const __nv_bfloat16* X, const __nv_bfloat16* D,
-                        float* part, float* grad, bool accumulate, const GridN& g);
+// The two uses of a network's layers: [l] the transposed use of layer l (X: the
+// gradient of its output, D: its input), [4 + l] the forward use (X: its input,
+// D: the gradient of its output).
+struct WgradJobs {
+  const __nv_bfloat16* X[2 * NET_LAYERS];
+  const __nv_bfloat16* D[2 * NET_LAYERS];
+};
+// grad (+)= dW of the network's layers; part: 8 conv_num_tiles(g) layers' worth
+void launch_conv3_wgrad(cudaStream_t s, const WgradJobs& jobs, float* part, float* grad,
+                        bool accumulate, const GridN& g);
 void launch_adam(cudaStream_t s, float* w, float* m, float* v, const float* grad,
                  const unsigned char* live, int n, float lr, int step);
-void launch_pack_weights(cudaStream_t s, const float* w, __nv_bfloat16* wf, __nv_bfloat16* wb);
+void launch_pack_weights(cudaStream_t s, const float* w, __nv_bfloat16* wf, __nv_bfloat16* wb,
+                         int layers);
 // level-1 field R (k D^-1/2 v) of a DOF vector, D^-1/2 = sqrt(minv) (k by
 // mode: 0 network input, 1 energy-loss gradient, 2 residual-loss gradient)
 template <typename T>

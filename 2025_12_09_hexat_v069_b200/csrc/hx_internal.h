@@ -284,12 +284,14 @@ struct hx_ctx {
   struct Net {
     bool ready = false;
     int step = 0;  // Adam steps taken
-    hx::DevBuf<float> w, m, v, grad, part;
+    hx::DevBuf<float> w, m, v, grad;
     hx::DevBuf<unsigned char> live;
-    hx::DevBuf<__nv_bfloat16> wf, wb, da, db, tmp[2];
+    hx::DevBuf<__nv_bfloat16> wf, wb, tmp[2];
     struct Level {  // one node-grid level (0 = the mesh's node grid)
       hx::DevBuf<float> x, acc, gx, feat;  // [node][3] fields, [node] feature
       hx::DevBuf<__nv_bfloat16> x0, y, act[7];  // network input, output, training activations
+      hx::DevBuf<__nv_bfloat16> ge[8];          // training: gradients (stack_backward_train)
+      hx::DevBuf<float> part;                   // training: weight-gradient partials
       hx::DevBuf<__nv_bfloat16> pp[2];          // application ping-pong (levels >= 2)
     } lv[8];
     // side streams and events: the coarser networks run beside the finest;

@@ -90,8 +90,7 @@ void check_conv_error(hx_ctx* c) {
 
 void net_pack(hx_ctx* c) {
   auto& N = c->net;
-  for (int l = 0; l < NET_PARAMS / LP; ++l)
-    launch_pack_weights(c->stream, N.w.p + l * LP, N.wf.p + l * LP, N.wb.p + l * LP);
+  launch_pack_weights(c->stream, N.w.p, N.wf.p, N.wb.p, NET_PARAMS / LP);
 }
 
 void net_upload(hx_ctx* c, const std::vector<float>& w) {
@@ -135,8 +134,11 @@ void net_buffers(hx_ctx* c, bool train) {
     if (l < NET_L0) continue;
     L.x0.ensure(nl * 16);
     L.y.ensure(nl * 8);
-    if (train)
+    if (train) {
       for (auto& a : L.act) a.ensure(nl * 16);
+      for (auto& a : L.ge) a.ensure(nl * 16);
+      L.part.ensure(2 * NET_LAYERS * conv_num_tiles(level_grid(c->g, l)) * LP);
+    }
     if (l > NET_L0)
       for (auto& b : L.pp) b.ensure(nl * 16);
   }
@@ -147,11 +149,6 @@ void net_buffers(hx_ctx* c, bool train) {
       HX_CUDA(cudaEventCreateWithFlags(&N.ev_join[i], cudaEventDisableTiming));
       HX_CUDA(cudaEventCreateWithFlags(&N.ev_x[i], cudaEventDisableTiming));
     }
-  }
-  if (train) {
-    N.da.ensure(a1);
-    N.db.ensure(a1);
-    N.part.ensure(conv_num_tiles(g1) * LP);
   }
 }
 
@@ -173,45 +170,43 @@ void stack_apply(hx_ctx* c, cudaStream_t s, int k, const GridN& g, const __nv_bf
 }
 
 // y = G_k^T G_k x0 keeping every activation: act = A1 A2 A3 H B3 B2 B1.
-void stack_forward_train(hx_ctx* c, int k, const GridN& g, const __nv_bfloat16* x0,
-                         DevBuf<__nv_bfloat16>* act, __nv_bfloat16* y) {
-  launch_conv3(c->stream, 16, x0, act[0].p, fwd_w(c, k, 0), g, c->net.err.p);
+void stack_forward_train(hx_ctx* c, cudaStream_t s, int k, const GridN& g,
+                         const __nv_bfloat16* x0, DevBuf<__nv_bfloat16>* act, __nv_bfloat16* y) {
+  launch_conv3(s, 16, x0, act[0].p, fwd_w(c, k, 0), g, c->net.err.p);
   for (int l = 1; l < 4; ++l)
-    launch_conv3(c->stream, 16, act[l - 1].p, act[l].p, fwd_w(c, k, l), g, c->net.err.p);
+    launch_conv3(s, 16, act[l - 1].p, act[l].p, fwd_w(c, k, l), g, c->net.err.p);
   for (int l = 3; l >= 1; --l)
-    launch_conv3(c->stream, 16, act[6 - l].p, act[7 - l].p, adj_w(c, k, l), g, c->net.err.p);
-  launch_conv3(c->stream, 8, act[6].p, y, adj_w(c, k, 0), g, c->net.err.p);
+    launch_conv3(s, 16, act[6 - l].p, act[7 - l].p, adj_w(c, k, l), g, c->net.err.p);
+  launch_conv3(s, 8, act[6].p, y, adj_w(c, k, 0), g, c->net.err.p);
 }
 
-// Gradients of network k into N.grad from da = dLoss/dB0 (16-channel
-// storage; overwritten).  B0 = G^T H with H = G x0: the G^T half is
-// differentiated first (E_{l+1} = dLoss/dB_{l+1} = W_l * E_l; the weight
-// gradient of a transposed use is wgrad(X = E_l, D = its input)), then the G
-// half from dLoss/dH = W_3 * E_3 (forward use: wgrad(X = its input,
-// D = dLoss/dout), dLoss/din = W^T * dLoss/dout).
-void stack_backward_train(hx_ctx* c, int k, const GridN& g, const __nv_bfloat16* x0,
-                          const DevBuf<__nv_bfloat16>* act, bool accumulate) {
-  auto& N = c->net;
-  float* grad = N.grad.p + k * NP;
-  __nv_bfloat16* e0 = N.da.p;
-  __nv_bfloat16* e1 = N.db.p;
-  // transposed uses: layer l maps B_{l+1} (H for l = 3) to B_l
+// Gradients of network k into N.grad from ge[0] = dLoss/dB0 (16-channel
+// storage).  B0 = G^T H with H = G x0: the G^T half is differentiated first
+// (ge[l + 1] = dLoss/dB_{l+1} = W_l * ge[l], up to dLoss/dH = ge[4]; the weight
+// gradient of a transposed use is wgrad(X = ge[l], D = its input)), then the G
+// half (forward use: wgrad(X = its input, D = dLoss/dout), dLoss/din = W^T *
+// dLoss/dout, kept in ge[5 ..]).  All gradients are kept, so that one launch
+// takes the weight gradients of all layers.
+void stack_backward_train(hx_ctx* c, cudaStream_t s, int k, const GridN& g,
+                          const __nv_bfloat16* x0, const DevBuf<__nv_bfloat16>* act,
+                          const DevBuf<__nv_bfloat16>* ge, float* part, bool accumulate) {
+  // transposed uses: layer l maps B_{l+1} (H for l = 3) to B_l; forward uses:
+  // layer l maps A_l (x0 for l = 0) to A_{l+1} (H for l = 3)
   const __nv_bfloat16* bin[4] = {act[6].p, act[5].p, act[4].p, act[3].p};
-  for (int l = 0; l < 4; ++l) {
-    launch_conv3_wgrad(c->stream, e0, bin[l], N.part.p, grad + l * LP, accumulate, g);
-    // E_{l+1}; l = 3: dLoss/dH
-    launch_conv3(c->stream, 16, e0, e1, fwd_w(c, k, l), g, c->net.err.p);
-    std::swap(e0, e1);
-  }
-  // forward uses: layer l maps A_l (x0 for l = 0) to A_{l+1} (H for l = 3)
   const __nv_bfloat16* ain[4] = {x0, act[0].p, act[1].p, act[2].p};
-  for (int l = 3; l >= 0; --l) {
-    launch_conv3_wgrad(c->stream, ain[l], e0, N.part.p, grad + l * LP, true, g);
-    if (l > 0) {
-      launch_conv3(c->stream, 16, e0, e1, adj_w(c, k, l), g, c->net.err.p);
-      std::swap(e0, e1);
-    }
+  WgradJobs jobs{};
+  for (int l = 0; l < 4; ++l) {
+    jobs.X[l] = ge[l].p;
+    jobs.D[l] = bin[l];
+    launch_conv3(s, 16, ge[l].p, ge[l + 1].p, fwd_w(c, k, l), g, c->net.err.p);
   }
+  for (int l = 3; l >= 0; --l) {
+    const __nv_bfloat16* d = ge[7 - l].p;  // dLoss/dout of layer l
+    jobs.X[4 + l] = ain[l];
+    jobs.D[4 + l] = d;
+    if (l > 0) launch_conv3(s, 16, d, ge[8 - l].p, adj_w(c, k, l), g, c->net.err.p);
+  }
+  launch_conv3_wgrad(s, jobs, part, c->net.grad.p + k * NP, accumulate, g);
 }
 
 // z = M^-1 r + s D^-1/2 sum_l R_l^T E_l^T G_l^T G_l E_l R_l (D^-1/2 r / s).
@@ -236,62 +231,53 @@ void precond_z(hx_ctx* c, const T* r, const T* minv, CgState* st, double scale_m
     ys = y;
   }
   launch_restrict_ys(c->stream, ys, st, scale_mul, N.lv[1].x.p, gl[0], gl[1]);
-  if (train) {
-    for (int l = 2; l <= NET_TOP; ++l)
-      launch_restrict(c->stream, 3, N.lv[l - 1].x.p, N.lv[l].x.p, gl[l - 1], gl[l], false);
-    for (int l = NET_TOP; l >= NET_L0; --l) {
-      auto& L = N.lv[l];
-      launch_lift(c->stream, L.x.p, L.feat.p, L.x0.p, gl[l]);
-      stack_forward_train(c, l - NET_L0, gl[l], L.x0.p, L.act, L.y.p);
+  auto stack = [&](cudaStream_t s, int l) {
+    auto& L = N.lv[l];
+    if (train)
+      stack_forward_train(c, s, l - NET_L0, gl[l], L.x0.p, L.act, L.y.p);
+    else
+      stack_apply(c, s, l - NET_L0, gl[l], L.x0.p, L.y.p, l == NET_L0 ? N.tmp[0].p : L.pp[0].p,
+                  l == NET_L0 ? N.tmp[1].p : L.pp[1].p);
+  };
+  for (int l = 2; l <= NET_L0; ++l)
+    launch_restrict(c->stream, 3, N.lv[l - 1].x.p, N.lv[l].x.p, gl[l - 1], gl[l], false);
+  // Each coarser network on its own side stream, the finest on the main
+  // one; a side stream also restricts its level's input (after its finer
+  // neighbour's, event ev_x) and sums its coarser neighbour's correction
+  // into its own (after ev_join of that neighbour), so that only the
+  // finest level's transfers stay on the main stream.  Inside a stream
+  // capture the events become edges between parallel graph branches.
+  HX_CUDA(cudaEventRecord(N.ev_fork, c->stream));
+  for (int l = NET_L0 + 1; l <= NET_TOP; ++l) {
+    const int side = l - NET_L0 - 1;
+    cudaStream_t ss = N.side[side];
+    auto& L = N.lv[l];
+    HX_CUDA(cudaStreamWaitEvent(ss, side == 0 ? N.ev_fork : N.ev_x[side - 1], 0));
+    launch_restrict(ss, 3, N.lv[l - 1].x.p, L.x.p, gl[l - 1], gl[l], false);
+    if (l < NET_TOP) HX_CUDA(cudaEventRecord(N.ev_x[side], ss));
+    launch_lift(ss, L.x.p, L.feat.p, L.x0.p, gl[l]);
+    stack(ss, l);
+  }
+  // corrections, coarsest first: acc_l = E_l^T y_l + R^T acc_{l+1}
+  for (int l = NET_TOP; l > NET_L0; --l) {
+    const int side = l - NET_L0 - 1;
+    cudaStream_t ss = N.side[side];
+    auto& L = N.lv[l];
+    launch_unlift(ss, L.y.p, L.feat.p, L.acc.p, false, nodes_of(gl[l]));
+    if (l < NET_TOP) {
+      HX_CUDA(cudaStreamWaitEvent(ss, N.ev_join[side + 1], 0));
+      launch_prolong(ss, N.lv[l + 1].acc.p, L.acc.p, gl[l], gl[l + 1], true);
     }
-    // acc_l = E_l^T y_l (network levels) + R^T acc_{l+1}, coarsest first
-    for (int l = NET_TOP; l >= NET_L0; --l) {
-      auto& L = N.lv[l];
-      launch_unlift(c->stream, L.y.p, L.feat.p, L.acc.p, false, nodes_of(gl[l]));
-      if (l < NET_TOP)
-        launch_prolong(c->stream, N.lv[l + 1].acc.p, L.acc.p, gl[l], gl[l + 1], true);
-    }
-  } else {
-    for (int l = 2; l <= NET_L0; ++l)
-      launch_restrict(c->stream, 3, N.lv[l - 1].x.p, N.lv[l].x.p, gl[l - 1], gl[l], false);
-    // Each coarser network on its own side stream, the finest on the main
-    // one; a side stream also restricts its level's input (after its finer
-    // neighbour's, event ev_x) and sums its coarser neighbour's correction
-    // into its own (after ev_join of that neighbour), so that only the
-    // finest level's transfers stay on the main stream.  Inside a stream
-    // capture the events become edges between parallel graph branches.
-    HX_CUDA(cudaEventRecord(N.ev_fork, c->stream));
-    for (int l = NET_L0 + 1; l <= NET_TOP; ++l) {
-      const int side = l - NET_L0 - 1;
-      cudaStream_t ss = N.side[side];
-      auto& L = N.lv[l];
-      HX_CUDA(cudaStreamWaitEvent(ss, side == 0 ? N.ev_fork : N.ev_x[side - 1], 0));
-      launch_restrict(ss, 3, N.lv[l - 1].x.p, L.x.p, gl[l - 1], gl[l], false);
-      if (l < NET_TOP) HX_CUDA(cudaEventRecord(N.ev_x[side], ss));
-      launch_lift(ss, L.x.p, L.feat.p, L.x0.p, gl[l]);
-      stack_apply(c, ss, l - NET_L0, gl[l], L.x0.p, L.y.p, L.pp[0].p, L.pp[1].p);
-    }
-    // corrections, coarsest first: acc_l = E_l^T y_l + R^T acc_{l+1}
-    for (int l = NET_TOP; l > NET_L0; --l) {
-      const int side = l - NET_L0 - 1;
-      cudaStream_t ss = N.side[side];
-      auto& L = N.lv[l];
-      launch_unlift(ss, L.y.p, L.feat.p, L.acc.p, false, nodes_of(gl[l]));
-      if (l < NET_TOP) {
-        HX_CUDA(cudaStreamWaitEvent(ss, N.ev_join[side + 1], 0));
-        launch_prolong(ss, N.lv[l + 1].acc.p, L.acc.p, gl[l], gl[l + 1], true);
-      }
-      HX_CUDA(cudaEventRecord(N.ev_join[side], ss));
-    }
-    auto& L1 = N.lv[NET_L0];
-    launch_lift(c->stream, L1.x.p, L1.feat.p, L1.x0.p, gl[NET_L0]);
-    stack_apply(c, c->stream, 0, gl[NET_L0], L1.x0.p, L1.y.p, N.tmp[0].p, N.tmp[1].p);
-    launch_unlift(c->stream, L1.y.p, L1.feat.p, L1.acc.p, false, nodes_of(gl[NET_L0]));
-    if (NET_TOP > NET_L0) {
-      HX_CUDA(cudaStreamWaitEvent(c->stream, N.ev_join[0], 0));
-      launch_prolong(c->stream, N.lv[NET_L0 + 1].acc.p, L1.acc.p, gl[NET_L0], gl[NET_L0 + 1],
-                     true);
-    }
+    HX_CUDA(cudaEventRecord(N.ev_join[side], ss));
+  }
+  auto& L1 = N.lv[NET_L0];
+  launch_lift(c->stream, L1.x.p, L1.feat.p, L1.x0.p, gl[NET_L0]);
+  stack(c->stream, NET_L0);
+  launch_unlift(c->stream, L1.y.p, L1.feat.p, L1.acc.p, false, nodes_of(gl[NET_L0]));
+  if (NET_TOP > NET_L0) {
+    HX_CUDA(cudaStreamWaitEvent(c->stream, N.ev_join[0], 0));
+    launch_prolong(c->stream, N.lv[NET_L0 + 1].acc.p, L1.acc.p, gl[NET_L0], gl[NET_L0 + 1],
+                   true);
   }
   // levels below the networks: acc_l = R^T acc_{l+1}
   for (int l = NET_L0 - 1; l >= 1; --l)
@@ -396,21 +382,21 @@ void net_forward_backward(hx_ctx* c, int nx, int ny, int nz, const float* x0, co
   const GridN g{nx, ny, nz};
   const int64_t nn = (int64_t)nx * ny * nz;
   auto& N = c->net;
-  DevBuf<__nv_bfloat16> bx0, by, act[7];
+  DevBuf<__nv_bfloat16> bx0, by, act[7], ge[8];
+  DevBuf<float> part;
   bx0.ensure(nn * 16);
   by.ensure(nn * 8);
   for (auto& a : act) a.ensure(nn * 16);
-  N.da.ensure(nn * 16);
-  N.db.ensure(nn * 16);
-  N.part.ensure(conv_num_tiles(g) * LP);
+  for (auto& a : ge) a.ensure(nn * 16);
+  part.ensure(2 * NET_LAYERS * conv_num_tiles(g) * LP);
   upload_act16(c, g, x0, bx0.p);
-  stack_forward_train(c, 0, g, bx0.p, act, by.p);
+  stack_forward_train(c, c->stream, 0, g, bx0.p, act, by.p);
   std::vector<__nv_bfloat16> hy((size_t)nn * 8);
   HX_CUDA(cudaMemcpyAsync(hy.data(), by.p, hy.size() * 2, cudaMemcpyDeviceToHost, c->stream));
-  upload_act16(c, g, dy, N.da.p);
+  upload_act16(c, g, dy, ge[0].p);
   HX_CUDA(cudaMemsetAsync(N.grad.p, 0, NET_PARAMS * sizeof(float), c->stream));
   HX_CUDA(cudaStreamSynchronize(c->stream));
-  stack_backward_train(c, 0, g, bx0.p, act, false);
+  stack_backward_train(c, c->stream, 0, g, bx0.p, act, ge, part.p, false);
   HX_CUDA(cudaMemcpyAsync(grads, N.grad.p, NET_PARAMS * sizeof(float), cudaMemcpyDeviceToHost,
                           c->stream));
   HX_CUDA(cudaStreamSynchronize(c->stream));
@@ -420,9 +406,11 @@ void net_forward_backward(hx_ctx* c, int nx, int ny, int nz, const float* x0, co
   check_conv_error(c);
 }
 
-// Loss of one residual (and error) of the current operator; with `grad`,
-// adds its parameter gradient to N.grad (`first`: overwrite instead).
-double net_loss_grad(hx_ctx* c, const double* r, const double* e, int loss_kind, bool first) {
+// Loss of one residual (and error) of the current operator into losses_dev[0]
+// (loss_kind 0) or the return value (loss_kind 1); adds its parameter gradient
+// to N.grad (`first`: overwrite instead).
+double net_loss_grad(hx_ctx* c, const double* r, const double* e, int loss_kind, bool first,
+                     double* losses_dev) {
   auto& N = c->net;
   const Grid& g = c->g;
   const int64_t n = g.dofs();
@@ -447,7 +435,7 @@ double net_loss_grad(hx_ctx* c, const double* r, const double* e, int loss_kind,
     launch_axpby(c->stream, zscr, z, e, n);  // d = z - e
     launch_matvec<double>(c->stream, 0, zscr, q, N.fac_last, c->d_nmask.p, g, c->K, 0.0, s3,
                           c->d_partials.p, nullptr);
-    launch_net_aloss(c->stream, zscr, q, e, r, n, c->d_partials.p, s2, N.scal.p);
+    launch_net_aloss(c->stream, zscr, q, e, r, n, c->d_partials.p, s2, losses_dev);
     gvec = q;  // 2 A d / e.r
   } else {
     // scaled residual loss |D^-1/2 (A z - r)|^2 / |D^-1/2 r|^2
@@ -467,23 +455,33 @@ double net_loss_grad(hx_ctx* c, const double* r, const double* e, int loss_kind,
   // output gradient is its lifting E_l
   launch_restrict_dof<double>(c->stream, gvec, c->d_minv.p, s3, s2, mode, scale_mul, N.lv[1].gx.p,
                       level_grid(g, 0), level_grid(g, 1));
-  for (int l = 2; l <= NET_TOP; ++l)
+  for (int l = 2; l <= NET_L0; ++l)
     launch_restrict(c->stream, 3, N.lv[l - 1].gx.p, N.lv[l].gx.p, level_grid(g, l - 1),
                     level_grid(g, l), false);
-  for (int l = NET_L0; l <= NET_TOP; ++l) {
+  // the networks side by side, as in the forward pass (precond_z)
+  auto backward = [&](cudaStream_t s, int l) {
+    auto& L = N.lv[l];
     const GridN gl = level_grid(g, l);
-    launch_lift(c->stream, N.lv[l].gx.p, N.lv[l].feat.p, N.da.p, gl);
-    stack_backward_train(c, l - NET_L0, gl, N.lv[l].x0.p, N.lv[l].act, !first);
+    launch_lift(s, L.gx.p, L.feat.p, L.ge[0].p, gl);
+    stack_backward_train(c, s, l - NET_L0, gl, L.x0.p, L.act, L.ge, L.part.p, !first);
+  };
+  HX_CUDA(cudaEventRecord(N.ev_fork, c->stream));
+  for (int l = NET_L0 + 1; l <= NET_TOP; ++l) {
+    const int side = l - NET_L0 - 1;
+    cudaStream_t ss = N.side[side];
+    HX_CUDA(cudaStreamWaitEvent(ss, side == 0 ? N.ev_fork : N.ev_x[side - 1], 0));
+    launch_restrict(ss, 3, N.lv[l - 1].gx.p, N.lv[l].gx.p, level_grid(g, l - 1), level_grid(g, l),
+                    false);
+    if (l < NET_TOP) HX_CUDA(cudaEventRecord(N.ev_x[side], ss));
+    backward(ss, l);
+    HX_CUDA(cudaEventRecord(N.ev_join[side], ss));
   }
-  double loss = 0;
-  if (host_ratio) {
-    const CgState a = get_state(c, 2), b = get_state(c, 3);
-    loss = b.rz > 0 ? a.rz / b.rz : 0.0;
-  } else {
-    HX_CUDA(cudaMemcpyAsync(&loss, N.scal.p, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    HX_CUDA(cudaStreamSynchronize(c->stream));
-  }
-  return loss;
+  backward(c->stream, NET_L0);
+  for (int l = NET_L0 + 1; l <= NET_TOP; ++l)
+    HX_CUDA(cudaStreamWaitEvent(c->stream, N.ev_join[l - NET_L0 - 1], 0));
+  if (!host_ratio) return 0.0;
+  const CgState a = get_state(c, 2), b = get_state(c, 3);
+  return b.rz > 0 ? a.rz / b.rz : 0.0;
 }
 
 // One Adam step on the summed gradient of `count` residual (and error)
@@ -497,12 +495,18 @@ double net_train_step(hx_ctx* c, const double* const* r, const double* const* e,
   net_buffers(c, true);
   ensure_workspace(c);
   double sum = 0.0;
+  double* losses = N.scal.ensure(std::max(8, count));
   for (int i = 0; i < count; ++i)
-    sum += net_loss_grad(c, r[i], e ? e[i] : nullptr, loss_kind, i == 0);
+    sum += net_loss_grad(c, r[i], e ? e[i] : nullptr, loss_kind, i == 0, losses + i);
   N.step += 1;
   launch_adam(c->stream, N.w.p, N.m.p, N.v.p, N.grad.p, N.live.p, NET_PARAMS, (float)lr, N.step);
   net_pack(c);
-  check_conv_error(c);
+  std::vector<double> h(count, 0.0);
+  if (loss_kind == 0)
+    HX_CUDA(cudaMemcpyAsync(h.data(), losses, count * sizeof(double), cudaMemcpyDeviceToHost,
+                            c->stream));
+  check_conv_error(c);  // synchronises
+  for (double v : h) sum += v;
   return sum / count;
 }
 
