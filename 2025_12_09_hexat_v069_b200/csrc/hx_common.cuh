@@ -266,7 +266,7 @@ __device__ __forceinline__ void cg_finish_iteration(CgState* st, const CgState& 
   const double rel = sqrt(rr) / s.bnorm;
   const bool tested = (iter % s.check_every) == 0;
   double best = s.best_rel, rel_res = tested ? rel : s.rel_res, peak = s.aux[2];
-  int status = HX_RUNNING, snap = s.snap;
+  int status = HX_RUNNING, snap = 0;
   // Order of tests as src/Solvers/GPUSolver.jl:478-511.
   if (s.div_ratio > 0.0 && iter > 50 && rel > s.div_ratio * best)
     status = HX_ST_DIVERGED;
@@ -275,7 +275,6 @@ __device__ __forceinline__ void cg_finish_iteration(CgState* st, const CgState& 
   else if (s.explode > 0.0 && rel > s.explode)
     status = HX_ST_DIVERGED;
   if (status == HX_RUNNING) {
-    snap = 0;
     if (rel < best) {
       best = rel;
       if (s.keep_best && rel < 1e-2) snap = 1;

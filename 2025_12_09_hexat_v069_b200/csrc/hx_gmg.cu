@@ -813,11 +813,10 @@ CgState solve_gmg(hx_ctx* c, const double* fac, const double* b, double* x, bool
   auto one = [&](double* pin, double* pout) {
     gmg_vcycle<double>(c, r, z, st);
     launch_fcg_coeffs<double>(c->stream, z, q, r, n, c->d_partials.p, st);
+    // (the best iterate goes to xbest: the reference's failure handling returns it)
     launch_fcg_step<double>(c->stream, pin, pout, z, x, q, fac, c->d_nmask.p, g, c->K, shift, st,
-                            c->d_partials.p);
+                            c->d_partials.p, xbest);
     launch_cg_update2<double>(c->stream, r, q, minv, n, st, c->d_partials.p);
-    // best-iterate snapshot (the reference's failure handling returns it)
-    if (xbest) launch_axpy_state<double>(c->stream, xbest, x, pout, n, st, pout == P0 ? 1 : 2);
   };
   auto body = [&]() {
     one(P1, P0);
@@ -830,6 +829,7 @@ CgState solve_gmg(hx_ctx* c, const double* fac, const double* b, double* x, bool
   CgState sf = loop.run(false, o.wall_limit_ms, t0, timed_out);
   if (sf.status != HX_ST_BREAKDOWN && sf.iter > 0) {
     double* pk = ((sf.iter - 1) % 2 == 0) ? P0 : P1;
+    if (xbest) launch_axpy_state<double>(c->stream, xbest, x, pk, n, st, 1);
     launch_axpy_state<double>(c->stream, x, x, pk, n, st, 0);
   }
   *iters_out = sf.iter;

@@ -60,18 +60,20 @@ void launch_matvec(cudaStream_t s, int mode, const T* x, T* y, const T* fac, con
                    double* out);
 // Fused PCG step (see hx_operator.cu): p_out = M^-1 r + beta p_in,
 // x += alpha_old p_in (owned nodes), q = mask(K p_out + s p_out),
-// st->alpha = rz / (p_out . q).
+// st->alpha = rz / (p_out . q).  xbest (FP64): also receives x where the last
+// iteration asked for a snapshot of it (st->snap).
 template <typename T>
 void launch_pcg_step(cudaStream_t s, const T* pin, T* pout, const T* r, const T* minv, T* x, T* q,
                      const T* fac, const uint8_t* nmask, const Grid& g, const ElemCoef<T>& K,
-                     T shift, CgState* st, double* partials);
+                     T shift, CgState* st, double* partials,
+                     T* xbest = nullptr);
 // Flexible-CG step: p_out = z + beta p_in, x += alpha_old p_in (owned
 // nodes), q = mask(K p_out + s p_out), st->alpha = (z . r) / (p_out . q)
 // with z . r in st->aux[3] (the preconditioner's output pass reduces it).
 template <typename T>
 void launch_fcg_step(cudaStream_t s, const T* pin, T* pout, const T* z, T* x, T* q, const T* fac,
                      const uint8_t* nmask, const Grid& g, const ElemCoef<T>& K, T shift,
-                     CgState* st, double* partials);
+                     CgState* st, double* partials, T* xbest = nullptr);
 // Multigrid smoothing (FP32): one Chebyshev step as a three-term recurrence,
 // xprev_new <- x + omega (x - xprev_new) + gamma M^-1 (b - (K + sI) x) on the
 // free DOFs (0 on the fixed ones; xprev_zero: x_prev = 0, not read); and the
@@ -109,7 +111,6 @@ void launch_dinv_bf16(cudaStream_t s, const T* r, const T* minv, __nv_bfloat16* 
 template <typename T>
 void launch_axpy_state(cudaStream_t s, T* dst, const T* x, const T* p, int64_t n,
                        const CgState* st, int when_snap);
-void launch_copy_if_snap(cudaStream_t s, double* dst, const double* src, int64_t n, CgState* st);
 // out = sum (b - q)^2 over the n entries, and sum b^2
 void launch_resid_norm(cudaStream_t s, const double* b, const double* q, int64_t n, CgState* st,
                        double* partials, double* out2);

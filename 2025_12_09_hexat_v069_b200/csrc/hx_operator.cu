@@ -240,6 +240,7 @@ struct OpArgs {
   T* x;           // FUSED: solution (x += alpha_old p_old on owned nodes); MODE 5:
                   // x_prev in, x_new out
   T* pout;        // FUSED: new direction p
+  T* xbest;       // FUSED, FP64: receives x too when the state asks for a snapshot (or null)
   T* q;           // output K p (masked, shifted)
   const T* fac;
   const uint8_t* nmask;
@@ -419,6 +420,9 @@ __global__ void __launch_bounds__(MV_BX* Tile<T, mode_fused(MODE)>::WARPS,
     alpha_old = (T)A.st->alpha;
     beta_old = (T)A.st->beta;
   }
+  // the iterate that the last iteration flagged as the best so far is complete
+  // only here (x + alpha p)
+  const bool snap = FUSED && sizeof(T) == 8 && A.xbest && A.st->snap;
   __syncthreads();
 
   // Node plane kp starts at value pv = kp * P3: a chunk's 16-byte aligned
@@ -543,6 +547,14 @@ __global__ void __launch_bounds__(MV_BX* Tile<T, mode_fused(MODE)>::WARPS,
             pd2[t] = pnew[t];
             xd[t] = xv[t];
           }
+      }
+      // (as a launch of its own the snapshot cost 1.3 us of 15 per iteration on
+      // 60 x 20 x 20 even where none was due)
+      if (snap) {
+        T* xs = plane_ptr(A.xbest, pv) + off;
+#pragma unroll
+        for (int t = 0; t < W; ++t)
+          if (d + t >= 0 && d + t < own_len) xs[t] = xv[t];
       }
     }
   };
@@ -1061,8 +1073,9 @@ template void launch_residual<float>(cudaStream_t, const float*, const float*, f
 template <typename T>
 void launch_pcg_step(cudaStream_t s, const T* pin, T* pout, const T* r, const T* minv, T* x, T* q,
                      const T* fac, const uint8_t* nmask, const Grid& g, const ElemCoef<T>& K,
-                     T shift, CgState* st, double* partials) {
+                     T shift, CgState* st, double* partials, T* xbest) {
   launch_struct<T, 3>(s, fac, nmask, g, K, shift, [&](auto& a) {
+    a.xbest = xbest;
     a.pin = pin;
     a.pout = pout;
     a.r = r;
@@ -1076,17 +1089,18 @@ void launch_pcg_step(cudaStream_t s, const T* pin, T* pout, const T* r, const T*
 template void launch_pcg_step<double>(cudaStream_t, const double*, double*, const double*,
                                       const double*, double*, double*, const double*,
                                       const uint8_t*, const Grid&, const ElemCoef<double>&,
-                                      double, CgState*, double*);
+                                      double, CgState*, double*, double*);
 template void launch_pcg_step<float>(cudaStream_t, const float*, float*, const float*,
                                      const float*, float*, float*, const float*, const uint8_t*,
                                      const Grid&, const ElemCoef<float>&, float, CgState*,
-                                     double*);
+                                     double*, float*);
 
 template <typename T>
 void launch_fcg_step(cudaStream_t s, const T* pin, T* pout, const T* z, T* x, T* q, const T* fac,
                      const uint8_t* nmask, const Grid& g, const ElemCoef<T>& K, T shift,
-                     CgState* st, double* partials) {
+                     CgState* st, double* partials, T* xbest) {
   launch_struct<T, 4>(s, fac, nmask, g, K, shift, [&](auto& a) {
+    a.xbest = xbest;
     a.pin = pin;
     a.pout = pout;
     a.minv = z;
@@ -1099,10 +1113,11 @@ void launch_fcg_step(cudaStream_t s, const T* pin, T* pout, const T* z, T* x, T*
 template void launch_fcg_step<double>(cudaStream_t, const double*, double*, const double*,
                                       double*, double*, const double*, const uint8_t*,
                                       const Grid&, const ElemCoef<double>&, double, CgState*,
-                                      double*);
+                                      double*, double*);
 template void launch_fcg_step<float>(cudaStream_t, const float*, float*, const float*, float*,
                                      float*, const float*, const uint8_t*, const Grid&,
-                                     const ElemCoef<float>&, float, CgState*, double*);
+                                     const ElemCoef<float>&, float, CgState*, double*,
+                                     float*);
 
 template <typename T>
 void launch_node_diag(cudaStream_t s, const T* fac, const uint8_t* bcfree, uint8_t* nmask, T* diag,

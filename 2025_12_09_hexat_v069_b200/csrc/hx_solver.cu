@@ -269,13 +269,11 @@ CgState pcg_fused(hx_ctx* c, int slot, const T* fac, const T* b, T* x, bool warm
   if (s0.status != HX_RUNNING || init.max_iter <= 0) return s0;
   auto body = [&]() {
     launch_pcg_step<T>(c->stream, P1, P0, r, minv, x, q, fac, c->d_nmask.p, g, K, shift, st,
-                       c->d_partials.p);
+                       c->d_partials.p, xbest);
     launch_cg_update2<T>(c->stream, r, q, minv, n, st, c->d_partials.p);
-    if (xbest) launch_axpy_state<T>(c->stream, xbest, x, P0, n, st, 1);
     launch_pcg_step<T>(c->stream, P0, P1, r, minv, x, q, fac, c->d_nmask.p, g, K, shift, st,
-                       c->d_partials.p);
+                       c->d_partials.p, xbest);
     launch_cg_update2<T>(c->stream, r, q, minv, n, st, c->d_partials.p);
-    if (xbest) launch_axpy_state<T>(c->stream, xbest, x, P1, n, st, 2);
   };
   GraphLoop loop(c, slot, std::max(1, check_every / 2), body);
   CgState sf = loop.run(true, wall_ms, t0, timed_out);
@@ -283,6 +281,7 @@ CgState pcg_fused(hx_ctx* c, int slot, const T* fac, const T* b, T* x, bool warm
   // whose alpha is invalid); p_k sits in P[(iter-1) % 2]
   if (sf.status != HX_ST_BREAKDOWN && sf.iter > 0) {
     T* pk = ((sf.iter - 1) % 2 == 0) ? P0 : P1;
+    if (xbest) launch_axpy_state<T>(c->stream, xbest, x, pk, n, st, 1);
     launch_axpy_state<T>(c->stream, x, x, pk, n, st, 0);
   }
   return sf;

@@ -154,28 +154,17 @@ __global__ void k_dinv_bf16(const T* __restrict__ r, const T* __restrict__ minv,
     ys[i] = __float2bfloat16_rn(dinv_sqrt((float)minv[i]) * (float)r[i]);
 }
 
-// dst = x + alpha p, with alpha from the state; `when_snap` restricts it to
-// iterations flagged as the best so far.
+// dst = x + alpha p, with alpha from the state; with when_snap only if the last
+// iteration was flagged as the best so far.
 template <typename T>
 __global__ void k_axpy_state(T* __restrict__ dst, const T* __restrict__ x,
                              const T* __restrict__ p, int64_t n, const CgState* st,
                              int when_snap) {
-  // when_snap 1 / 2: a best-iterate snapshot, taken only if the last
-  // iteration asked for one and its direction p_k is the buffer given (P0
-  // after iteration k = iter - 1 even, P1 after an odd one).  Launches of a
-  // batch that run after the loop stopped then rewrite the same snapshot
-  // instead of combining x with an older direction.
   pdl_wait();
   pdl_trigger();
-  if (when_snap && !(st->snap && ((st->iter - 1) & 1) == when_snap - 1)) return;
+  if (when_snap && !st->snap) return;
   const T a = (T)st->alpha;
   for (int64_t i = gtid(); i < n; i += gstride()) dst[i] = x[i] + a * p[i];
-}
-
-__global__ void k_copy_if_snap(double* __restrict__ dst, const double* __restrict__ src,
-                               int64_t n, const CgState* st) {
-  if (!st->snap) return;
-  for (int64_t i = gtid(); i < n; i += gstride()) dst[i] = src[i];
 }
 
 __global__ void k_resid_norm(const double* __restrict__ b, const double* __restrict__ q,
@@ -296,11 +285,6 @@ void launch_axpy_state(cudaStream_t s, T* dst, const T* x, const T* p, int64_t n
                                      const CgState*, int);
 HX_INST_CG(double)
 HX_INST_CG(float)
-
-void launch_copy_if_snap(cudaStream_t s, double* dst, const double* src, int64_t n, CgState* st) {
-  k_copy_if_snap<<<vec_blocks(n), VEC_THREADS, 0, s>>>(dst, src, n, st);
-  HX_CHECK_LAUNCH();
-}
 
 void launch_resid_norm(cudaStream_t s, const double* b, const double* q, int64_t n, CgState* st,
                        double* partials, double* out2) {
