@@ -155,8 +155,8 @@ __global__ void k_coarse_finish(float* __restrict__ x, const float* __restrict__
 // flexible-CG coefficients for a preconditioned residual z: beta =
 // -(z.q_old) / (p_old.q_old) (st->pq), st->aux[3] = z.r (the step length's
 // numerator, used by the flexible-CG step)
-template <typename T>
-__global__ void k_fcg_coeffs(const T* __restrict__ z, const T* __restrict__ q_old,
+template <typename TZ, typename T>
+__global__ void k_fcg_coeffs(const TZ* __restrict__ z, const T* __restrict__ q_old,
                              const T* __restrict__ r, int64_t n, double* partials, CgState* st) {
   pdl_wait();
   pdl_trigger();
@@ -755,15 +755,13 @@ void gmg_vcycle(hx_ctx* c, const T* r, T* z, const CgState* st) {
 template void gmg_vcycle<double>(hx_ctx*, const double*, double*, const CgState*);
 template void gmg_vcycle<float>(hx_ctx*, const float*, float*, const CgState*);
 
-template <typename T>
-void launch_fcg_coeffs(cudaStream_t s, const T* z, const T* q_old, const T* r, int64_t n,
+template <typename TZ, typename T>
+void launch_fcg_coeffs(cudaStream_t s, const TZ* z, const T* q_old, const T* r, int64_t n,
                        double* partials, CgState* st) {
-  launch_dep(small_vec(n), k_fcg_coeffs<T>, gblocks(n), 256, 0, s, z, q_old, r, n, partials, st);
+  launch_dep(small_vec(n), k_fcg_coeffs<TZ, T>, gblocks(n), 256, 0, s, z, q_old, r, n, partials, st);
   HX_CHECK_LAUNCH();
 }
-template void launch_fcg_coeffs<double>(cudaStream_t, const double*, const double*,
-                                        const double*, int64_t, double*, CgState*);
-template void launch_fcg_coeffs<float>(cudaStream_t, const float*, const float*, const float*,
+template void launch_fcg_coeffs<float, float>(cudaStream_t, const float*, const float*, const float*,
                                        int64_t, double*, CgState*);
 
 // ---------------------------------------------------------------------------
@@ -784,7 +782,10 @@ CgState solve_gmg(hx_ctx* c, const double* fac, const double* b, double* x, bool
   double* P0 = c->d_p.ensure(n);
   double* P1 = c->d_p2.ensure(n);
   double* q = c->d_q.ensure(n);
-  double* z = c->gmg.z.ensure(n);
+  // the cycle works on FP32 vectors of level 0 directly: its right-hand side
+  // is written with r, and its result read as it is by the coefficients and the step
+  float* r32 = c->gmg.lv[0].b.p;
+  float* z32 = c->gmg.lv[0].x.p;
   double* s64 = c->gmg.s.ensure(n);
   double* xbest = o.keep_best ? c->d_xbest.ensure(n) : nullptr;
   const double* minv = c->d_minv.p;
@@ -810,13 +811,15 @@ CgState solve_gmg(hx_ctx* c, const double* fac, const double* b, double* x, bool
   s0.alpha = 0.0;
   s0.beta = 0.0;
   put_state(c, 0, s0);
+  k_copy_cvt<float, double><<<gblocks(n), 256, 0, c->stream>>>(r32, r, n, nullptr);
+  HX_CHECK_LAUNCH();
   auto one = [&](double* pin, double* pout) {
-    gmg_vcycle<double>(c, r, z, st);
-    launch_fcg_coeffs<double>(c->stream, z, q, r, n, c->d_partials.p, st);
+    gmg_vcycle<float>(c, r32, z32, st);
+    launch_fcg_coeffs<float, double>(c->stream, z32, q, r, n, c->d_partials.p, st);
     // (the best iterate goes to xbest: the reference's failure handling returns it)
-    launch_fcg_step<double>(c->stream, pin, pout, z, x, q, fac, c->d_nmask.p, g, c->K, shift, st,
+    launch_fcg_step<double>(c->stream, pin, pout, z32, x, q, fac, c->d_nmask.p, g, c->K, shift, st,
                             c->d_partials.p, xbest);
-    launch_cg_update2<double>(c->stream, r, q, minv, n, st, c->d_partials.p);
+    launch_fcg_update(c->stream, r, q, c->d_nmask.p, n, st, c->d_partials.p, r32);
   };
   auto body = [&]() {
     one(P1, P0);

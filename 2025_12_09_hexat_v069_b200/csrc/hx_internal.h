@@ -70,8 +70,9 @@ void launch_pcg_step(cudaStream_t s, const T* pin, T* pout, const T* r, const T*
 // Flexible-CG step: p_out = z + beta p_in, x += alpha_old p_in (owned
 // nodes), q = mask(K p_out + s p_out), st->alpha = (z . r) / (p_out . q)
 // with z . r in st->aux[3] (the preconditioner's output pass reduces it).
-template <typename T>
-void launch_fcg_step(cudaStream_t s, const T* pin, T* pout, const T* z, T* x, T* q, const T* fac,
+// z: in T, or in FP32 for an FP64 step.
+template <typename T, typename TZ>
+void launch_fcg_step(cudaStream_t s, const T* pin, T* pout, const TZ* z, T* x, T* q, const T* fac,
                      const uint8_t* nmask, const Grid& g, const ElemCoef<T>& K, T shift,
                      CgState* st, double* partials, T* xbest = nullptr);
 // Multigrid smoothing (FP32): one Chebyshev step as a three-term recurrence,
@@ -106,6 +107,11 @@ void launch_cg_init(cudaStream_t s, const T* b, const T* q, const T* minv, T* r,
 template <typename T>
 void launch_cg_update2(cudaStream_t s, T* r, const T* q, const T* minv, int64_t n, CgState* st,
                        double* partials, __nv_bfloat16* ys = nullptr);
+// the same for the flexible CG of the multigrid solve: no M^-1 (r.z comes with
+// the next preconditioned residual), the free DOFs from nmask, and r32 = the
+// new residual in FP32, the next cycle's right-hand side
+void launch_fcg_update(cudaStream_t s, double* r, const double* q, const uint8_t* nmask, int64_t n,
+                       CgState* st, double* partials, float* r32);
 template <typename T>
 void launch_dinv_bf16(cudaStream_t s, const T* r, const T* minv, __nv_bfloat16* ys, int64_t n);
 template <typename T>
@@ -248,7 +254,7 @@ struct hx_ctx {
     GmgLevel lv[HX_GMG_MAX_LEVELS];
     hx::DevBuf<hx::CgState> coarse_st;
     hx::DevBuf<float> p0, p1;   // coarse PCG directions
-    hx::DevBuf<double> z, s;    // FCG: preconditioned residual, scratch
+    hx::DevBuf<double> s;       // FCG: scratch
     // direct coarsest-level solve: dense inverse (FP32, n x n) of the masked
     // coarsest operator, formed in FP64 at set-up
     bool direct = false;

@@ -71,6 +71,10 @@ __device__ __forceinline__ void cp_async16(unsigned sdst, const void* gsrc, unsi
 __device__ __forceinline__ void cp_async16(unsigned sdst, const void* gsrc) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sdst), "l"(gsrc));
 }
+__device__ __forceinline__ void cp_async8(unsigned sdst, const void* gsrc, unsigned bytes = 8) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sdst), "l"(gsrc),
+               "r"(bytes));
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
@@ -98,7 +102,7 @@ template <typename T>
 using VecOf = typename Tile<T, false>::V;
 template <typename T, bool FUSED>
 constexpr int mv_by() { return Tile<T, FUSED>::WARPS * Tile<T, FUSED>::R; }  // element rows of a CTA
-constexpr bool mode_fused(int mode) { return mode == 3 || mode == 4; }
+constexpr bool mode_fused(int mode) { return mode == 3 || mode == 4 || mode == 7; }
 
 __device__ __forceinline__ double vadd(double a, double b) { return a + b; }
 __device__ __forceinline__ double vmul(double a, double b) { return a * b; }
@@ -237,6 +241,7 @@ struct OpArgs {
   const T* pin;   // vector to multiply (MODE 0, 1, 5, 6) or p_old (FUSED)
   const T* r;     // MODE 3: residual; MODE 5, 6: right-hand side b
   const T* minv;  // MODE 3, 5: Jacobi inverse diagonal; MODE 4: preconditioned z
+  const float* z32;  // MODE 7: preconditioned z
   T* x;           // FUSED: solution (x += alpha_old p_old on owned nodes); MODE 5:
                   // x_prev in, x_new out
   T* pout;        // FUSED: new direction p
@@ -343,7 +348,11 @@ __device__ __forceinline__ void lambda_pair(const CoefV<V, true>& K, V (&s)[3], 
 //         with A x = mask(K x + s x); x_prev (A.x) is overwritten by x_new
 //         (each node's x_prev is read and written by its owner only; the
 //         staged x, read by the neighbours, is not written);
-// MODE 6: residual r = mask(b - K x - s x) into A.q.
+// MODE 6: residual r = mask(b - K x - s x) into A.q;
+// MODE 7: MODE 4 of an FP64 solve with z in FP32, as the multigrid cycle leaves
+//         it (two z's fill the first half of a 16-byte slot of their plane).
+//         With an FP64 copy of z, the copy took 48 us at 320 x 160 x 160, the
+//         coefficients 93 (now 81) and this step 307 (now 296).
 template <typename T, int MODE, bool CUBE>
 __global__ void __launch_bounds__(MV_BX* Tile<T, mode_fused(MODE)>::WARPS,
                                   Tile<T, mode_fused(MODE)>::RESIDENT)
@@ -353,6 +362,8 @@ __global__ void __launch_bounds__(MV_BX* Tile<T, mode_fused(MODE)>::WARPS,
   using V = VecOf<T>;
   constexpr bool FUSED = S::FUSED;
   constexpr bool DOT = MODE == 1 || FUSED;  // reduces x.q / p.q
+  constexpr bool FCG = MODE == 4 || MODE == 7;
+  static_assert(MODE != 7 || sizeof(T) == 8, "an FP64 step");
   constexpr int R = Tile<T, FUSED>::R, WARPS = S::WARPS, BY = WARPS * R;
   constexpr int NT = MV_BX * WARPS;
   constexpr int W = G::W, CPR = G::CPR, RS = G::RS, PLANE = G::PLANE;
@@ -440,6 +451,12 @@ __global__ void __launch_bounds__(MV_BX* Tile<T, mode_fused(MODE)>::WARPS,
         (at >= 0 && left > 0) ? (unsigned)((left < W ? left : (int64_t)W) * sizeof(T)) : 0u;
     cp_async16(smem_u32(sdst + sbase(q)), v + (bytes ? at : 0), bytes);
   };
+  auto cut_z32 = [&](T* sdst, int q, int64_t pv) {
+    const int64_t at = (pv & ~(int64_t)(W - 1)) + chunk_off(q, pv), left = P3 * (int64_t)nzn - at;
+    const unsigned bytes =
+        (at >= 0 && left > 0) ? (unsigned)((left < W ? left : (int64_t)W) * sizeof(float)) : 0u;
+    cp_async8(smem_u32(sdst + sbase(q)), A.z32 + (bytes ? at : 0), bytes);
+  };
   auto issue = [&](int kp, T* p) {
     if ((unsigned)kp > (unsigned)kp_last) return;
     const int64_t pv = (int64_t)kp * P3;
@@ -450,7 +467,10 @@ __global__ void __launch_bounds__(MV_BX* Tile<T, mode_fused(MODE)>::WARPS,
         if (!use[q]) continue;
         cut(A.pin, p, q, pv);
         if (FUSED) {
-          cut(A.minv, p + PLANE, q, pv);
+          if (MODE == 7)
+            cut_z32(p + PLANE, q, pv);
+          else
+            cut(A.minv, p + PLANE, q, pv);
           if (own[q] && kown) cut(A.x, p + 2 * PLANE, q, pv);
           if (MODE == 3) cut(A.r, p + 3 * PLANE, q, pv);
         }
@@ -458,7 +478,8 @@ __global__ void __launch_bounds__(MV_BX* Tile<T, mode_fused(MODE)>::WARPS,
       return;
     }
     const T* bp = plane_ptr(A.pin, pv);
-    const T* bm = FUSED ? plane_ptr(A.minv, pv) : nullptr;
+    const T* bm = FUSED && MODE != 7 ? plane_ptr(A.minv, pv) : nullptr;
+    const float* bz = MODE == 7 ? plane_ptr(A.z32, pv) : nullptr;
     const T* bx = FUSED ? plane_ptr((const T*)A.x, pv) : nullptr;
     const T* br = MODE == 3 ? plane_ptr(A.r, pv) : nullptr;
     const unsigned d0 = smem_u32(p);
@@ -468,7 +489,10 @@ __global__ void __launch_bounds__(MV_BX* Tile<T, mode_fused(MODE)>::WARPS,
       const unsigned d = d0 + sbase(q) * (int)sizeof(T);
       if (use[q]) {
         cp_async16(d, bp + off);
-        if (FUSED) cp_async16(d + PLANE * sizeof(T), bm + off);
+        if (MODE == 7)
+          cp_async8(d + PLANE * sizeof(T), bz + off);
+        else if (FUSED)
+          cp_async16(d + PLANE * sizeof(T), bm + off);
         if (MODE == 3) cp_async16(d + 3 * PLANE * sizeof(T), br + off);
       }
       if (FUSED && own[q] && kown) cp_async16(d + 2 * PLANE * sizeof(T), bx + off);
@@ -516,7 +540,13 @@ __global__ void __launch_bounds__(MV_BX* Tile<T, mode_fused(MODE)>::WARPS,
       if (!use[q]) continue;
       const T* a = src + sbase(q);
       const VecT po = *reinterpret_cast<const VecT*>(a);
-      const VecT mv = *reinterpret_cast<const VecT*>(a + PLANE);
+      VecT mv;
+      if constexpr (MODE == 7) {
+        const float2 zf = *reinterpret_cast<const float2*>(a + PLANE);
+        mv = VecT{zf.x, zf.y};
+      } else {
+        mv = *reinterpret_cast<const VecT*>(a + PLANE);
+      }
       const T* pa = reinterpret_cast<const T*>(&po);
       const T* ma = reinterpret_cast<const T*>(&mv);
       VecT rv{};
@@ -524,7 +554,7 @@ __global__ void __launch_bounds__(MV_BX* Tile<T, mode_fused(MODE)>::WARPS,
       const T* ra = reinterpret_cast<const T*>(&rv);
       T pnew[W];
 #pragma unroll
-      for (int t = 0; t < W; ++t) pnew[t] = (MODE == 4 ? ma[t] : ma[t] * ra[t]) + beta_old * pa[t];
+      for (int t = 0; t < W; ++t) pnew[t] = (FCG ? ma[t] : ma[t] * ra[t]) + beta_old * pa[t];
       *reinterpret_cast<VecT*>(pd + sbase(q)) = *reinterpret_cast<const VecT*>(pnew);
       if (!kown || !own[q]) continue;
       const VecT xw = *reinterpret_cast<const VecT*>(a + 2 * PLANE);
@@ -876,9 +906,9 @@ __global__ void __launch_bounds__(MV_BX* Tile<T, mode_fused(MODE)>::WARPS,
       if (MODE == 1) {
         A.out[0] = v[0];
       } else {
-        const double pq = v[0], num = MODE == 4 ? A.st->aux[3] : A.st->rz;
+        const double pq = v[0], num = FCG ? A.st->aux[3] : A.st->rz;
         A.st->pq = pq;
-        if (!(pq > 0.0) || !isfinite(pq) || (MODE == 4 && !isfinite(num)))
+        if (!(pq > 0.0) || !isfinite(pq) || (FCG && !isfinite(num)))
           A.st->status = HX_ST_BREAKDOWN;
         else
           A.st->alpha = num / pq;
@@ -1095,15 +1125,19 @@ template void launch_pcg_step<float>(cudaStream_t, const float*, float*, const f
                                      const Grid&, const ElemCoef<float>&, float, CgState*,
                                      double*, float*);
 
-template <typename T>
-void launch_fcg_step(cudaStream_t s, const T* pin, T* pout, const T* z, T* x, T* q, const T* fac,
+template <typename T, typename TZ>
+void launch_fcg_step(cudaStream_t s, const T* pin, T* pout, const TZ* z, T* x, T* q, const T* fac,
                      const uint8_t* nmask, const Grid& g, const ElemCoef<T>& K, T shift,
                      CgState* st, double* partials, T* xbest) {
-  launch_struct<T, 4>(s, fac, nmask, g, K, shift, [&](auto& a) {
+  constexpr bool SAME = std::is_same<T, TZ>::value;
+  launch_struct<T, SAME ? 4 : 7>(s, fac, nmask, g, K, shift, [&](auto& a) {
     a.xbest = xbest;
     a.pin = pin;
     a.pout = pout;
-    a.minv = z;
+    if constexpr (SAME)
+      a.minv = z;
+    else
+      a.z32 = z;
     a.x = x;
     a.q = q;
     a.st = st;
@@ -1114,6 +1148,10 @@ template void launch_fcg_step<double>(cudaStream_t, const double*, double*, cons
                                       double*, double*, const double*, const uint8_t*,
                                       const Grid&, const ElemCoef<double>&, double, CgState*,
                                       double*, double*);
+template void launch_fcg_step<double, float>(cudaStream_t, const double*, double*, const float*,
+                                             double*, double*, const double*, const uint8_t*,
+                                             const Grid&, const ElemCoef<double>&, double,
+                                             CgState*, double*, double*);
 template void launch_fcg_step<float>(cudaStream_t, const float*, float*, const float*, float*,
                                      float*, const float*, const uint8_t*, const Grid&,
                                      const ElemCoef<float>&, float, CgState*, double*,

@@ -106,8 +106,8 @@ void gmg_setup(hx_ctx* c, const double* fac, double shift);
 // levels do nothing once that has stopped), or null
 template <typename T>
 void gmg_vcycle(hx_ctx* c, const T* r, T* z, const CgState* st = nullptr);
-template <typename T>
-void launch_fcg_coeffs(cudaStream_t s, const T* z, const T* q_old, const T* r, int64_t n,
+template <typename TZ, typename T>
+void launch_fcg_coeffs(cudaStream_t s, const TZ* z, const T* q_old, const T* r, int64_t n,
                        double* partials, CgState* st);
 CgState solve_gmg(hx_ctx* c, const double* fac, const double* b, double* x, bool warm,
                   double shift, const hx_solve_opts& o, double t0, bool* timed_out,

@@ -145,6 +145,59 @@ __global__ void k_cg_update2(T* __restrict__ r, const T* __restrict__ q,
     cg_finish_iteration(st, s0, v[0], v[1]);
 }
 
+// k_cg_update2 of the multigrid solve (see launch_fcg_update).  Bound by its 28
+// bytes per DOF: reading M^-1 for the mask, and a copy of r to FP32 as a
+// launch of its own, made it 44 (320 x 160 x 160: 119 us instead of 126 + 39).
+__global__ void k_fcg_update(double* __restrict__ r, const double* __restrict__ q,
+                             const uint8_t* __restrict__ nmask, int64_t n, CgState* st,
+                             double* partials, float* __restrict__ r32) {
+  pdl_wait();
+  pdl_trigger();
+  if (st->status != HX_RUNNING) return;
+  const double alpha = st->alpha;
+  __shared__ CgState s0;  // read after grid_reduce's barriers
+  load_state(&s0, st);
+  double rr = 0;
+  auto upd = [&](unsigned free, double ri, double qi) {
+    const double v = free ? ri - alpha * qi : 0.0;
+    rr += v * v;
+    return v;
+  };
+  const int64_t nv = n / 2;
+  double2* rV = reinterpret_cast<double2*>(r);
+  const double2* qV = reinterpret_cast<const double2*>(q);
+  float2* sV = reinterpret_cast<float2*>(r32);
+  // entry 2 i is component c of `node`; both advance with i (no division)
+  int64_t node = 2 * gtid() / 3;
+  int c = (int)(2 * gtid() - 3 * node);
+  const int64_t dn = 2 * gstride() / 3;
+  const int dc = (int)(2 * gstride() - 3 * dn);
+#pragma unroll 2
+  for (int64_t i = gtid(); i < nv; i += gstride()) {
+    double2 a = rV[i];
+    const double2 b = qV[i];
+    const unsigned m0 = nmask[node], m1 = nmask[node + (c == 2)];
+    a.x = upd((m0 >> c) & 1u, a.x, b.x);
+    a.y = upd((m1 >> (c == 2 ? 0 : c + 1)) & 1u, a.y, b.y);
+    rV[i] = a;
+    sV[i] = make_float2((float)a.x, (float)a.y);
+    node += dn;
+    c += dc;
+    if (c >= 3) {
+      c -= 3;
+      ++node;
+    }
+  }
+  for (int64_t i = 2 * nv + gtid(); i < n; i += gstride()) {
+    r[i] = upd(((unsigned)nmask[i / 3] >> (int)(i % 3)) & 1u, r[i], q[i]);
+    r32[i] = (float)r[i];
+  }
+  // (r.z = r.r: the flexible step sets its own coefficients before they are used)
+  double v[1] = {rr};
+  if (grid_reduce<1>(v, partials, &st->ticket[TK_UPDATE]) && threadIdx.x == 0)
+    cg_finish_iteration(st, s0, v[0], v[0]);
+}
+
 // ys = BF16(D^-1/2 r), as k_cg_update2 writes it (for a residual that
 // another kernel produced).
 template <typename T>
@@ -257,6 +310,13 @@ void launch_cg_update2(cudaStream_t s, T* r, const T* q, const T* minv, int64_t 
                        double* partials, __nv_bfloat16* ys) {
   launch_dep(small_vec(n), k_cg_update2<T>, vec_blocks(n), VEC_THREADS, 0, s, r, q, minv, n, st,
              partials, ys);
+  HX_CHECK_LAUNCH();
+}
+
+void launch_fcg_update(cudaStream_t s, double* r, const double* q, const uint8_t* nmask, int64_t n,
+                       CgState* st, double* partials, float* r32) {
+  launch_dep(small_vec(n), k_fcg_update, vec_blocks(n), VEC_THREADS, 0, s, r, q, nmask, n, st,
+             partials, r32);
   HX_CHECK_LAUNCH();
 }
 
