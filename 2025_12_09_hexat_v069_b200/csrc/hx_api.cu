@@ -247,6 +247,37 @@ void up_nodes3(hx_ctx* c, int32_t dt, const void* h, double* d) {
 void down_nodes3(hx_ctx* c, int32_t dt, const double* d, void* h) {
   download(c, dt, d, c->node_map, c->n_user_nodes, c->g.nodes(), 3, h);
 }
+// Nodal host arrays in grid numbering copied on c->copy, after what c->stream
+// holds (it may still read the buffers), and used by c->stream from join() on.
+// The caller's memory is not in use any more once the object is gone.
+struct LateNodes {
+  hx_ctx* c;
+  bool started = false;
+  void start() {
+    if (!c->copy) HX_CUDA(cudaStreamCreateWithFlags(&c->copy, cudaStreamNonBlocking));
+    if (!c->ev_copy) HX_CUDA(cudaEventCreateWithFlags(&c->ev_copy, cudaEventDisableTiming));
+    HX_CUDA(cudaEventRecord(c->ev_copy, c->stream));
+    HX_CUDA(cudaStreamWaitEvent(c->copy, c->ev_copy, 0));
+    started = true;
+  }
+  // to dev (Float64) or to the staging buffer (Float32)
+  void copy(int32_t dt, const void* host, double* dev, hx::DevBuf<char>& stage) {
+    const size_t cnt = (size_t)c->g.nodes() * 3, w = dt == HX_F64 ? sizeof(double) : sizeof(float);
+    void* dst = dt == HX_F64 ? (void*)dev : (void*)stage.ensure(cnt * w);
+    HX_CUDA(cudaMemcpyAsync(dst, host, cnt * w, cudaMemcpyHostToDevice, c->copy));
+  }
+  void join() {
+    HX_CUDA(cudaEventRecord(c->ev_copy, c->copy));
+    HX_CUDA(cudaStreamWaitEvent(c->stream, c->ev_copy, 0));
+  }
+  void convert(int32_t dt, double* dev, hx::DevBuf<char>& stage) {
+    if (dt != HX_F64)
+      hx::launch_convert<double, float>(c->stream, dev, (const float*)stage.p, 3 * c->g.nodes());
+  }
+  ~LateNodes() {
+    if (started) cudaStreamSynchronize(c->copy);
+  }
+};
 void up_elems(hx_ctx* c, int32_t dt, const void* h, double* d, int w = 1) {
   upload(c, dt, h, c->elem_map, c->n_user_elem, c->g.elems(), w, d);
 }
@@ -361,6 +392,8 @@ HX_API void hx_destroy(hx_ctx* c) {
     if (st) cudaStreamDestroy(st);
   for (auto& e : {c->gmg.ev_fork, c->gmg.ev_join[0], c->gmg.ev_join[1]})
     if (e) cudaEventDestroy(e);
+  if (c->copy) cudaStreamDestroy(c->copy);
+  if (c->ev_copy) cudaEventDestroy(c->ev_copy);
   if (c->ev_in) cudaEventDestroy(c->ev_in);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
@@ -498,12 +531,28 @@ HX_API hx_status hx_solve(hx_ctx* c, int32_t dt, const void* f, const void* fact
     double* df = c->d_f.ensure(n);
     double* dfac = c->d_fac.ensure(c->g.elems());
     double* du = c->d_x.ensure(n);
-    up_nodes3(c, dt, f, df);
+    // A multigrid set-up needs only the factors: f and u follow on a stream of
+    // their own meanwhile (320 x 160 x 160, Float32: 1.9 ms of copies beside
+    // 4.7 ms of set-up)
+    const bool beside = o.preconditioner == HX_PC_MULTIGRID && identity(c);
+    LateNodes in{c};
+    if (!beside) up_nodes3(c, dt, f, df);
     if (!identity(c)) HX_CUDA(cudaMemsetAsync(dfac, 0, c->g.elems() * sizeof(double), c->stream));
     up_elems(c, dt, factor, dfac);
-    if (o.warm_start) up_nodes3(c, dt, u, du);
+    if (beside) {
+      in.start();
+      in.copy(dt, f, df, c->d_stage_f);
+      if (o.warm_start) in.copy(dt, u, du, c->d_stage_u);
+    } else if (o.warm_start) {
+      up_nodes3(c, dt, u, du);
+    }
+    const std::function<void()> late = [&] {
+      in.join();
+      in.convert(dt, df, c->d_stage_f);
+      if (o.warm_start) in.convert(dt, du, c->d_stage_u);
+    };
     hx_solve_report R{};
-    hx_status s = hx::solve_grid(c, df, dfac, du, o, &R);
+    hx_status s = hx::solve_grid(c, df, dfac, du, o, &R, beside ? &late : nullptr);
     down_nodes3(c, dt, du, u);
     R.time_device_ms = ev.stop();
     R.time_total_ms = now_ms() - t0;

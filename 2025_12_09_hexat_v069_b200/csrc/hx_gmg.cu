@@ -777,7 +777,7 @@ CgState solve_gmg(hx_ctx* c, const double* fac, const double* b, double* x, bool
   const Grid& g = c->g;
   const int64_t n = g.dofs();
   c->gmg.degree = o.mg_smooth_degree > 0 ? o.mg_smooth_degree : GMG_DEFAULT_DEGREE;
-  gmg_setup(c, fac, shift);
+  gmg_prepare(c, fac, shift);
   double* r = c->d_r.ensure(n);
   double* P0 = c->d_p.ensure(n);
   double* P1 = c->d_p2.ensure(n);

@@ -226,6 +226,11 @@ struct hx_ctx {
 
   // host<->device staging for F32 callers
   hx::DevBuf<char> d_stage;
+  // a host call's right-hand side and initial guess on their way beside the
+  // multigrid set-up (see hx_solve)
+  hx::DevBuf<char> d_stage_f, d_stage_u;
+  cudaStream_t copy = nullptr;
+  cudaEvent_t ev_copy = nullptr;
 
   // grid of the last filter (for timing) and its work vectors
   hx::Grid fg{};
@@ -252,6 +257,7 @@ struct hx_ctx {
     bool ready = false;
     int nl = 0;
     GmgLevel lv[HX_GMG_MAX_LEVELS];
+    bool prepared = false;      // the hierarchy is that of solve_grid's current attempt
     hx::DevBuf<hx::CgState> coarse_st;
     hx::DevBuf<float> p0, p1;   // coarse PCG directions
     hx::DevBuf<double> s;       // FCG: scratch

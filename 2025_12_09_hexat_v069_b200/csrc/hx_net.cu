@@ -712,7 +712,7 @@ static CgState learned_fcg_mixed(hx_ctx* c, const double* fac, const double* b, 
   const int64_t n = g.dofs(), ne = g.elems();
   if (multigrid) {
     c->gmg.degree = o.mg_smooth_degree > 0 ? o.mg_smooth_degree : GMG_DEFAULT_DEGREE;
-    gmg_setup(c, fac, shift);
+    gmg_prepare(c, fac, shift);
   } else {
     net_operator_inputs(c, fac);
   }

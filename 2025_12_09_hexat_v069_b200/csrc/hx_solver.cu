@@ -470,7 +470,8 @@ static hx_status map_status(int st) {
 // Device-level solve in grid numbering.  f, fac, u are FP64 device arrays.
 // ---------------------------------------------------------------------------
 hx_status solve_grid(hx_ctx* c, const double* f, const double* fac, double* u,
-                     const hx_solve_opts& o, hx_solve_report* rep) {
+                     const hx_solve_opts& o, hx_solve_report* rep,
+                     const std::function<void()>* late) {
   const double t0 = now_ms();
   HX_REQUIRE(c->has_mesh, "no mesh: call hx_set_grid or hx_set_mesh first");
   HX_REQUIRE(o.tol > 0, "tol must be > 0");
@@ -503,9 +504,18 @@ hx_status solve_grid(hx_ctx* c, const double* f, const double* fac, double* u,
   bool use_mg = o.preconditioner == HX_PC_MULTIGRID;
   bool can_switch = o.ref_retry && o.multigrid_fallback && o.preconditioner == HX_PC_JACOBI;
   for (int attempt = 1; attempt <= attempts; ++attempt) {
-    const double ts = now_ms();
+    double ts = now_ms();
+    c->gmg.prepared = false;
     if (attempt == 1) {
       maxd = jacobi_setup_public(c, fac, factor, &shift);
+      if (late) {
+        if (use_mg) {
+          const double tg = now_ms();
+          gmg_prepare(c, fac, shift);
+          ts += now_ms() - tg;  // reported as the preconditioner's
+        }
+        (*late)();
+      }
       launch_mask_rhs<double>(c->stream, f, c->d_minv.p, b, n);
     } else {
       shift = factor * maxd;

@@ -76,8 +76,11 @@ int pcg_snapshots(hx_ctx* c, const double* f, const double* fac, int every, int 
                   double tol, double* snaps);
 void ensure_workspace(hx_ctx* c);
 void upload_bc(hx_ctx* c);
+// late (or null): called before f, and u of a warm start, are first read; a
+// multigrid set-up of the first attempt, which needs neither, runs before it
 hx_status solve_grid(hx_ctx* c, const double* f, const double* fac, double* u,
-                     const hx_solve_opts& o, hx_solve_report* rep);
+                     const hx_solve_opts& o, hx_solve_report* rep,
+                     const std::function<void()>* late = nullptr);
 // Filter on the grid g with element size h (FP64 device arrays, grid numbering).
 hx_status filter_grid(hx_ctx* c, const Grid& g, const double h[3], const double* rho, double* out,
                       double radius, int ref_compat, double tol, int max_iter,
@@ -102,6 +105,11 @@ hx_status export_webdata(hx_ctx* c, const char* path, const T* dens, const T* l1
 // default Chebyshev degree of the multigrid smoothing
 constexpr int GMG_DEFAULT_DEGREE = 2;
 void gmg_setup(hx_ctx* c, const double* fac, double shift);
+// gmg_setup unless this attempt of the solve has done it
+inline void gmg_prepare(hx_ctx* c, const double* fac, double shift) {
+  if (!c->gmg.prepared) gmg_setup(c, fac, shift);
+  c->gmg.prepared = true;
+}
 // st: the flexible-CG state that the cycle belongs to (its kernels on large
 // levels do nothing once that has stopped), or null
 template <typename T>
