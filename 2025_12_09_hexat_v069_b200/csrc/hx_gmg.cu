@@ -825,9 +825,9 @@ CgState solve_gmg(hx_ctx* c, const double* fac, const double* b, double* x, bool
     one(P1, P0);
     one(P0, P1);
   };
-  // a multigrid solve takes tens of iterations and the V-cycle's kernels run
-  // whole even after the state has stopped: two iterations per graph launch
-  // waste at most one cycle
+  // a multigrid solve takes tens of iterations, and the small levels' kernels
+  // run whole even after the state has stopped: two iterations per graph
+  // launch waste at most one such cycle
   GraphLoop loop(c, 0, 1, body);
   CgState sf = loop.run(false, o.wall_limit_ms, t0, timed_out);
   if (sf.status != HX_ST_BREAKDOWN && sf.iter > 0) {

@@ -528,7 +528,8 @@ enum {
   HX_KERNEL_PCG_UPDATE_FP64 = 1, /* r update + r.z, r.r reductions */
   HX_KERNEL_APPLY_FP64 = 2,      /* plain K.x */
   HX_KERNEL_PCG_STEP_FP32 = 3,
-  HX_KERNEL_FILTER_MATVEC = 4,
+  HX_KERNEL_FILTER_MATVEC = 4,   /* CG step of the last filter: direction, x update,
+                                    operator product, p.q */
   HX_KERNEL_CONV3 = 5,           /* one 16 -> 16 BF16 conv3d layer on the node grid */
   HX_KERNEL_NET_APPLY = 6,       /* one learned-preconditioner application */
   HX_KERNEL_FCG_STEP_FP32 = 7    /* flexible-CG step of the mixed learned solve:
