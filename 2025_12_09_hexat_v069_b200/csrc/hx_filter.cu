@@ -18,7 +18,7 @@
 // types), so no vector holds it.  The update (k_filter_update) is the rest.  At
 // a million nodes the vectors fit the L2 and latency bounds both kernels: an
 // iteration at 161 x 81 x 81 nodes took 56 us (plain product from 27 global
-// loads per node, then two passes over five vectors) and takes 33 us.
+// loads per node, then two passes over five vectors) and takes 32 us.
 #include "hx_internal.h"
 
 namespace hx {
@@ -59,14 +59,19 @@ __device__ __forceinline__ int row_type(int i, int n) {
 
 constexpr int FB_X = 32, FB_Y = 8, FB_NT = FB_X * FB_Y;
 constexpr int FS_X = FB_X + 2, FS_Y = FB_Y + 2;  // staged tile with its halo
-constexpr int FB_RESIDENT = 3;
+constexpr int FS_R = 2, FS_NT = FB_NT / FS_R;    // node rows and threads of the step
+constexpr int FB_RESIDENT = 4;
 
 // One CTA owns a 32 x 8 node column over planes [k0, k1) and marches along z:
 // plane kp's new direction p = D^-1 r + beta p_in goes to shared memory (tile
 // and halo; the owner also stores it and x + alpha p_in), its sums a, b to
 // registers, and q of plane kp - 1 follows from three planes' sums.  r, p_in and
-// x are loaded two planes ahead.
-__global__ void __launch_bounds__(FB_NT, FB_RESIDENT)
+// x are loaded two planes ahead.  A thread has two adjacent rows: they share
+// two of their four staged rows' x sums, and the index and bounds arithmetic,
+// most of the instructions of a plane (a filter of 30 iterations at 161 x 81 x 81
+// nodes 0.985 -> 0.947 ms; one row per thread issued 214 instructions per plane and
+// warp, 65% of the issue slots).
+__global__ void __launch_bounds__(FS_NT, FB_RESIDENT)
     k_filter_step(const double* __restrict__ pin, double* __restrict__ pout,
                   const double* __restrict__ r, double* __restrict__ x, double* __restrict__ q,
                   Grid g, const __grid_constant__ FilterCoef F, int kchunk, CgState* st,
@@ -77,17 +82,26 @@ __global__ void __launch_bounds__(FB_NT, FB_RESIDENT)
   const bool first = st->iter == 0;  // x = p_in = 0
   const double alpha = first ? 0.0 : st->alpha, beta = first ? 0.0 : st->beta;
   __shared__ double tile[2][FS_Y][FS_X];
-  const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + FB_X * ty;
+  const int tx = threadIdx.x, ty = FS_R * threadIdx.y, tid = tx + FB_X * threadIdx.y;
   const int i = blockIdx.x * FB_X + tx, j = blockIdx.y * FB_Y + ty;
   const int k0 = blockIdx.z * kchunk, k1 = min(k0 + kchunk, g.nzn);
-  const bool act = i < g.nxn && j < g.nyn;
+  const bool act[FS_R] = {i < g.nxn && j < g.nyn, i < g.nxn && j + 1 < g.nyn};
   const int64_t pl = (int64_t)g.nxn * g.nyn;
-  const int rx = row_type(min(i, g.nxn - 1), g.nxn), ry = row_type(min(j, g.nyn - 1), g.nyn);
+  const int rx = row_type(min(i, g.nxn - 1), g.nxn);
   // Nodes outside the grid are staged as 0, so that only the diagonal entries
   // depend on the row; the off-diagonal ones are m and -s everywhere.
-  const double mx1 = F.M[0][rx][1], sx1 = F.S[0][rx][1], my1 = F.M[1][ry][1], sy1 = F.S[1][ry][1];
+  const double mx1 = F.M[0][rx][1], sx1 = F.S[0][rx][1];
+  int ry[FS_R];
+  double my1[FS_R], sy1[FS_R];
+#pragma unroll
+  for (int b = 0; b < FS_R; ++b) {
+    ry[b] = row_type(min(j + b, g.nyn - 1), g.nyn);
+    my1[b] = F.M[1][ry[b]][1];
+    sy1[b] = F.S[1][ry[b]][1];
+  }
   // halo node of the staged tile that this thread fills besides its own: two
   // rows of 34, then two columns of 8
+  static_assert(2 * FS_X + 2 * FB_Y <= FS_NT, "one halo node per thread");
   const bool halo = tid < 2 * FS_X + 2 * FB_Y;
   int hx, hy;
   if (tid < 2 * FS_X) {
@@ -105,74 +119,100 @@ __global__ void __launch_bounds__(FB_NT, FB_RESIDENT)
   // values of the next plane and of the one after it: one plane's work does not
   // cover the latency of its loads
   struct In {
-    double r, p, x, hr, hp;
+    double r[FS_R], p[FS_R], x[FS_R], hr, hp;
   };
   auto load = [&](int kp, int64_t o) {
-    double nr = 0, np = 0, nx = 0, nhr = 0, nhp = 0;
-    if (kp < 0 || kp >= g.nzn || kp > k1) return In{0, 0, 0, 0, 0};
-    if (act) {
-      nr = r[o + own];
-      if (!first) {
-        np = pin[o + own];
-        if (kp >= k0 && kp < k1) nx = x[o + own];
+    In v{};
+    if (kp < 0 || kp >= g.nzn || kp > k1) return v;
+    const double *rp = r + (o + own), *pp = pin + (o + own), *xp = x + (o + own);
+    const bool kown = kp >= k0 && kp < k1;
+#pragma unroll
+    for (int b = 0; b < FS_R; ++b)
+      if (act[b]) {
+        v.r[b] = rp[b * g.nxn];
+        if (!first) {
+          v.p[b] = pp[b * g.nxn];
+          if (kown) v.x[b] = xp[b * g.nxn];
+        }
       }
-    }
     if (hact) {
-      nhr = r[o + hown];
-      if (!first) nhp = pin[o + hown];
+      v.hr = r[o + hown];
+      if (!first) v.hp = pin[o + hown];
     }
-    return In{nr, np, nx, nhr, nhp};
+    return v;
   };
   In n0 = load(k0 - 1, (k0 - 1) * pl), n1 = load(k0, k0 * pl);
-  double a0 = 0, a1 = 0, b0 = 0, b1 = 0, p1 = 0, dsum = 0.0;  // planes kp - 2, kp - 1
+  double a0[FS_R] = {}, a1[FS_R] = {}, b0[FS_R] = {}, b1[FS_R] = {};  // planes kp - 2, kp - 1
+  double p1[FS_R] = {}, dsum = 0.0;
   const int rz0 = row_type(max(k0 - 1, 0), g.nzn);
-  double iv = F.inv[rx][ry][rz0], ivh = F.inv[hrx][hry][rz0];  // of plane kp
-  int64_t o = (k0 - 1) * pl;                                   // first node of plane kp
+  double iv[FS_R], ivh = F.inv[hrx][hry][rz0];  // of plane kp
+#pragma unroll
+  for (int b = 0; b < FS_R; ++b) iv[b] = F.inv[rx][ry[b]][rz0];
+  int64_t o = (k0 - 1) * pl;  // first node of plane kp
   for (int kp = k0 - 1; kp <= k1; ++kp) {
     double(*t)[FS_X] = tile[kp & 1];
     if (kp == 1 || kp == g.nzn - 1) {
       const int rz = row_type(kp, g.nzn);
-      iv = F.inv[rx][ry][rz];
+#pragma unroll
+      for (int b = 0; b < FS_R; ++b) iv[b] = F.inv[rx][ry[b]][rz];
       ivh = F.inv[hrx][hry][rz];
     }
-    const double pn = iv * n0.r + beta * n0.p;
-    const double xn = n0.x + alpha * n0.p;
-    t[ty + 1][tx + 1] = pn;
-    if (halo) t[hy][hx] = ivh * n0.hr + beta * n0.hp;
-    if (act && kp >= k0 && kp < k1) {
-      pout[o + own] = pn;
-      x[o + own] = xn;
+    const bool kown = kp >= k0 && kp < k1;
+    double *po = pout + (o + own), *xo = x + (o + own);
+    double pn[FS_R];
+#pragma unroll
+    for (int b = 0; b < FS_R; ++b) {
+      pn[b] = iv[b] * n0.r[b] + beta * n0.p[b];
+      t[ty + b + 1][tx + 1] = pn[b];
+      if (act[b] && kown) {
+        po[b * g.nxn] = pn[b];
+        xo[b * g.nxn] = n0.x[b] + alpha * n0.p[b];
+      }
     }
+    if (halo) t[hy][hx] = ivh * n0.hr + beta * n0.hp;
     n0 = n1;
     n1 = load(kp + 2, o + 2 * pl);
     __syncthreads();  // plane kp staged (its buffer was last read two planes ago)
-    double a2 = 0.0, b2 = 0.0;
+    double a2[FS_R] = {}, b2[FS_R] = {};
     if (kp >= 0 && kp < g.nzn) {
-      double xm[3], xs[3];
+      double xm[FS_R + 2], xs[FS_R + 2];
 #pragma unroll
-      for (int b = 0; b < 3; ++b) {
+      for (int b = 0; b < FS_R + 2; ++b) {
         const double v = t[ty + b][tx + 1], w = t[ty + b][tx] + t[ty + b][tx + 2];
         xm[b] = fma(mx1, v, F.M[0][1][0] * w);
         xs[b] = fma(sx1, v, F.S[0][1][0] * w);
       }
-      const double wm = xm[0] + xm[2];
-      const double mm = fma(my1, xm[1], F.M[1][1][0] * wm), ms = fma(sy1, xm[1], F.S[1][1][0] * wm);
-      const double sm = fma(my1, xs[1], F.M[1][1][0] * (xs[0] + xs[2]));
-      a2 = fma(F.r2, sm + ms, mm);
-      b2 = F.r2 * mm;
+#pragma unroll
+      for (int b = 0; b < FS_R; ++b) {
+        const double wm = xm[b] + xm[b + 2];
+        const double mm = fma(my1[b], xm[b + 1], F.M[1][1][0] * wm),
+                     ms = fma(sy1[b], xm[b + 1], F.S[1][1][0] * wm);
+        const double sm = fma(my1[b], xs[b + 1], F.M[1][1][0] * (xs[b] + xs[b + 2]));
+        a2[b] = fma(F.r2, sm + ms, mm);
+        b2[b] = F.r2 * mm;
+      }
     }
-    if (kp > k0 && act) {
+    if (kp > k0) {
       const int zt = row_type(kp - 1, g.nzn);
-      const double v = fma(F.M[2][zt][1], a1, F.M[2][1][0] * (a0 + a2)) +
-                       fma(F.S[2][zt][1], b1, F.S[2][1][0] * (b0 + b2));
-      q[o - pl + own] = v;
-      dsum += p1 * v;
+      const double mz = F.M[2][zt][1], sz = F.S[2][zt][1];
+      double* qo = q + (o - pl + own);
+#pragma unroll
+      for (int b = 0; b < FS_R; ++b)
+        if (act[b]) {
+          const double v = fma(mz, a1[b], F.M[2][1][0] * (a0[b] + a2[b])) +
+                           fma(sz, b1[b], F.S[2][1][0] * (b0[b] + b2[b]));
+          qo[b * g.nxn] = v;
+          dsum += p1[b] * v;
+        }
     }
-    a0 = a1;
-    a1 = a2;
-    b0 = b1;
-    b1 = b2;
-    p1 = pn;
+#pragma unroll
+    for (int b = 0; b < FS_R; ++b) {
+      a0[b] = a1[b];
+      a1[b] = a2[b];
+      b0[b] = b1[b];
+      b1[b] = b2[b];
+      p1[b] = pn[b];
+    }
     o += pl;
   }
   double vv[1] = {dsum};
@@ -314,7 +354,7 @@ void launch_filter_step(cudaStream_t s, const double* pin, double* pout, const d
   int kc;
   const dim3 grid = step_grid(g, &kc);
   launch_dep(one_wave((int64_t)grid.x * grid.y * grid.z, FB_RESIDENT), k_filter_step, grid,
-             dim3(FB_X, FB_Y), 0, s, pin, pout, r, x, q, g, F, kc, st, partials);
+             dim3(FB_X, FB_Y / FS_R), 0, s, pin, pout, r, x, q, g, F, kc, st, partials);
   HX_CHECK_LAUNCH();
 }
 
