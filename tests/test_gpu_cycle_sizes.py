@@ -1,8 +1,8 @@
 """Multigrid cycles on the row lengths where the row-wise grid transfers and
 the FP32 cycle vectors of the FP64 solve change form: rows shorter than a
-warp, more than 128 coarse nodes (two chunks), more than 1024 DOFs (two
-passes of a CTA), odd DOF counts (every grid here has an odd node count,
-so the 2-wide residual update ends in a scalar tail)."""
+warp, rows of more than one pass of a CTA (256 coarse DOFs in the restriction,
+512 fine ones in the prolongation), odd DOF counts (every grid here has an odd
+node count, so the 2-wide residual update ends in a scalar tail)."""
 import numpy as np
 import pytest
 
