@@ -51,9 +51,12 @@ struct DevBuf {
 };
 
 // ---- operator (hx_operator.cu) ----
-// CTAs of one launch (each leaves a partial sum in the reduction workspace)
+// CTAs of one launch (each leaves a partial sum in the reduction workspace):
+// the most of any mode, and those of FP64 K x alone, whose CTAs own more nodes
+// than those of the fused steps
 template <typename T>
 size_t mv_num_blocks(const Grid& g);
+size_t mv_apply_blocks(const Grid& g);
 template <typename T>
 void launch_matvec(cudaStream_t s, int mode, const T* x, T* y, const T* fac, const uint8_t* nmask,
                    const Grid& g, const ElemCoef<T>& K, T shift, CgState* st, double* partials,

@@ -86,8 +86,8 @@ extern "C" HX_API hx_status hx_apply_stiffness_noalloc(int64_t nx, int64_t ny, i
   g.nxn = g.nxe + 1;
   g.nyn = g.nye + 1;
   g.nzn = g.nze + 1;
-  // The reduction writes one partial sum per CTA of the operator kernel.
-  if (hx::mv_num_blocks<double>(g) > (size_t)HX_NOALLOC_MAX_BLOCKS) return HX_BAD_ARG;
+  // The reduction writes one partial sum per CTA of the one launch below.
+  if (hx::mv_apply_blocks(g) > (size_t)HX_NOALLOC_MAX_BLOCKS) return HX_BAD_ARG;
   unsigned char* base = nullptr;
   const hx_status st = scratch_address(&base);
   if (st != HX_OK) return st;

@@ -1035,16 +1035,22 @@ void launch_struct(cudaStream_t s, const T* fac, const uint8_t* nmask, const Gri
     go(std::false_type{});
 }
 
+template <typename T, bool FUSED>
+size_t num_blocks(const Grid& g) {
+  const dim3 a = mv_grid<T, FUSED>(g, mv_kchunk<T, FUSED>(g));
+  return (size_t)a.x * a.y * a.z;
+}
+
 }  // namespace
 
 template <typename T>
 size_t mv_num_blocks(const Grid& g) {
-  const dim3 a = mv_grid<T, true>(g, mv_kchunk<T, true>(g));
-  const dim3 b = mv_grid<T, false>(g, mv_kchunk<T, false>(g));
-  return std::max((size_t)a.x * a.y * a.z, (size_t)b.x * b.y * b.z);
+  return std::max(num_blocks<T, true>(g), num_blocks<T, false>(g));
 }
 template size_t mv_num_blocks<float>(const Grid&);
 template size_t mv_num_blocks<double>(const Grid&);
+
+size_t mv_apply_blocks(const Grid& g) { return num_blocks<double, false>(g); }
 
 template <typename T>
 void launch_matvec(cudaStream_t s, int mode, const T* x, T* y, const T* fac, const uint8_t* nmask,
