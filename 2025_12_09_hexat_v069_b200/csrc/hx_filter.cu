@@ -301,7 +301,8 @@ __global__ void __launch_bounds__(FB_NT)
   }
 }
 
-// element value = mean of its 8 nodal values (GPUHelmholtz.jl:78-89)
+// element value = mean of its 8 nodal values (GPUHelmholtz.jl:78-89) of x + alpha p,
+// of x alone without p
 __global__ void __launch_bounds__(FB_NT)
     k_filter_extract(const double* __restrict__ x, const double* __restrict__ p, double alpha,
                      double* __restrict__ out, Grid g) {
@@ -311,7 +312,7 @@ __global__ void __launch_bounds__(FB_NT)
     const int k = row / (unsigned)g.nye, j = row - k * (unsigned)g.nye;
     for (int i = threadIdx.x; i < g.nxe; i += FB_X) {
       const int64_t n0 = (int64_t)k * pl + (int64_t)j * g.nxn + i;
-      auto at = [&](int64_t n) { return x[n] + alpha * p[n]; };
+      auto at = [&](int64_t n) { return p ? x[n] + alpha * p[n] : x[n]; };
       const double s = at(n0) + at(n0 + 1) + at(n0 + g.nxn + 1) + at(n0 + g.nxn) + at(n0 + pl) +
                        at(n0 + pl + 1) + at(n0 + pl + g.nxn + 1) + at(n0 + pl + g.nxn);
       out[(int64_t)row * g.nxe + i] = s / 8.0;

@@ -168,7 +168,8 @@ void launch_filter_step(cudaStream_t s, const double* pin, double* pout, const d
                         double* partials);
 void launch_filter_update(cudaStream_t s, double* r, const double* q, const Grid& g,
                           const FilterCoef& F, CgState* st, double* partials);
-// out = element means of x + alpha p (alpha: the pending step of the state)
+// out = element means of x + alpha p (alpha: the pending step of the state), of
+// x where p is null
 void launch_filter_extract(cudaStream_t s, const double* x, const double* p, double alpha,
                            double* out, const Grid& g);
 

@@ -708,9 +708,9 @@ hx_status filter_grid(hx_ctx* c, const Grid& g, const double h[3], const double*
     launch_fill_zero(c->stream, out, g.elems() * sizeof(double));
   } else {
     // the last step x += alpha p is pending (after a breakdown alpha is invalid
-    // and no step is)
+    // and no step is; in iteration 0 the other p was not written either)
     const bool pending = sf.status != HX_ST_BREAKDOWN;
-    launch_filter_extract(c->stream, x, p[(sf.iter + 1) & 1], pending ? sf.alpha : 0.0, out, g);
+    launch_filter_extract(c->stream, x, pending ? p[(sf.iter + 1) & 1] : nullptr, sf.alpha, out, g);
   }
   HX_CUDA(cudaStreamSynchronize(c->stream));
   R.iterations = sf.iter;
