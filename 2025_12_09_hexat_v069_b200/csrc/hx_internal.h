@@ -50,6 +50,13 @@ struct DevBuf {
   }
 };
 
+// Training buffers of one network: its activations, the gradients with respect
+// to them (stack_backward_train) and the weight-gradient partials.
+struct NetTrain {
+  __nv_bfloat16 *act[7] = {}, *ge[8] = {};
+  float* part = nullptr;
+};
+
 // ---- operator (hx_operator.cu) ----
 // CTAs of one launch (each leaves a partial sum in the reduction workspace):
 // the most of any mode, and those of FP64 K x alone, whose CTAs own more nodes
@@ -305,12 +312,13 @@ struct hx_ctx {
     hx::DevBuf<unsigned char> live;
     hx::DevBuf<__nv_bfloat16> wf, wb, tmp[2];
     struct Level {  // one node-grid level (0 = the mesh's node grid)
-      hx::DevBuf<float> x, acc, gx, feat;  // [node][3] fields, [node] feature
-      hx::DevBuf<__nv_bfloat16> x0, y, act[7];  // network input, output, training activations
-      hx::DevBuf<__nv_bfloat16> ge[8];          // training: gradients (stack_backward_train)
-      hx::DevBuf<float> part;                   // training: weight-gradient partials
-      hx::DevBuf<__nv_bfloat16> pp[2];          // application ping-pong (levels >= 2)
+      hx::DevBuf<float> x, acc, feat;       // [node][3] fields, [node] feature
+      hx::DevBuf<__nv_bfloat16> x0, y;      // network input, output
+      hx::DevBuf<__nv_bfloat16> pp[2];      // application ping-pong (levels >= 2)
+      float* gx = nullptr;                  // training: gradient field (in `train`)
+      hx::NetTrain t;                       // training: the network's buffers (in `train`)
     } lv[8];
+    hx::DevBuf<unsigned char> train;  // the training buffers of all levels
     // side streams and events: the coarser networks run beside the finest;
     // ev_x[i]: side i's level restricted, ev_join[i]: its correction summed
     cudaStream_t side[2] = {nullptr, nullptr};
