@@ -196,8 +196,13 @@ CgState GraphLoop::run(bool ahead, double wall_limit_ms, double t0, bool* timed_
   ahead = ahead && max_launches == 0;
   CgState st{};
   for (int i = 0;; ++i) {
-    while (launched <= i + (ahead ? 1 : 0)) launch();
+    if (launched <= i) launch();
+    const double from = now_ms();
+    if (ahead && (wall_limit_ms <= 0 ||
+                  (graph_ms_ >= 0 && from - t0 + graph_ms_ <= wall_limit_ms)))
+      launch();
     HX_CUDA(cudaEventSynchronize(ev_[i & 1]));
+    graph_ms_ = std::max(graph_ms_, now_ms() - from);
     st = c_->h_state[4 + (i & 1)];
     if (st.status != HX_RUNNING) break;
     if (max_launches > 0 && i + 1 >= max_launches) break;
@@ -207,8 +212,9 @@ CgState GraphLoop::run(bool ahead, double wall_limit_ms, double t0, bool* timed_
       break;
     }
   }
-  // a launch ahead may have moved a state that was still running
+  // a launch ahead may have moved, and ended, a state that was still running
   if (ahead) st = get_state(c_, slot_);
+  if (st.status != HX_RUNNING) *timed_out = false;
   return st;
 }
 

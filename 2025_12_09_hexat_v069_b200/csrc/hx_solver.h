@@ -25,7 +25,9 @@ class GraphLoop {
   // for the state read after a launch.  ahead: launch the next graph before
   // the state of the last one is read (not with max_launches), so that the GPU
   // does not wait for the host; once the state has stopped, one launch more
-  // runs through without effect.  Returns the state after all launches.
+  // runs through without effect.  With a wall limit, only where the graph in
+  // flight should end within it: the launches are those that would be made one
+  // by one.  Returns the state after all launches; *timed_out: it still runs.
   CgState run(bool ahead, double wall_limit_ms, double t0, bool* timed_out, int max_launches = 0,
               const std::function<bool(const CgState&)>& keep_going = {});
 
@@ -35,6 +37,7 @@ class GraphLoop {
   int slot_;
   cudaGraphExec_t exec_ = nullptr;
   int64_t per_graph_ = 0;
+  double graph_ms_ = -1;  // the longest that the host waited for a graph (< 0: not known)
   cudaEvent_t ev_[2] = {nullptr, nullptr};
 };
 // node masks, diagonal, shift and M^-1 (FP64) for `fac`; returns max diag
