@@ -628,6 +628,11 @@ std::function<void()> net_time_body(hx_ctx* c, int which) {
   };
 }
 
+// Pairs of iterations per graph of the learned forms: one, unless the caller
+// asks for a poll period, since the preconditioner's kernels run whole after the
+// state has stopped.
+static int fcg_reps(int check_every) { return std::max(1, check_every / 2); }
+
 // ---------------------------------------------------------------------------
 // Flexible CG with the network preconditioner (FP64 vectors and operator,
 // BF16 network).  Falls back to Jacobi-PCG from the current iterate when
@@ -694,7 +699,7 @@ static CgState learned_fcg(hx_ctx* c, const double* fac, const double* b, double
     stalled = !o.learned_no_fallback && sv.iter - best_it > std::max(500, sv.iter / 4);
     return !stalled;
   };
-  GraphLoop loop(c, 0, 1, body);
+  GraphLoop loop(c, 0, fcg_reps(o.check_every), body);
   sf = loop.run(true, o.wall_limit_ms, t0, timed_out, 0, keep_going);
   if (sf.status != HX_RUNNING) stalled = false;
   // pending x += alpha p of the last completed iteration
@@ -831,9 +836,8 @@ static CgState learned_fcg_mixed(hx_ctx* c, const double* fac, const double* b, 
                            si, c->d_partials.p);
     launch_cg_update2<float>(c->stream, r32, q32, minv32, n, si, c->d_partials.p, ys);
   };
-  // iterations alternate p from P1 to P0 and back.  Two iterations per launch:
-  // the preconditioner's kernels run whole after the state has stopped
-  GraphLoop loop(c, 1, 1, [&]() {
+  // iterations alternate p from P1 to P0 and back
+  GraphLoop loop(c, 1, multigrid ? 1 : fcg_reps(o.check_every), [&]() {
     one(P1, P0);
     one(P0, P1);
   });

@@ -76,7 +76,8 @@ typedef struct hx_solve_opts {
   int32_t warm_start;      /* 1: u_inout holds the initial guess */
   double shift_factor;     /* shift s = shift_factor * max(diag over free DOFs) */
   double wall_limit_ms;    /* 0: no limit */
-  int32_t check_every;     /* host poll period in iterations (0: automatic) */
+  int32_t check_every;     /* host poll period in iterations (0: automatic; the
+                              multigrid forms poll every 2) */
   int32_t keep_best;       /* 1: keep the best iterate (reference semantics) */
   double inner_tol;        /* mixed precision: the FP32 recursive residual is
                               replaced by the FP64 true residual each time it
