@@ -99,8 +99,10 @@ static double now_ms() {
 void ensure_workspace(hx_ctx* c) {
   if (!c->h_state) HX_CUDA(cudaMallocHost(&c->h_state, 6 * sizeof(CgState)));
   c->d_state.ensure(4);
-  const size_t nb = std::max<size_t>(
-      std::max(mv_num_blocks<float>(c->g), mv_num_blocks<double>(c->g)), 64ull * sm_count());
+  // (the filter and the density update bring their own grid: no mesh, no operator)
+  size_t nb = 64ull * sm_count();
+  if (c->has_mesh)
+    nb = std::max({nb, mv_num_blocks<float>(c->g), mv_num_blocks<double>(c->g)});
   c->d_partials.ensure(4 * nb);
   c->d_scalars.ensure(16);
 }
