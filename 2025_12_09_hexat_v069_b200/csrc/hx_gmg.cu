@@ -518,9 +518,16 @@ void gmg_setup(hx_ctx* c, const double* fac, double shift) {
   HX_CUDA(cudaMemsetAsync(lst, 0, HX_GMG_MAX_LEVELS * sizeof(CgState), s));
   HX_CUDA(cudaEventRecord(G.ev_join[0], s));
   HX_CUDA(cudaStreamWaitEvent(G.side[0], G.ev_join[0], 0));
-  // the second half of the partial sums serves the side stream: a launch leaves
-  // at most two per CTA, and the workspace holds four for the largest grid
-  double* part[2] = {c->d_partials.p, c->d_partials.p + c->d_partials.n / 2};
+  // partial sums of level 0's launches, then those of the side stream: one per
+  // CTA of a step, three per CTA of k_cg_init.  (A level's chunks are chosen for its
+  // own grid, so level 0 need not have the most CTAs; the coarsest level's PCG in
+  // the cycles needs no more than a part either.)
+  size_t most = 0;
+  for (int l = 0; l < G.nl; ++l)
+    most = std::max({most, mv_num_blocks<float>(G.lv[l].g),
+                     (size_t)3 * vec_blocks(G.lv[l].g.dofs())});
+  double* sums = c->d_partials.ensure(2 * most);
+  double* part[2] = {sums, sums + most};
   int64_t off = 0;
   for (int l = 0; l + 1 < G.nl; ++l) {
     auto& L = G.lv[l];
