@@ -61,6 +61,7 @@ constexpr int FB_X = 32, FB_Y = 8, FB_NT = FB_X * FB_Y;
 constexpr int FS_X = FB_X + 2, FS_Y = FB_Y + 2;  // staged tile with its halo
 constexpr int FS_R = 2, FS_NT = FB_NT / FS_R;    // node rows and threads of the step
 constexpr int FB_RESIDENT = 4;
+constexpr int FB_ROW_RESIDENT = 6;  // CTAs per SM of the row kernels (40 registers)
 
 // One CTA owns a 32 x 8 node column over planes [k0, k1) and marches along z:
 // plane kp's new direction p = D^-1 r + beta p_in goes to shared memory (tile
@@ -227,11 +228,15 @@ __global__ void __launch_bounds__(FS_NT, FB_RESIDENT)
 }
 
 // The kernels below take node (element) rows by warp: no division per entry.
+// Few long rows are cut into segments of `len` entries (blockIdx.y; see
+// row_grid).
+__device__ __forceinline__ int seg_begin(int len) { return blockIdx.y * len + threadIdx.x; }
+__device__ __forceinline__ int seg_end(int len, int n) { return min((int)(blockIdx.y + 1) * len, n); }
 
 // r -= alpha q, r.D^-1 r and r.r, tests, beta.
-__global__ void __launch_bounds__(FB_NT)
+__global__ void __launch_bounds__(FB_NT, FB_ROW_RESIDENT)
     k_filter_update(double* __restrict__ r, const double* __restrict__ q, Grid g,
-                    const __grid_constant__ FilterCoef F, CgState* st, double* partials) {
+                    const __grid_constant__ FilterCoef F, int len, CgState* st, double* partials) {
   pdl_wait();
   pdl_trigger();
   if (st->status != HX_RUNNING) return;
@@ -239,6 +244,7 @@ __global__ void __launch_bounds__(FB_NT)
   __shared__ CgState s0;  // read after grid_reduce's barriers
   load_state(&s0, st);
   double rz = 0, rr = 0;
+  const int i0 = seg_begin(len), i1 = seg_end(len, g.nxn);
   const unsigned rows = (unsigned)g.nyn * (unsigned)g.nzn;
   for (unsigned row = blockIdx.x * FB_Y + threadIdx.y; row < rows; row += gridDim.x * FB_Y) {
     const int k = row / (unsigned)g.nyn, j = row - k * (unsigned)g.nyn;
@@ -246,7 +252,7 @@ __global__ void __launch_bounds__(FB_NT)
     const double in = F.inv[1][ty][tz], lo = F.inv[0][ty][tz], hi = F.inv[2][ty][tz];
     const int64_t o = (int64_t)row * g.nxn;
 #pragma unroll 4
-    for (int i = threadIdx.x; i < g.nxn; i += FB_X) {
+    for (int i = i0; i < i1; i += FB_X) {
       const double ri = r[o + i] - alpha * q[o + i];
       r[o + i] = ri;
       const double d = i == 0 ? lo : (i == g.nxn - 1 ? hi : in);
@@ -264,13 +270,14 @@ __global__ void __launch_bounds__(FB_NT)
 // state of x = 0.
 __global__ void __launch_bounds__(FB_NT)
     k_filter_init(const double* __restrict__ rho, double* __restrict__ r, Grid g,
-                  const __grid_constant__ FilterCoef F, CgState* st, double* partials) {
+                  const __grid_constant__ FilterCoef F, int len, CgState* st, double* partials) {
   double rz = 0, rr = 0;
+  const int i0 = seg_begin(len), i1 = seg_end(len, g.nxn);
   const unsigned rows = (unsigned)g.nyn * (unsigned)g.nzn;
   for (unsigned row = blockIdx.x * FB_Y + threadIdx.y; row < rows; row += gridDim.x * FB_Y) {
     const int k = row / (unsigned)g.nyn, j = row - k * (unsigned)g.nyn;
     const int ty = row_type(j, g.nyn), tz = row_type(k, g.nzn);
-    for (int i = threadIdx.x; i < g.nxn; i += FB_X) {
+    for (int i = i0; i < i1; i += FB_X) {
       double s = 0.0;
 #pragma unroll
       for (int dk = -1; dk <= 0; ++dk)
@@ -303,14 +310,15 @@ __global__ void __launch_bounds__(FB_NT)
 
 // element value = mean of its 8 nodal values (GPUHelmholtz.jl:78-89) of x + alpha p,
 // of x alone without p
-__global__ void __launch_bounds__(FB_NT)
+__global__ void __launch_bounds__(FB_NT, FB_ROW_RESIDENT)
     k_filter_extract(const double* __restrict__ x, const double* __restrict__ p, double alpha,
-                     double* __restrict__ out, Grid g) {
+                     double* __restrict__ out, Grid g, int len) {
+  const int i0 = seg_begin(len), i1 = seg_end(len, g.nxe);
   const unsigned rows = (unsigned)g.nye * (unsigned)g.nze;
   const int64_t pl = (int64_t)g.nxn * g.nyn;
   for (unsigned row = blockIdx.x * FB_Y + threadIdx.y; row < rows; row += gridDim.x * FB_Y) {
     const int k = row / (unsigned)g.nye, j = row - k * (unsigned)g.nye;
-    for (int i = threadIdx.x; i < g.nxe; i += FB_X) {
+    for (int i = i0; i < i1; i += FB_X) {
       const int64_t n0 = (int64_t)k * pl + (int64_t)j * g.nxn + i;
       auto at = [&](int64_t n) { return p ? x[n] + alpha * p[n] : x[n]; };
       const double s = at(n0) + at(n0 + 1) + at(n0 + g.nxn + 1) + at(n0 + g.nxn) + at(n0 + pl) +
@@ -320,8 +328,19 @@ __global__ void __launch_bounds__(FB_NT)
   }
 }
 
-unsigned row_blocks(int64_t rows) {
-  return (unsigned)std::max<int64_t>(1, std::min<int64_t>(cdiv(rows, FB_Y), 8LL * sm_count()));
+// CTAs for `rows` rows of n entries (at most one wave of resident ones), and the
+// entries of a segment.  A warp that owns a row takes n / 32 steps; where the rows
+// fill less than four CTAs per SM they are cut, down to 128 entries (four loads in
+// flight per lane), until they do.  By whole rows a filter (radius 4) took 45 ms on
+// 100000 x 1 x 1 elements and 1.5 ms on 2000 x 40 x 2, where most SMs had no row;
+// now 1.9 and 0.7 ms.
+dim3 row_grid(int64_t rows, int n, int* len) {
+  const unsigned bx = (unsigned)std::max<int64_t>(
+      1, std::min<int64_t>(cdiv(rows, FB_Y), (int64_t)FB_ROW_RESIDENT * sm_count()));
+  const int64_t want = std::max<int64_t>(1, 4LL * sm_count() / bx);
+  const unsigned seg = (unsigned)std::min<int64_t>(want, cdiv(n, 4 * FB_X));
+  *len = (int)cdiv(cdiv(n, seg), FB_X) * FB_X;
+  return dim3(bx, cdiv(n, *len));
 }
 
 // Planes per CTA of the step: one wave of resident CTAs (two halo planes are
@@ -337,15 +356,16 @@ dim3 step_grid(const Grid& g, int* kchunk) {
 }  // namespace
 
 size_t filter_blocks(const Grid& g) {
-  int kc;
-  const dim3 a = step_grid(g, &kc);
-  return std::max<size_t>((size_t)a.x * a.y * a.z, row_blocks((int64_t)g.nyn * g.nzn));
+  int kc, len;
+  const dim3 a = step_grid(g, &kc), b = row_grid((int64_t)g.nyn * g.nzn, g.nxn, &len);
+  return std::max((size_t)a.x * a.y * a.z, (size_t)b.x * b.y);
 }
 
 void launch_filter_init(cudaStream_t s, const double* rho, double* r, const Grid& g,
                         const FilterCoef& F, CgState* st, double* partials) {
-  k_filter_init<<<row_blocks((int64_t)g.nyn * g.nzn), dim3(FB_X, FB_Y), 0, s>>>(rho, r, g, F, st,
-                                                                              partials);
+  int len;
+  const dim3 grid = row_grid((int64_t)g.nyn * g.nzn, g.nxn, &len);
+  k_filter_init<<<grid, dim3(FB_X, FB_Y), 0, s>>>(rho, r, g, F, len, st, partials);
   HX_CHECK_LAUNCH();
 }
 
@@ -361,16 +381,18 @@ void launch_filter_step(cudaStream_t s, const double* pin, double* pout, const d
 
 void launch_filter_update(cudaStream_t s, double* r, const double* q, const Grid& g,
                           const FilterCoef& F, CgState* st, double* partials) {
-  const unsigned blocks = row_blocks((int64_t)g.nyn * g.nzn);
-  launch_dep(one_wave(blocks, 7), k_filter_update, blocks, dim3(FB_X, FB_Y), 0, s, r, q, g, F, st,
-             partials);
+  int len;
+  const dim3 grid = row_grid((int64_t)g.nyn * g.nzn, g.nxn, &len);
+  launch_dep(one_wave((int64_t)grid.x * grid.y, FB_ROW_RESIDENT), k_filter_update, grid, dim3(FB_X, FB_Y), 0, s,
+             r, q, g, F, len, st, partials);
   HX_CHECK_LAUNCH();
 }
 
 void launch_filter_extract(cudaStream_t s, const double* x, const double* p, double alpha,
                            double* out, const Grid& g) {
-  k_filter_extract<<<row_blocks((int64_t)g.nye * g.nze), dim3(FB_X, FB_Y), 0, s>>>(x, p, alpha,
-                                                                                 out, g);
+  int len;
+  const dim3 grid = row_grid((int64_t)g.nye * g.nze, g.nxe, &len);
+  k_filter_extract<<<grid, dim3(FB_X, FB_Y), 0, s>>>(x, p, alpha, out, g, len);
   HX_CHECK_LAUNCH();
 }
 
