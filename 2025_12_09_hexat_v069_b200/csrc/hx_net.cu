@@ -412,26 +412,27 @@ void net_forward_backward(hx_ctx* c, int nx, int ny, int nz, const float* x0, co
   const GridN g{nx, ny, nz};
   const int64_t nn = (int64_t)nx * ny * nz;
   auto& N = c->net;
-  DevBuf<__nv_bfloat16> bx0, by;
-  DevBuf<unsigned char> train;
-  bx0.ensure(nn * 16);
-  by.ensure(nn * 8);
+  // in the block of the training steps, which place their buffers anew (with
+  // buffers of its own a call took 2.8 ms on 9 x 9 x 9 nodes, now 0.26)
+  __nv_bfloat16 *bx0, *by;
   NetTrain t;
   auto place = [&](unsigned char* base) {
     Carve m{base};
+    bx0 = m.take<__nv_bfloat16>(nn * 16);
+    by = m.take<__nv_bfloat16>(nn * 8);
     place_train(m, g, t);
     return m.at;
   };
   const size_t bytes = place(nullptr);
-  place(train.ensure(bytes));
-  upload_act16(c, g, x0, bx0.p);
-  stack_forward_train(c, c->stream, 0, g, bx0.p, t, by.p);
+  place(N.train.ensure(bytes));
+  upload_act16(c, g, x0, bx0);
+  stack_forward_train(c, c->stream, 0, g, bx0, t, by);
   std::vector<__nv_bfloat16> hy((size_t)nn * 8);
-  HX_CUDA(cudaMemcpyAsync(hy.data(), by.p, hy.size() * 2, cudaMemcpyDeviceToHost, c->stream));
+  HX_CUDA(cudaMemcpyAsync(hy.data(), by, hy.size() * 2, cudaMemcpyDeviceToHost, c->stream));
   upload_act16(c, g, dy, t.ge[0]);
   HX_CUDA(cudaMemsetAsync(N.grad.p, 0, NET_PARAMS * sizeof(float), c->stream));
   HX_CUDA(cudaStreamSynchronize(c->stream));
-  stack_backward_train(c, c->stream, 0, g, bx0.p, t, false);
+  stack_backward_train(c, c->stream, 0, g, bx0, t, false);
   HX_CUDA(cudaMemcpyAsync(grads, N.grad.p, NET_PARAMS * sizeof(float), cudaMemcpyDeviceToHost,
                           c->stream));
   HX_CUDA(cudaStreamSynchronize(c->stream));

@@ -1,5 +1,5 @@
-"""Device allocations of training steps: the first step of a context makes a
-few, later ones none.  Counted in a child process whose cudaMalloc is wrapped
+"""Device allocations of training steps and gradient checks: the first of a
+context makes a few, later ones none.  Counted in a child process whose cudaMalloc is wrapped
 by a small preloaded library."""
 import os
 import subprocess
@@ -27,6 +27,7 @@ int cuda_mallocs(void) { return n; }
 
 CHILD = r"""
 import ctypes, importlib, sys
+import numpy as np
 import torch
 hx = importlib.import_module("2025_12_09_hexat_v069_b200")
 learned = importlib.import_module("2025_12_09_hexat_v069_b200.learned")
@@ -45,7 +46,23 @@ with hx.Context(0) as ctx:
     for _ in range(2):
         ctx.net_train_batch([r.data_ptr()], [e.data_ptr()], 1e-4)
         c.append(count())
-print("allocations", c[0], c[1] - c[0], c[2] - c[1])
+    a = np.random.default_rng(0).standard_normal((9 * 9 * 9, 16)).astype(np.float32)
+    y, grads = ctx.net_forward_backward((9, 9, 9), a, a)
+    c.append(count())
+    y2, grads2 = ctx.net_forward_backward((9, 9, 9), a, a)
+    assert np.array_equal(y, y2) and np.array_equal(grads, grads2)
+    c.append(count())
+    # a training step after it places its buffers anew
+    p = learned.load_params()
+    out = []
+    for fb in (False, True):
+        ctx.net_set_params(p)
+        if fb:
+            ctx.net_forward_backward((9, 9, 9), a, a)
+        ctx.net_train_batch([r.data_ptr()], [e.data_ptr()], 1e-4)
+        out.append(ctx.net_get_params())
+    assert np.array_equal(*out)
+print("allocations", c[0], *(b - a for a, b in zip(c, c[1:])))
 """
 
 
@@ -57,7 +74,9 @@ def test_allocations_of_training_steps(tmp_path):
     out = subprocess.run([sys.executable, "-c", CHILD, str(lib)], env=env, cwd=ROOT, timeout=300,
                          capture_output=True, text=True)
     assert out.returncode == 0, out.stderr
-    before, first, second = map(int, out.stdout.split("allocations")[1].split())
+    before, first, second, fb, fb2 = map(int, out.stdout.split("allocations")[1].split())
     assert before > 0  # the wrapper is in place
     # vectors of the mesh and one block for the networks' training buffers
     assert first <= 12 and second == 0, (first, second)
+    # the gradient check on given data uses that block
+    assert fb <= 1 and fb2 == 0, (fb, fb2)
