@@ -973,16 +973,20 @@ __global__ void k_minv(const uint8_t* __restrict__ nmask, const T* __restrict__ 
 // CTAs) x (element layers each CTA works on, kc + 1, and one for its start and
 // end).  A last wave that fills few SMs costs as much as a full one; ties go
 // to the longer chunk.  Short chunks win only where the grid leaves SMs idle.
+// For a number of chunks only the shortest length counts, so a grid of n planes has
+// about 2 sqrt(n) candidates (1001 planes: 0.75 us instead of 3.5 for all lengths;
+// a call asks up to five times).
 template <typename T, bool FUSED>
 int mv_kchunk(const Grid& g) {
   const int64_t cols = (int64_t)cdiv(g.nxn, MV_BX - 1) * cdiv(g.nyn, mv_by<T, FUSED>() - 1);
   const int64_t slots = (int64_t)Tile<T, FUSED>::RESIDENT * sm_count();
   int best_kc = g.nzn;
   int64_t best = INT64_MAX;
-  for (int kc = 1; kc <= g.nzn; ++kc) {
-    const int64_t waves = cdiv(cols * cdiv(g.nzn, kc), slots);
-    const int64_t cost = waves * (kc + 2);
-    if (cost <= best) {
+  for (int kc = g.nzn; kc >= 1; --kc) {
+    const int chunks = cdiv(g.nzn, kc);
+    kc = cdiv(g.nzn, chunks);
+    const int64_t cost = (int64_t)cdiv(cols * chunks, slots) * (kc + 2);
+    if (cost < best) {
       best = cost;
       best_kc = kc;
     }

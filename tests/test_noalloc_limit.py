@@ -5,6 +5,7 @@ more than 16384 of them (about 1880 x 1880 nodes per plane).
 Without a device an accepted grid ends with HX_CUDA_ERROR when the scratch
 array's address is asked for, a refused one with HX_BAD_ARG before that."""
 import ctypes
+import time
 
 import numpy as np
 import pytest
@@ -32,6 +33,21 @@ def test_grids_taken_without_a_device(hx, dims, want):
     a = np.zeros(8)
     p = a.ctypes.data + (-a.ctypes.data) % 16
     assert _call(hx, dims, p, p, p, p) == want
+
+
+def test_blocks_of_a_tall_grid_are_counted_quickly(hx):
+    """A million planes: 25 us over the useful chunk lengths, 3.5 ms over all of them."""
+    import torch
+    if torch.cuda.is_available():
+        pytest.skip("a GPU is present: the call would run")
+    a = np.zeros(8)
+    p = a.ctypes.data + (-a.ctypes.data) % 16
+    best = 1e9
+    for _ in range(10):
+        t = time.perf_counter()
+        assert _call(hx, (1, 1, 1000000), p, p, p, p) == CUDA_ERROR
+        best = min(best, time.perf_counter() - t)
+    assert best < 1e-3
 
 
 @pytest.mark.gpu
