@@ -49,6 +49,7 @@
 // twice 179-208 us; positions advanced per plane instead of recomputed 176-182
 // us.
 #include <type_traits>
+#include <utility>
 
 #include "hx_internal.h"
 
@@ -251,6 +252,7 @@ struct OpArgs {
   const uint8_t* nmask;
   Grid g;
   int kchunk;
+  int yx;  // 1: blockIdx.x counts the columns in y (see mv_grid)
   CoefV<VecOf<T>, CUBE> K;
   T shift;
   T omega, gamma;  // MODE 5: recurrence coefficients
@@ -378,7 +380,8 @@ __global__ void __launch_bounds__(MV_BX* Tile<T, mode_fused(MODE)>::WARPS,
   const Grid& g = A.g;
   const int lx = threadIdx.x, wy = threadIdx.y;
   const int tid = lx + MV_BX * wy;
-  const int i0 = blockIdx.x * (MV_BX - 1), j0 = blockIdx.y * (BY - 1);
+  const int i0 = (A.yx ? blockIdx.y : blockIdx.x) * (MV_BX - 1);
+  const int j0 = (A.yx ? blockIdx.x : blockIdx.y) * (BY - 1);
   const int k0 = blockIdx.z * A.kchunk;
   const int k1 = min(k0 + A.kchunk, g.nzn);
   const int in = i0 - 1 + lx, jn = j0 - 1 + R * wy;  // first element column, first node
@@ -994,6 +997,10 @@ int mv_kchunk(const Grid& g) {
   return best_kc;
 }
 
+// CTA columns in x, columns in y, chunks.  A grid's y extent ends at 65535, which
+// more than 327000 node rows in y reach (the columns in x never do: 2^20 nodes
+// are 33826 of them): x and y are exchanged there.
+constexpr unsigned MAX_GRID_Y = 65535;
 template <typename T, bool FUSED>
 dim3 mv_grid(const Grid& g, int kchunk) {
   return dim3(cdiv(g.nxn, MV_BX - 1), cdiv(g.nyn, mv_by<T, FUSED>() - 1), cdiv(g.nzn, kchunk));
@@ -1013,7 +1020,9 @@ void launch_one(cudaStream_t s, OpArgs<T, CUBE>& a, const ElemCoef<T>& K) {
   });
   coef_v(K, a.K);
   a.kchunk = mv_kchunk<T, FUSED>(a.g);
-  const dim3 grid = mv_grid<T, FUSED>(a.g, a.kchunk);
+  dim3 grid = mv_grid<T, FUSED>(a.g, a.kchunk);
+  a.yx = grid.y > MAX_GRID_Y;
+  if (a.yx) std::swap(grid.x, grid.y);
   launch_dep(one_wave((int64_t)grid.x * grid.y * grid.z, Form::RESIDENT), k_struct<T, MODE, CUBE>,
              grid, dim3(MV_BX, Form::WARPS), smem, s, a);
   HX_CHECK_LAUNCH();
