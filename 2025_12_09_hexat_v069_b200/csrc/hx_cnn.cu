@@ -65,18 +65,19 @@ __device__ __forceinline__ unsigned swz(int row, int h) {
 // w+24 over all 512 nodes of the tile; the result goes to part[cta][27*256]
 // (FP32), summed later in fixed order.
 // ---------------------------------------------------------------------------
-// One launch takes all 8 uses of a network's 4 layers (job = blockIdx.z mod 8:
-// layer job & 3, transposed use below 4, forward use from there on): a layer's
-// tiles alone leave most SMs idle on the coarse levels.
+// One launch takes all 8 uses of a network's 4 layers (job = blockIdx.x mod 8:
+// layer job & 3, transposed use below 4, forward use from there on; x, since a
+// grid's y and z end at 65535): a layer's tiles alone leave most SMs idle on the
+// coarse levels.
 __global__ void __launch_bounds__(NTHREADS)
     k_conv3_wgrad(const __grid_constant__ WgradJobs jobs, float* __restrict__ part, GridN g) {
-  const int job = blockIdx.z & 7;
+  const int job = blockIdx.x & 7;
   const __nv_bfloat16* __restrict__ X = jobs.X[job];
   const __nv_bfloat16* __restrict__ D = jobs.D[job];
   extern __shared__ __align__(128) unsigned char smraw[];
   __nv_bfloat16* xs = reinterpret_cast<__nv_bfloat16*>(smraw);
   __nv_bfloat16* ds = xs + HNODES * C;  // [512 nodes][16], swizzled rows
-  const int x0 = blockIdx.x * TX, y0 = blockIdx.y * TY, z0 = (blockIdx.z >> 3) * TZ;
+  const int x0 = (blockIdx.x >> 3) * TX, y0 = blockIdx.y * TY, z0 = blockIdx.z * TZ;
   const unsigned xb = su32(xs), db = su32(ds);
   for (int ch = threadIdx.x; ch < HNODES * 2; ch += NTHREADS) {
     const int node = ch >> 1, h = ch & 1;
@@ -99,8 +100,9 @@ __global__ void __launch_bounds__(NTHREADS)
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int gq = lane >> 2, tq = lane & 3;
-  const size_t tile = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * (size_t)(blockIdx.z >> 3));
-  const size_t tiles = (size_t)gridDim.x * gridDim.y * (gridDim.z >> 3);
+  const unsigned nx = gridDim.x >> 3;
+  const size_t tile = (blockIdx.x >> 3) + nx * (blockIdx.y + gridDim.y * (size_t)blockIdx.z);
+  const size_t tiles = (size_t)nx * gridDim.y * gridDim.z;
   float* out = part + (job * tiles + tile) * (27 * 256);
   // ldmatrix.trans row addresses: matrix mi = lane/8, row r = lane%8
   const int mi = lane >> 3, rr = lane & 7;
@@ -888,7 +890,7 @@ void launch_conv3_wgrad(cudaStream_t s, const WgradJobs& jobs, float* part, floa
                                  (int)smem));
   });
   dim3 grid = conv_grid(g);
-  grid.z *= 8;
+  grid.x *= 8;
   k_conv3_wgrad<<<grid, NTHREADS, smem, s>>>(jobs, part, g);
   HX_CHECK_LAUNCH();
   const int len = 27 * 256;

@@ -1,7 +1,7 @@
-"""Meshes of several hundred thousand elements along one axis: the operator's
-columns in y pass the extent of a launch's y dimension there.
+"""Meshes and grids that are very long along one axis, where a kernel's blocks
+pass the extent (65535) of a launch's y or z dimension.
 
-The same beam along y and along x: 20 iterations of each CG form from zero,
+The same beam of several hundred thousand elements along y and along x: 20 iterations of each CG form from zero,
 which differ by rounding only (K x of a mesh with its axes exchanged; 1e-9 of the
 largest displacement for FP64, 1e-4 for the FP32 iterations)."""
 import numpy as np
@@ -45,3 +45,30 @@ def test_a_long_beam_along_y(hx, kw, tol):
     ux, uy = _iterate(hx, 0, **kw), _iterate(hx, 1, **kw)
     assert np.abs(ux).max() > 0
     assert np.abs(ux - uy).max() <= tol * np.abs(ux).max()
+
+
+def test_network_gradients_on_a_long_grid(hx):
+    """A grid of 33000 nodes in z (8250 tiles for each of the layers' 8 uses) against its four
+    quarters: dy is 0 but for the middle of each, 16 nodes (the reach of 8 layers and as much
+    again) from the ends, so that the gradients are the sums of the quarters' (FP32 sums in
+    another order: 1e-4 of the largest)."""
+    import importlib
+    learned = importlib.import_module("2025_12_09_hexat_v069_b200.learned")
+    nz, q = 33000, 8250
+    rng = np.random.default_rng(5)
+    x0 = rng.standard_normal((nz, 2, 2, 16)).astype(np.float32)
+    dy = np.zeros_like(x0)
+    for i in range(4):
+        dy[i * q + 16:(i + 1) * q - 16] = rng.standard_normal((q - 32, 2, 2, 16))
+    with hx.Context(0) as ctx:
+        ctx.set_grid(4, 4, 4)
+        ctx.set_material(1.0, 0.3)
+        ctx.net_set_params(learned.load_params())
+        _, g = ctx.net_forward_backward((2, 2, nz), x0.reshape(-1, 16), dy.reshape(-1, 16))
+        s = np.zeros_like(g)
+        for i in range(4):
+            cut = slice(i * q, (i + 1) * q)
+            s += ctx.net_forward_backward((2, 2, q), x0[cut].reshape(-1, 16),
+                                          dy[cut].reshape(-1, 16))[1]
+    assert np.abs(g).max() > 0
+    assert np.abs(g - s).max() <= 1e-4 * np.abs(g).max()
