@@ -101,6 +101,8 @@ template <typename T>
 void launch_node_diag(cudaStream_t s, const T* fac, const uint8_t* bcfree, uint8_t* nmask, T* diag,
                       const Grid& g, const ElemCoef<double>& K, double* partials, CgState* st,
                       double* out);
+void launch_bounded_factors(cudaStream_t s, const double* fac, const uint8_t* nmask, double* out,
+                            const Grid& g);
 template <typename T>
 void launch_minv(cudaStream_t s, const uint8_t* nmask, const T* diag, T* minv, int64_t nn,
                  double shift);
@@ -231,6 +233,8 @@ struct hx_ctx {
   hx::DevBuf<double> d_f, d_b, d_fac, d_x, d_r, d_p, d_p2, d_q, d_minv, d_xbest;
   hx::DevBuf<double> d_partials, d_scalars;
   hx::DevBuf<hx::CgState> d_state;
+  bool wild_factors = false;          // the last set-up met factors beyond range
+  hx::DevBuf<double> d_fac_bounded;   // (see operator_factors)
   hx::DevBuf<float> d_fac32, d_minv32, d_r32, d_p32, d_p32b, d_q32, d_x32;
   hx::DevBuf<double> d_aux0, d_aux1, d_aux2, d_aux3, d_aux4, d_aux5;
   hx::CgState* h_state = nullptr;  // pinned mirror

@@ -947,6 +947,7 @@ int pcg_snapshots(hx_ctx* c, const double* f, const double* fac, int every, int 
   if (c->bc_dirty) upload_bc(c);
   double shift = 0;
   jacobi_setup_public(c, fac, 0.0, &shift);
+  fac = operator_factors(c, fac);
   double* b = c->d_b.ensure(n);
   launch_mask_rhs<double>(c->stream, f, c->d_minv.p, b, n);
   double* x = c->d_x.ensure(n);

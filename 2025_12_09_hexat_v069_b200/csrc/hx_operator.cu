@@ -920,16 +920,20 @@ __global__ void __launch_bounds__(MV_BX* Tile<T, mode_fused(MODE)>::WARPS,
   }
 }
 
+// Factors beyond the range of the FP32 forms, infinite or NaN.
+__device__ __forceinline__ bool beyond_range(double f) { return !(fabs(f) <= 3e38); }
+
 // Per-node Jacobi diagonal: diag(n,c) = kd[c] * sum of the factors of the
 // (up to 8) elements around n; node mask = free-DOF bits of `bcfree`
-// cleared where the node carries no stiffness.  Writes diag into `diag`,
-// the mask into `nmask`, and reduces the max diagonal over free DOFs.
+// cleared where the node carries no stiffness (or a NaN).  Writes diag into `diag`,
+// the mask into `nmask`, and reduces the max diagonal over free DOFs (out[0]) and
+// whether any node's sum is beyond_range (out[1]).
 template <typename T>
 __global__ void k_node_diag(const T* __restrict__ fac, const uint8_t* __restrict__ bcfree,
                             uint8_t* __restrict__ nmask, T* __restrict__ diag, Grid g,
                             ElemCoef<double> K, double* partials, CgState* st, double* out) {
   const int64_t nn = (int64_t)g.nxn * g.nyn * g.nzn;
-  double mx = 0.0;
+  double mx = 0.0, wild = 0.0;
   for (int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; n < nn;
        n += (int64_t)gridDim.x * blockDim.x) {
     const int i = (int)(n % g.nxn);
@@ -947,6 +951,7 @@ __global__ void k_node_diag(const T* __restrict__ fac, const uint8_t* __restrict
           if (ei >= 0 && ej >= 0 && ek >= 0 && ei < g.nxe && ej < g.nye && ek < g.nze)
             s += (double)fac[((int64_t)ek * g.nye + ej) * g.nxe + ei];
         }
+    if (beyond_range(s)) wild = 1.0;
     const unsigned m = (s > 0.0) ? (bcfree ? bcfree[n] : 7u) : 0u;
     nmask[n] = (uint8_t)m;
 #pragma unroll
@@ -956,8 +961,32 @@ __global__ void k_node_diag(const T* __restrict__ fac, const uint8_t* __restrict
       if ((m >> c) & 1u) mx = fmax(mx, d);
     }
   }
-  double v[1] = {mx};
-  if (grid_reduce<1, true>(v, partials, &st->ticket[TK_AUX]) && threadIdx.x == 0) out[0] = v[0];
+  double v[2] = {mx, wild};
+  if (grid_reduce<2, true>(v, partials, &st->ticket[TK_AUX]) && threadIdx.x == 0) {
+    out[0] = v[0];
+    out[1] = v[1];
+  }
+}
+
+// The factors with those beyond_range set to 0 where all nodes of the element are
+// fixed: it has no part in any free row, but 0 times such a factor is a NaN.
+__global__ void k_bounded_factors(const double* __restrict__ fac,
+                                  const uint8_t* __restrict__ nmask, double* __restrict__ out,
+                                  Grid g) {
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < g.elems();
+       e += (int64_t)gridDim.x * blockDim.x) {
+    double f = fac[e];
+    if (beyond_range(f)) {
+      const int i = (int)(e % g.nxe);
+      const int64_t r = e / g.nxe;
+      const int j = (int)(r % g.nye), k = (int)(r / g.nye);
+      unsigned free = 0;
+      for (int b = 0; b < 8; ++b)
+        free |= nmask[((int64_t)(k + (b >> 2)) * g.nyn + j + ((b >> 1) & 1)) * g.nxn + i + (b & 1)];
+      if (!free) f = 0.0;
+    }
+    out[e] = f;
+  }
 }
 
 // minv = free ? 1/(diag + shift) : 0   (src/Solvers/GPUSolver.jl:402)
@@ -1191,6 +1220,13 @@ template void launch_node_diag<double>(cudaStream_t, const double*, const uint8_
 template void launch_node_diag<float>(cudaStream_t, const float*, const uint8_t*, uint8_t*, float*,
                                       const Grid&, const ElemCoef<double>&, double*, CgState*,
                                       double*);
+
+void launch_bounded_factors(cudaStream_t s, const double* fac, const uint8_t* nmask, double* out,
+                            const Grid& g) {
+  const unsigned blocks = std::min<int64_t>(cdiv(g.elems(), 256), 8LL * sm_count());
+  k_bounded_factors<<<blocks, 256, 0, s>>>(fac, nmask, out, g);
+  HX_CHECK_LAUNCH();
+}
 
 template <typename T>
 void launch_minv(cudaStream_t s, const uint8_t* nmask, const T* diag, T* minv, int64_t nn,

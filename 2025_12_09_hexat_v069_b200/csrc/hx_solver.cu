@@ -236,15 +236,22 @@ double jacobi_setup_public(hx_ctx* c, const double* fac, double shift_factor, do
   put_state(c, 3, CgState{});
   launch_node_diag<double>(c->stream, fac, c->d_bcfree.p, c->d_nmask.p, c->d_minv.p, g, c->K,
                            c->d_partials.p, c->d_state.p + 3, c->d_scalars.p);
-  double maxd = 0;
-  HX_CUDA(cudaMemcpyAsync(&c->h_state[3].aux[0], c->d_scalars.p, sizeof(double),
+  HX_CUDA(cudaMemcpyAsync(&c->h_state[3].aux[0], c->d_scalars.p, 2 * sizeof(double),
                           cudaMemcpyDeviceToHost, c->stream));
   HX_CUDA(cudaStreamSynchronize(c->stream));
-  maxd = c->h_state[3].aux[0];
+  const double maxd = c->h_state[3].aux[0];
+  c->wild_factors = c->h_state[3].aux[1] != 0.0;
   const double shift = shift_factor * maxd;
   launch_minv<double>(c->stream, c->d_nmask.p, c->d_minv.p, c->d_minv.p, nn, shift);
   *shift_out = shift;
   return maxd;
+}
+
+const double* operator_factors(hx_ctx* c, const double* fac) {
+  if (!c->wild_factors) return fac;
+  double* bounded = c->d_fac_bounded.ensure(c->g.elems());
+  launch_bounded_factors(c->stream, fac, c->d_nmask.p, bounded, c->g);
+  return bounded;
 }
 
 // ---------------------------------------------------------------------------
@@ -506,6 +513,7 @@ hx_status solve_grid(hx_ctx* c, const double* f, const double* fac, double* u,
   CgState last{};
   bool timed_out = false;
   int total_iters = 0;
+  const double* op = fac;  // the factors that the operator works with
   double t_setup = 0;
   // the reference's Jacobi -> AMG switch (GPUSolver.jl:540-579), with the
   // multigrid preconditioner in place of the CPU AMG
@@ -516,10 +524,11 @@ hx_status solve_grid(hx_ctx* c, const double* f, const double* fac, double* u,
     c->gmg.prepared = false;
     if (attempt == 1) {
       maxd = jacobi_setup_public(c, fac, factor, &shift);
+      op = operator_factors(c, fac);
       if (late) {
         if (use_mg) {
           const double tg = now_ms();
-          gmg_prepare(c, fac, shift);
+          gmg_prepare(c, op, shift);
           ts += now_ms() - tg;  // reported as the preconditioner's
         }
         (*late)();
@@ -539,9 +548,9 @@ hx_status solve_grid(hx_ctx* c, const double* f, const double* fac, double* u,
     if (o.preconditioner == HX_PC_LEARNED) {
       int fb = 0, its = 0;
       if (o.precision == HX_PREC_FP64) {
-        st = solve_learned(c, fac, b, u, warm, shift, o, t0, &timed_out, &fb, &its);
+        st = solve_learned(c, op, b, u, warm, shift, o, t0, &timed_out, &fb, &its);
       } else {
-        st = solve_learned_mixed(c, fac, b, u, warm, shift, o, t0, &timed_out, &fb, &its);
+        st = solve_learned_mixed(c, op, b, u, warm, shift, o, t0, &timed_out, &fb, &its);
         R.refinements = c->h_state[0].iter;
       }
       total_iters += its;
@@ -549,21 +558,21 @@ hx_status solve_grid(hx_ctx* c, const double* f, const double* fac, double* u,
     } else if (use_mg) {
       int its = 0;
       if (o.precision == HX_PREC_FP64) {
-        st = solve_gmg(c, fac, b, u, warm, shift, o, t0, &timed_out, &its);
+        st = solve_gmg(c, op, b, u, warm, shift, o, t0, &timed_out, &its);
         if (o.preconditioner != HX_PC_MULTIGRID) R.fallback_used = 1;
       } else {
         int fb = 0;
-        st = solve_gmg_mixed(c, fac, b, u, warm, shift, o, t0, &timed_out, &fb, &its);
+        st = solve_gmg_mixed(c, op, b, u, warm, shift, o, t0, &timed_out, &fb, &its);
         R.refinements = c->h_state[0].iter;
         R.fallback_used = fb || o.preconditioner != HX_PC_MULTIGRID;
       }
       total_iters += its;
     } else if (o.precision == HX_PREC_FP64) {
-      st = pcg_fp64(c, fac, b, u, warm, shift, o, t0, &timed_out);
+      st = pcg_fp64(c, op, b, u, warm, shift, o, t0, &timed_out);
       total_iters += st.iter;
     } else {
       int inner = 0;
-      st = solve_mixed(c, fac, b, u, warm, shift, o, t0, &timed_out, &inner);
+      st = solve_mixed(c, op, b, u, warm, shift, o, t0, &timed_out, &inner);
       total_iters += inner;
       R.refinements = c->h_state[0].iter;
     }
@@ -577,7 +586,7 @@ hx_status solve_grid(hx_ctx* c, const double* f, const double* fac, double* u,
     for (int restart = 0; restart < 2 && !o.ref_retry && o.precision == HX_PREC_FP64 &&
                           st.status == HX_ST_CONVERGED && !timed_out;
          ++restart) {
-      if (true_residual(c, fac, b, u, shift) < o.tol) break;
+      if (true_residual(c, op, b, u, shift) < o.tol) break;
       hx_solve_opts oc = o;
       oc.max_iter = o.max_iter - total_iters;
       if (oc.max_iter <= 0) {
@@ -586,15 +595,15 @@ hx_status solve_grid(hx_ctx* c, const double* f, const double* fac, double* u,
       }
       if (o.preconditioner == HX_PC_LEARNED) {
         int fb = 0, its = 0;
-        st = solve_learned(c, fac, b, u, true, shift, oc, t0, &timed_out, &fb, &its);
+        st = solve_learned(c, op, b, u, true, shift, oc, t0, &timed_out, &fb, &its);
         total_iters += its;
         R.fallback_used |= fb;
       } else if (use_mg) {
         int its = 0;
-        st = solve_gmg(c, fac, b, u, true, shift, oc, t0, &timed_out, &its);
+        st = solve_gmg(c, op, b, u, true, shift, oc, t0, &timed_out, &its);
         total_iters += its;
       } else {
-        st = pcg_fp64(c, fac, b, u, true, shift, oc, t0, &timed_out);
+        st = pcg_fp64(c, op, b, u, true, shift, oc, t0, &timed_out);
         total_iters += st.iter;
       }
       R.refinements += 1;
@@ -651,7 +660,7 @@ hx_status solve_grid(hx_ctx* c, const double* f, const double* fac, double* u,
   R.rel_res = last.rel_res;
   R.shift = shift;
   if (o.verify_true_residual) {
-    R.true_rel_res = (last.status == HX_ST_ZERO_RHS) ? 0.0 : true_residual(c, fac, b, u, shift);
+    R.true_rel_res = (last.status == HX_ST_ZERO_RHS) ? 0.0 : true_residual(c, op, b, u, shift);
   } else {
     R.true_rel_res = NAN;
   }

@@ -42,6 +42,10 @@ class GraphLoop {
 };
 // node masks, diagonal, shift and M^-1 (FP64) for `fac`; returns max diag
 double jacobi_setup_public(hx_ctx* c, const double* fac, double shift_factor, double* shift_out);
+// after it: the factors to work with.  The fused steps and the smoother leave
+// the fixed DOFs of K p unmasked (p, M^-1 and z are 0 there), so an infinite or NaN factor among
+// fixed nodes only would reach p.q as 0 times NaN; such factors are 0 in a copy.
+const double* operator_factors(hx_ctx* c, const double* fac);
 template <typename T>
 CgState pcg_fused(hx_ctx* c, int slot, const T* fac, const T* b, T* x, bool warm, T shift,
                   const ElemCoef<T>& K, T* r, T* P0, T* P1, T* q, const T* minv, T* xbest,
