@@ -969,6 +969,9 @@ void launch_restrict(cudaStream_t s, int ch, const float* in, float* out, const 
   const int64_t ctas = cdiv((int64_t)gc.ny * gc.nz, block.y);
   const unsigned nb = vec_blocks((int64_t)gc.nx * gc.ny * gc.nz);
   const int nrm = normalise ? 1 : 0;
+  // by row while the CTAs are one wave (61 x 21 x 21 coarse nodes, 441 CTAs: 5.0 us by row, 8.1
+  // by node); at two waves the forms are equal (65 x 33 x 33: 8.2 and 8.3), from there
+  // on the node form wins (73 x 37 x 37: 9.7 and 9.6, 97 x 49 x 49: 18.9 and 12.3)
   if (ch == 3 && one_wave(ctas, 4))
     launch_pdl(k_restrict_row, dim3((unsigned)ctas), block, 0, s, in, out, gf, gc, nrm, cmask, st);
   else if (ch == 3)

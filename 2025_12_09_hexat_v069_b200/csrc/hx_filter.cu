@@ -18,7 +18,7 @@
 // types), so no vector holds it.  The update (k_filter_update) is the rest.  At
 // a million nodes the vectors fit the L2 and latency bounds both kernels: an
 // iteration at 161 x 81 x 81 nodes took 56 us (plain product from 27 global
-// loads per node, then two passes over five vectors) and takes 32 us.
+// loads per node, then two passes over five vectors) and takes 30 us.
 #include "hx_internal.h"
 
 namespace hx {

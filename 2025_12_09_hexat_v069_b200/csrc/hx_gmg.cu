@@ -702,7 +702,10 @@ void gmg_vcycle(hx_ctx* c, const T* r, T* z, const CgState* st) {
     b = l == 0 ? b0 : G.lv[l].b.p;
     x = l == 0 ? x0 : G.lv[l].x.p;
   };
-  // the test of the state costs a small kernel more than it can save
+  // Kernels of levels beyond 500000 DOFs test the state: the last cycle of a solve runs
+  // in vain (a graph holds two).  A solve (13 iterations) at 320 x 160 x 160 takes 19.1 ms
+  // so, 19.8 without the test; with it on the small levels too 19.15, and 3.60 instead of
+  // 3.55 ms at 128 x 64 x 64: there it costs what it saves.
   auto level_st = [&](int l) { return G.lv[l].g.dofs() > 500000 ? st : nullptr; };
   for (int l = 0; l + 1 < nl; ++l) {
     auto& L = G.lv[l];

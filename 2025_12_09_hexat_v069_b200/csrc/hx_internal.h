@@ -69,8 +69,9 @@ void launch_matvec(cudaStream_t s, int mode, const T* x, T* y, const T* fac, con
                    const Grid& g, const ElemCoef<T>& K, T shift, CgState* st, double* partials,
                    double* out);
 // Fused PCG step (see hx_operator.cu): p_out = M^-1 r + beta p_in,
-// x += alpha_old p_in (owned nodes), q = mask(K p_out + s p_out),
-// st->alpha = rz / (p_out . q).  xbest (FP64): also receives x where the last
+// x += alpha_old p_in (owned nodes), q = K p_out + s p_out, st->alpha = rz /
+// (p_out . q).  q is not masked: on the fixed DOFs, where p_out is 0, it holds the
+// reactions, and what reads it multiplies by, or tests, M^-1, z or the node mask.  xbest (FP64): also receives x where the last
 // iteration asked for a snapshot of it (st->snap).
 template <typename T>
 void launch_pcg_step(cudaStream_t s, const T* pin, T* pout, const T* r, const T* minv, T* x, T* q,
@@ -78,7 +79,7 @@ void launch_pcg_step(cudaStream_t s, const T* pin, T* pout, const T* r, const T*
                      T shift, CgState* st, double* partials,
                      T* xbest = nullptr);
 // Flexible-CG step: p_out = z + beta p_in, x += alpha_old p_in (owned
-// nodes), q = mask(K p_out + s p_out), st->alpha = (z . r) / (p_out . q)
+// nodes), q = K p_out + s p_out (not masked, as above), st->alpha = (z . r) / (p_out . q)
 // with z . r in st->aux[3] (the preconditioner's output pass reduces it).
 // z: in T, or in FP32 for an FP64 step.
 template <typename T, typename TZ>

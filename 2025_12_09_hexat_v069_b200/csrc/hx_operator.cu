@@ -42,7 +42,9 @@
 // both precisions, 45-term product, two barriers per plane) and now: FP64 PCG
 // step 402 -> 319 us, FP64 K x 260 -> 205 us, FP32 PCG step 220 -> 182 us, FP32
 // flexible-CG step 207 -> 170 us; FP32 Chebyshev step and residual at 192 x 96
-// x 96: 55 -> 36 and 50 -> 36 us.
+// x 96: 55 -> 36 and 50 -> 36 us.  Boxes (sides 1 : 0.8 : 1.25), whose coefficients
+// come from the kernel's arguments, in the same order: 402 -> 328, 259 -> 209, 220 ->
+// 182, 208 -> 170 us, and a V-cycle 1607 -> 1003 us (cubes 983).
 // Measured and dropped (FP32 flexible-CG step, 320 x 160 x 160): one element
 // row per thread at 24 warps per SM 188 us; 8 warps x 2 CTAs (128 registers,
 // spills) 189-204 us; 12 x 1 201 us; 6 x 2 178 us; the plane loop unrolled
@@ -247,7 +249,8 @@ struct OpArgs {
                   // x_prev in, x_new out
   T* pout;        // FUSED: new direction p
   T* xbest;       // FUSED, FP64: receives x too when the state asks for a snapshot (or null)
-  T* q;           // output K p (masked, shifted)
+  T* q;           // output K x + s x, masked; FUSED: not masked (0 for p, not for q, on
+                  // the fixed DOFs); MODE 6: the residual
   const T* fac;
   const uint8_t* nmask;
   Grid g;
